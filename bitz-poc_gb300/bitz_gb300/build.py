@@ -18,7 +18,7 @@ BUILD = os.path.join(ROOT, "build")
 LIB = os.path.join(PKG, "libbitzgpu.so")
 INCLUDE = os.path.join(os.path.dirname(ROOT), "include")
 
-SOURCES = ["ntt.cu", "merkle.cu", "fold.cu", "runtime.cu", "batch.cu", "serve.cu", "pipeline.cu", "noalloc.cu",
+SOURCES = ["ntt.cu", "ntt_group.cu", "merkle.cu", "fold.cu", "runtime.cu", "batch.cu", "serve.cu", "pipeline.cu", "noalloc.cu",
            "transcript.cu", "pow.cu", "open.cu", "codec.cpp", "ligerito.cu",
            "pcs_open.cu", "ingest.cu", "shard.cu", "gkr.cu", "persist.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -201,6 +201,7 @@ int bz_autotune(bz_ctx *ctx, const bz_params *params, int reps, uint32_t *chosen
     }
     std::vector<uint32_t> cands;
     const int b = s.log_dim();
+    cands.push_back(default_schedule(s));
     if (s.log_lanes >= 9 && s.k_code() - s.log_inv_rate >= 3) {
         // radix-8 passes, the leftover layers last or first
         cands.push_back(SCHED_RADIX8);

@@ -52,7 +52,9 @@ struct LaunchLog {
 // generic one-layer-per-launch kernels (reference / fallback path), bit 6 =
 // fuse the last table layers with the deep layers into one tail pass, bits
 // 7..8 = narrow-multiply variant (0 shifts, 1 wide multiplies, 2 alternate),
-// bit 14 = radix-4 passes with narrow (<= 25-bit) twiddles use compact tables.
+// bit 14 = radix-4 passes with narrow (<= 25-bit) twiddles use compact tables,
+// bit 17 = the group passes for the deepest layers (overrides the bits above
+// where the shape has at least three layers).
 enum : uint32_t {
     SCHED_DEEP_MASK = 0xF,
     SCHED_RADIX2 = 0x10,
@@ -66,6 +68,7 @@ enum : uint32_t {
     SCHED_NARROW = 0x4000,        // compact 32-bit tables for the deepest layers' twiddles
     SCHED_RADIX8 = 0x8000,        // radix-8 passes (eight 32 KB byte tables per twiddle)
     SCHED_R8_HEAD = 0x10000,      // with SCHED_RADIX8: the 1-2 leftover layers run first
+    SCHED_GROUP = 0x20000,        // the deepest layers as group passes (ntt_group.cuh)
     SCHED_SHORT_CTAS = 0x200000,  // table passes in 16 CTAs per SM instead of one long one
 };
 uint32_t default_schedule(const Shape &s);
@@ -84,6 +87,14 @@ int launch_ntt(const Shape &s, uint32_t schedule, const uint4 *d_msg, uint4 *d_c
 int launch_table_pass(const Shape &s, int layer, int layers, const uint4 *src, int src_bits,
                       uint4 *dst, const uint4 *tw, uint64_t p0, uint64_t p1, int threads,
                       cudaStream_t st, int num_sms, uint32_t schedule);
+// Group passes (ntt_group.cu): the last four layers of the transform (at
+// least 512 lanes), and three layers ending at `depth` for any lane count.
+bool group16_ok(const Shape &s);
+bool group8_ok(const Shape &s);
+int launch_group16(const Shape &s, const uint4 *src, int src_bits, uint4 *dst, const uint4 *tw,
+                   cudaStream_t st, int num_sms, int waves);
+int launch_group8(const Shape &s, int depth, const uint4 *src, int src_bits, uint4 *dst,
+                  const uint4 *tw, cudaStream_t st, int num_sms, int waves);
 // Bit length of the widest twiddle of `layer` in the ell-layer transform.
 int twiddle_bits(int ell, int layer);
 // Shapes whose whole transform runs in one ntt_small_kernel launch.
@@ -220,6 +231,7 @@ int launch_unpack_columns(const uint64_t *d_packed, int row_vars, int col_vars, 
 // One-time kernel attributes (large dynamic shared memory), called when a
 // context is created so no attribute call happens during graph capture.
 void init_ntt_kernels();
+void init_group_kernels();
 void init_fold_kernels();
 
 // Host GF(2^128) (twiddle tables, host-side checks of transcript values).

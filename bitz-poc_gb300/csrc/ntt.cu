@@ -126,18 +126,21 @@ int twiddle_bits(int ell, int layer) {
     return it->second[layer];
 }
 
-// Schedule of a shape the autotuner has not timed.  With at least 512 lanes
-// every layer fits the table passes (each 512-thread chunk stays inside one
-// block); radix-8 passes (three layers per sweep) measured faster than the
-// prefetching radix-4 passes at 2^20, 2^24 and 2^28 (3.33 against 3.49 ms at
-// 2^24); narrower shapes run their last three layers in the
-// register-resident deep pass.
+// Schedule of a shape the autotuner has not timed: radix-8 passes over the
+// wide layers and group passes over the deepest (launch_ntt), measured faster
+// than the prefetching radix-4 passes and the shift-and-XOR pass at every
+// lane count (2^22 elements, rate 1/2: 32 lanes 0.96 -> 0.72 ms, 4 lanes 1.37
+// -> 1.15 ms; 2^24, rate 1/4, 4096 lanes 2.73 -> 2.60 ms).  The other bits
+// are what a caller that does not know the group passes runs: from 512 lanes
+// radix-8 passes, below it the last three layers in the register-resident
+// deep pass.
 uint32_t default_schedule(const Shape &s) {
-    if (s.log_lanes >= 9 && s.k_code() - s.log_inv_rate >= 3) return SCHED_RADIX8;
+    const uint32_t group = group8_ok(s) ? SCHED_GROUP : 0u;
+    if (s.log_lanes >= 9 && s.k_code() - s.log_inv_rate >= 3) return SCHED_RADIX8 | group;
     if (s.log_lanes >= 9) return SCHED_PREFETCH | SCHED_NARROW;
     const int layers = s.log_dim();
     const int deep = std::min(layers, 3);
-    return (uint32_t)deep;
+    return (uint32_t)deep | group;
 }
 
 // CTAs per SM a table pass is cut into: 1 (one long CTA per SM) or, under
@@ -347,6 +350,7 @@ static inline unsigned grid_for(uint64_t n, int threads, int num_sms, int per_sm
 #define BZ_TAIL_ATTR_M(DT, DN) BZ_TAIL_ATTR(DT, DN, 0); BZ_TAIL_ATTR(DT, DN, 1); BZ_TAIL_ATTR(DT, DN, 2)
 
 void init_ntt_kernels() {
+    init_group_kernels();
     cudaFuncSetAttribute(ntt_table_pass<2, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)table_smem(2));
     cudaFuncSetAttribute(ntt_table_pass<1, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -540,6 +544,78 @@ int launch_ntt(const Shape &s, uint32_t schedule, const uint4 *d_msg, uint4 *d_c
             ++launches;
             src = d_cw;
             src_bits = 62;
+        }
+        return launches;
+    }
+    if ((schedule & SCHED_GROUP) && group8_ok(s)) {
+        // Passes of three layers, the last of three or (from 512 lanes, when
+        // that leaves no layer over) four as a group pass.  One layer over is
+        // taken with three others as two radix-4 passes (2^24 elements of 256
+        // lanes: 145 + 155 us against 126 us for the layer and 199 for the
+        // three), two layers as one.  They run after the first pass where
+        // that is a radix-8 pass, whose block of zero twiddles is worth the
+        // most layers.
+        const int waves = cta_waves(schedule);
+        const int last = group16_ok(s) && (ell - r) % 3 == 1 ? 4 : 3;
+        const int mid = ell - r - last;
+        int quads = mid % 3 == 2 ? 1 : mid % 3 == 1 && mid >= 4 ? 2 : 0;
+        int layer = r;
+        auto done = [&](const char *name, int layers) {
+            if (log) log->mark((std::string(name) + (src == d_msg ? "_first" : "") + "@" +
+                                std::to_string(layer)).c_str());
+            src = d_cw;
+            src_bits = 62;
+            layer += layers;
+            ++launches;
+        };
+        auto generic_layers = [&](int layers) {
+            const uint64_t n_tasks = ((uint64_t)1 << (ell - 1)) << L;
+            for (int k = 0; k < layers; ++k) {
+                ntt_generic_layer<<<grid_for(n_tasks, 256, num_sms, 8), 256, 0, st>>>(
+                    src, d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
+                done("ntt_generic_layer", 1);
+            }
+        };
+        auto table_layers = [&](int layers) {
+            if (!table_pass_ok(ell, layer, layers, L)) return generic_layers(layers);
+            launch_table_pass(s, layer, layers, src, src_bits, d_cw, d_tw, 0, P, 512, st, num_sms,
+                              SCHED_PREFETCH | SCHED_NARROW | (schedule & SCHED_SHORT_CTAS));
+            done(layers == 2 ? "ntt_table_pass2" : "ntt_table_pass1", layers);
+        };
+        // A radix-8 pass takes blocks of at least one chunk of 512 tasks, and
+        // below 512 lanes a chunk for every SM (2^18 elements of 32 lanes: 16
+        // us a pass against 14 us for a group pass of smaller CTAs).
+        auto radix8 = [&] {
+            return ell - layer - 3 + L >= 9 &&
+                   (L >= 9 || (P << L) >> 12 >= (uint64_t)num_sms);
+        };
+        auto three = [&] {
+            if (radix8()) {
+                const bool nw = launch_pass8(s, layer, src, src_bits, d_cw, d_tw, st, num_sms,
+                                             waves);
+                done(nw ? "ntt_pass8_nw" : "ntt_pass8", 3);
+            } else if (L >= 2) {
+                launch_group8(s, ell - layer - 3, src, src_bits, d_cw, d_tw, st, num_sms, waves);
+                done("ntt_group8", 3);
+            } else {
+                // the offsets of one or two lanes differ within a warp, and
+                // the generic multiply is faster (2^22 elements of one lane,
+                // depths 3-5: 184 us against 250 us)
+                generic_layers(3);
+            }
+        };
+        if (mid == 1) table_layers(1);
+        const int threes = (mid - 2 * quads) / 3;
+        const bool first8 = threes > 0 && radix8();
+        if (first8) three();
+        for (; quads; --quads) table_layers(2);
+        for (int k = first8; k < threes; ++k) three();
+        if (last == 4) {
+            launch_group16(s, src, src_bits, d_cw, d_tw, st, num_sms, waves);
+            done("ntt_group16", 4);
+        } else {
+            launch_group8(s, 0, src, src_bits, d_cw, d_tw, st, num_sms, waves);
+            done("ntt_group8", 3);
         }
         return launches;
     }
