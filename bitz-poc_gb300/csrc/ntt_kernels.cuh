@@ -381,11 +381,13 @@ __device__ __forceinline__ uint4 pass_mul(const T8Lane &lc, const char *tb, uint
 }
 
 //
-// Body: task chunks [c_beg, c_end) of blockDim.x tasks; tbl holds the seven
-// tables (kPass8Smem bytes), tw_buf kTw8Window * 7 twiddles, win two words.
+// Body: task chunks c_beg, c_beg + c_step, .. below c_end of blockDim.x tasks;
+// tbl holds the seven tables (kPass8Smem bytes), tw_buf kTw8Window * 7
+// twiddles, win two words.
 template <int W0, int W1, int W2>
 __device__ __forceinline__ void pass8_body(const TablePassArgs &a, uint64_t c_beg, uint64_t c_end,
-                                           char *tbl, uint4 *tw_buf, uint64_t *win) {
+                                           char *tbl, uint4 *tw_buf, uint64_t *win,
+                                           uint64_t c_step = 1) {
     if (threadIdx.x == 0) win[0] = win[1] = 0;
     T8Lane lc;
     lc.init();
@@ -399,7 +401,7 @@ __device__ __forceinline__ void pass8_body(const TablePassArgs &a, uint64_t c_be
     uint32_t zmask = 0;  // zero twiddles of the current block
     constexpr int n0 = build_items<W0>(), n1 = build_items<W1>(), n2 = build_items<W2>();
     constexpr int n_items = n0 + 2 * n1 + 4 * n2;
-    for (uint64_t c = c_beg; c < c_end; ++c) {
+    for (uint64_t c = c_beg; c < c_end; c += c_step) {
         const uint64_t task = a.task_base + c * blockDim.x + threadIdx.x;
         const uint64_t B = task >> log_task_per_b;  // uniform across the CTA
         if ((int64_t)B != cur_b) {
