@@ -115,7 +115,10 @@ __device__ __forceinline__ void b3_parent(const uint32_t l[8], const uint32_t r[
 // ---------------------------------------------------------------------------
 // SHA-256
 // ---------------------------------------------------------------------------
-__device__ __constant__ uint32_t kSHA[64] = {
+struct ShaWords {
+    uint32_t w[64];
+};
+constexpr ShaWords kShaK = {{
     0x428a2f98, 0x71374491, 0xb5c0fbcf, 0xe9b5dba5, 0x3956c25b, 0x59f111f1, 0x923f82a4, 0xab1c5ed5,
     0xd807aa98, 0x12835b01, 0x243185be, 0x550c7dc3, 0x72be5d74, 0x80deb1fe, 0x9bdc06a7, 0xc19bf174,
     0xe49b69c1, 0xefbe4786, 0x0fc19dc6, 0x240ca1cc, 0x2de92c6f, 0x4a7484aa, 0x5cb0a9dc, 0x76f988da,
@@ -123,49 +126,93 @@ __device__ __constant__ uint32_t kSHA[64] = {
     0x27b70a85, 0x2e1b2138, 0x4d2c6dfc, 0x53380d13, 0x650a7354, 0x766a0abb, 0x81c2c92e, 0x92722c85,
     0xa2bfe8a1, 0xa81a664b, 0xc24b8b70, 0xc76c51a3, 0xd192e819, 0xd6990624, 0xf40e3585, 0x106aa070,
     0x19a4c116, 0x1e376c08, 0x2748774c, 0x34b0bcb5, 0x391c0cb3, 0x4ed8aa4a, 0x5b9cca4f, 0x682e6ff3,
-    0x748f82ee, 0x78a5636f, 0x84c87814, 0x8cc70208, 0x90befffa, 0xa4506ceb, 0xbef9a3f7, 0xc67178f2};
+    0x748f82ee, 0x78a5636f, 0x84c87814, 0x8cc70208, 0x90befffa, 0xa4506ceb, 0xbef9a3f7, 0xc67178f2}};
 
-// w: 16 big-endian message words (already byte-swapped).
+// kSHA[i] + w_i over the 64 rounds of a block known in advance: the padding
+// block of a message of bitlen bits that ends on a block boundary.
+constexpr ShaWords sha_pad_kw(uint64_t bitlen) {
+    ShaWords r = {};
+    uint32_t w[64] = {};
+    w[0] = 0x80000000u;
+    w[14] = (uint32_t)(bitlen >> 32);
+    w[15] = (uint32_t)bitlen;
+    for (int i = 16; i < 64; ++i) {
+        const uint32_t x = w[i - 15], y = w[i - 2];
+        const uint32_t s0 = ((x >> 7) | (x << 25)) ^ ((x >> 18) | (x << 14)) ^ (x >> 3);
+        const uint32_t s1 = ((y >> 17) | (y << 15)) ^ ((y >> 19) | (y << 13)) ^ (y >> 10);
+        w[i] = w[i - 16] + s0 + w[i - 7] + s1;
+    }
+    for (int i = 0; i < 64; ++i) r.w[i] = kShaK.w[i] + w[i];
+    return r;
+}
+__device__ __constant__ ShaWords kSHA = kShaK;
+__device__ __constant__ ShaWords kShaPairPad = sha_pad_kw(512);  // after a 64-byte pair
+
+// One round; kw = kSHA[i] + w_i.  The additions off the chain from e to the
+// next e and from a to the next a are multiply-adds by a runtime 1, as in
+// BLAKE3 above: on the FMA pipe they leave the ALU pipe its rotates and logic.
+#define BZ_SHA_ROUND(a, b, c, d, e, f, g, h, kw)                                        \
+    do {                                                                                \
+        const uint32_t hkw = h * one + (kw);                                            \
+        const uint32_t S1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);                     \
+        const uint32_t ch = (e & f) ^ (~e & g);                                         \
+        const uint32_t t1 = S1 + ch + hkw;                                              \
+        const uint32_t S0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);                     \
+        const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);                                \
+        d = S1 + ch + (d * one + hkw);                                                  \
+        h = t1 + S0 + mj;                                                               \
+    } while (0)
+#define BZ_SHA_ROUND_AT(v, i, kw)                                                       \
+    BZ_SHA_ROUND(v[(64 - (i)) & 7], v[(65 - (i)) & 7], v[(66 - (i)) & 7],               \
+                 v[(67 - (i)) & 7], v[(68 - (i)) & 7], v[(69 - (i)) & 7],               \
+                 v[(70 - (i)) & 7], v[(71 - (i)) & 7], kw)
+
+// w: 16 big-endian message words (already byte-swapped).  ROLLED: sixteen
+// rounds are unrolled (register names and schedule slots repeat with that
+// period) and the rest loops, 12 KB of code instead of 30: trees and the upper
+// levels run a few warps that otherwise spend a quarter of their stalls
+// fetching instructions (nine levels over 512 nodes: 31 us against 49 us).  A
+// full GPU of leaves is bound by the ALU pipe and takes the plain additions
+// and no loop (2^18 leaves of 512 bytes: 174 us against 182 us).
+template <bool ROLLED>
 __device__ __forceinline__ void sha256_compress(uint32_t st[8], const uint32_t w_in[16]) {
-    uint32_t w[16];
+    const uint32_t one = ROLLED ? kOne : 1u;
+    uint32_t w[16], v[8];
 #pragma unroll
     for (int i = 0; i < 16; ++i) w[i] = w_in[i];
-    uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6],
-             h = st[7];
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-        uint32_t wi;
-        if (i < 16) {
-            wi = w[i];
-        } else {
-            const uint32_t x = w[(i - 15) & 15], y = w[(i - 2) & 15];
+    for (int i = 0; i < 8; ++i) v[i] = st[i];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) BZ_SHA_ROUND_AT(v, i, w[i] * one + kSHA.w[i]);
+#pragma unroll(ROLLED ? 1 : 3)
+    for (int r = 16; r < 64; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
             const uint32_t s0 = rotr(x, 7) ^ rotr(x, 18) ^ (x >> 3);
             const uint32_t s1 = rotr(y, 17) ^ rotr(y, 19) ^ (y >> 10);
-            wi = w[i & 15] + s0 + w[(i - 7) & 15] + s1;
-            w[i & 15] = wi;
+            w[i] = s1 * one + (s0 * one + (w[(i + 9) & 15] * one + w[i]));
+            BZ_SHA_ROUND_AT(v, i, w[i] * one + kSHA.w[r + i]);
         }
-        const uint32_t S1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);
-        const uint32_t ch = (e & f) ^ (~e & g);
-        const uint32_t t1 = h + S1 + ch + kSHA[i] + wi;
-        const uint32_t S0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);
-        const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
-        h = g;
-        g = f;
-        f = e;
-        e = d + t1;
-        d = c;
-        c = b;
-        b = a;
-        a = t1 + S0 + mj;
     }
-    st[0] += a;
-    st[1] += b;
-    st[2] += c;
-    st[3] += d;
-    st[4] += e;
-    st[5] += f;
-    st[6] += g;
-    st[7] += h;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] += v[i];
+}
+
+// A block whose kSHA[i] + w_i are known: no message schedule.
+template <bool ROLLED>
+__device__ __forceinline__ void sha256_compress_kw(uint32_t st[8], const ShaWords &kw) {
+    const uint32_t one = ROLLED ? kOne : 1u;
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = st[i];
+#pragma unroll(ROLLED ? 1 : 4)
+    for (int r = 0; r < 64; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) BZ_SHA_ROUND_AT(v, i, kw.w[r + i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] += v[i];
 }
 
 __device__ __forceinline__ uint32_t bswap32(uint32_t x) { return __byte_perm(x, 0, 0x0123); }

@@ -41,9 +41,10 @@ __global__ void __launch_bounds__(256) merkle_levels(LevelsArgs a) {
     merkle_levels_body(a, blockIdx.x, nodes);
 }
 
-__global__ void sha_leaves(const uint4 *cw, int log_lanes, uint64_t n_leaves,
-                           uint32_t *tree_leaves) {
-    sha_leaves_body(cw, log_lanes, n_leaves, tree_leaves,
+__global__ void __launch_bounds__(128) sha_leaves(const uint4 *cw, int log_lanes,
+                                                  uint64_t n_leaves, uint32_t *tree_leaves,
+                                                  const __grid_constant__ ShaWords pad) {
+    sha_leaves_body(cw, log_lanes, n_leaves, tree_leaves, pad,
                     (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
 }
@@ -105,6 +106,34 @@ __global__ void __launch_bounds__(kTreeSmallMax) b3_tree_small(const uint4 *cw, 
         }
         __syncthreads();
         off += half;
+    }
+}
+
+// A small SHA-256 tree in one CTA: thread i hashes leaf i, then the CTA builds
+// every level.  Up to one warp per scheduler, so no leaf's chain waits for
+// another's.
+constexpr int kShaTreeSmallMax = 128;  // leaves (threads)
+__global__ void __launch_bounds__(kShaTreeSmallMax) sha_tree_small(
+    const uint4 *cw, int log_lanes, uint32_t n_leaves, uint32_t *tree,
+    const __grid_constant__ ShaWords pad) {
+    __shared__ uint32_t nodes[kShaTreeSmallMax][9];  // padded rows
+    const uint32_t t = threadIdx.x;
+    uint32_t o[8];
+    sha_leaf<true>(cw + ((uint64_t)t << log_lanes), log_lanes, pad, o);
+    uint64_t off = 0;
+    for (uint32_t n = n_leaves;; n >>= 1) {
+        if (t < n) {
+            uint4 *po = reinterpret_cast<uint4 *>(tree + (off + t) * 8);
+            po[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            po[1] = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
+        }
+        if (n == 1) break;
+        __syncthreads();
+        if (t < n / 2) sha256_pair(nodes[2 * t], nodes[2 * t + 1], o);
+        __syncthreads();  // every read of this level precedes the overwrite
+        off += n;
     }
 }
 
@@ -177,7 +206,8 @@ int launch_leaves_range(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint
                 cw, n_chunks, leaves, log_c, s.chunk0);
         }
     } else {
-        sha_leaves<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(cw, s.log_lanes, n, leaves);
+        sha_leaves<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(cw, s.log_lanes, n, leaves,
+                                                                sha_pad_kw(s.leaf_bytes() * 8));
     }
     return 1;
 }
@@ -281,8 +311,15 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
             }
         }
     } else {
+        const ShaWords pad = sha_pad_kw(s.leaf_bytes() * 8);
+        if (n_leaves <= (uint64_t)kShaTreeSmallMax) {
+            sha_tree_small<<<1, (unsigned)n_leaves, 0, st>>>(d_cw, s.log_lanes,
+                                                             (uint32_t)n_leaves, tree, pad);
+            mark("sha_tree_small");
+            return 1;
+        }
         sha_leaves<<<(unsigned)((n_leaves + 127) / 128), 128, 0, st>>>(d_cw, s.log_lanes,
-                                                                       n_leaves, tree);
+                                                                       n_leaves, tree, pad);
         mark("sha_leaves");
         ++launches;
     }

@@ -117,12 +117,8 @@ __device__ __forceinline__ void sha256_pair(const uint32_t l[8], const uint32_t 
         w[i] = bswap32(l[i]);
         w[8 + i] = bswap32(r[i]);
     }
-    sha256_compress(st, w);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) w[i] = 0;
-    w[0] = 0x80000000u;
-    w[15] = 512;
-    sha256_compress(st, w);
+    sha256_compress<true>(st, w);
+    sha256_compress_kw<true>(st, kShaPairPad);
 #pragma unroll
     for (int i = 0; i < 8; ++i) out[i] = bswap32(st[i]);
 }
@@ -148,40 +144,32 @@ struct LevelsArgs {
 // the CTA only take part in its barriers.  nodes holds 256 padded rows.
 __device__ __forceinline__ void merkle_levels_body(const LevelsArgs &a, uint64_t u,
                                                    uint32_t (*nodes)[9]) {
-    const uint64_t base_in = u * 512;
     const int t = threadIdx.x;
-    const bool lane_ok = t < 256;
-    // level 0 of this CTA: parents of input pairs
-    uint64_t n_lvl = a.n_in >> 1;  // nodes at the first output level
-    {
-        const uint64_t j = (u * 256) + t;
-        uint32_t o[8];
-        if (lane_ok && j < n_lvl) {
-            uint32_t l[8], r[8];
-            const uint4 *pl = reinterpret_cast<const uint4 *>(a.in + (base_in + 2 * t) * 8);
-            const uint4 l0 = pl[0], l1 = pl[1], r0 = pl[2], r1 = pl[3];
-            l[0] = l0.x; l[1] = l0.y; l[2] = l0.z; l[3] = l0.w;
-            l[4] = l1.x; l[5] = l1.y; l[6] = l1.z; l[7] = l1.w;
-            r[0] = r0.x; r[1] = r0.y; r[2] = r0.z; r[3] = r0.w;
-            r[4] = r1.x; r[5] = r1.y; r[6] = r1.z; r[7] = r1.w;
-            hash_pair(a.kind, l, r, o);
-            uint4 *po = reinterpret_cast<uint4 *>(a.out[0] + j * 8);
-            po[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            po[1] = make_uint4(o[4], o[5], o[6], o[7]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
-        }
-    }
-    __syncthreads();
-    uint64_t cta_nodes = n_lvl < 256 ? n_lvl : 256;  // nodes of this CTA at the current level
-    for (int lv = 1; lv < a.k; ++lv) {
-        const uint64_t half = cta_nodes >> 1;
-        const bool active = (uint64_t)t < half;
+    // every level through the same code: the first reads its pairs from
+    // global memory, the others from shared memory
+    uint64_t cta_nodes = min(a.n_in >> 1, (uint64_t)256);  // nodes of this CTA at the level
+    for (int lv = 0; lv < a.k; ++lv) {
+        const bool active = (uint64_t)t < cta_nodes &&
+                            u * (256 >> lv) + t < (a.n_in >> (lv + 1));
         uint32_t o[8];
         if (active) {
-            hash_pair(a.kind, nodes[2 * t], nodes[2 * t + 1], o);
-            const uint64_t j = u * (256 >> lv) + t;
-            uint4 *po = reinterpret_cast<uint4 *>(a.out[lv] + j * 8);
+            uint32_t l[8], r[8];
+            if (lv == 0) {
+                const uint4 *pl = reinterpret_cast<const uint4 *>(a.in + (u * 512 + 2 * t) * 8);
+                const uint4 l0 = pl[0], l1 = pl[1], r0 = pl[2], r1 = pl[3];
+                l[0] = l0.x; l[1] = l0.y; l[2] = l0.z; l[3] = l0.w;
+                l[4] = l1.x; l[5] = l1.y; l[6] = l1.z; l[7] = l1.w;
+                r[0] = r0.x; r[1] = r0.y; r[2] = r0.z; r[3] = r0.w;
+                r[4] = r1.x; r[5] = r1.y; r[6] = r1.z; r[7] = r1.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    l[i] = nodes[2 * t][i];
+                    r[i] = nodes[2 * t + 1][i];
+                }
+            }
+            hash_pair(a.kind, l, r, o);
+            uint4 *po = reinterpret_cast<uint4 *>(a.out[lv] + (u * (256 >> lv) + t) * 8);
             po[0] = make_uint4(o[0], o[1], o[2], o[3]);
             po[1] = make_uint4(o[4], o[5], o[6], o[7]);
         }
@@ -191,23 +179,20 @@ __device__ __forceinline__ void merkle_levels_body(const LevelsArgs &a, uint64_t
             for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
         }
         __syncthreads();
-        cta_nodes = half;
+        cta_nodes >>= 1;
     }
 }
 
-// SHA-256 leaves: one thread per leaf, sequential over the row.
-// Body: leaves first, first + step, .. below n_leaves.
-__device__ __forceinline__ void sha_leaves_body(const uint4 *cw, int log_lanes, uint64_t n_leaves,
-                                                uint32_t *tree_leaves, uint64_t first,
-                                                uint64_t step) {
-    for (uint64_t leaf = first; leaf < n_leaves; leaf += step) {
-        const uint64_t elems = (uint64_t)1 << log_lanes;
-        const uint64_t bytes = elems * 16;
-        const uint4 *p = cw + leaf * elems;
-        uint32_t st[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
-                          0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
-        const uint64_t full = bytes / 64;  // full 64-byte blocks
-        for (uint64_t blk = 0; blk < full; ++blk) {
+// SHA-256 of one row of 16 * 2^log_lanes bytes; pad: sha_pad_kw of its bit
+// length (read from 4 lanes up, where the row ends on a block boundary).
+template <bool ROLLED>
+__device__ __forceinline__ void sha_leaf(const uint4 *p, int log_lanes, const ShaWords &pad,
+                                         uint32_t out[8]) {
+    uint32_t st[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
+                      0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
+    if (log_lanes >= 2) {
+        const uint64_t blocks = (uint64_t)1 << (log_lanes - 2);
+        for (uint64_t blk = 0; blk < blocks; ++blk) {
             uint32_t w[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -217,32 +202,43 @@ __device__ __forceinline__ void sha_leaves_body(const uint4 *cw, int log_lanes, 
                 w[4 * q + 2] = bswap32(v.z);
                 w[4 * q + 3] = bswap32(v.w);
             }
-            sha256_compress(st, w);
+            sha256_compress<ROLLED>(st, w);
         }
-        // tail: remaining (bytes % 64) bytes, then 0x80, zeros, 64-bit length
-        const uint32_t rem = (uint32_t)(bytes - full * 64);  // 0, 16, 32 or 48
+        sha256_compress_kw<ROLLED>(st, pad);
+    } else {
+        // one block: 16 or 32 bytes, 0x80, zeros, the length
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = 0;
-        for (uint32_t e = 0; e < rem / 16; ++e) {
-            const uint4 v = p[full * 4 + e];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            if (e >> log_lanes) break;
+            const uint4 v = p[e];
             w[4 * e] = bswap32(v.x);
             w[4 * e + 1] = bswap32(v.y);
             w[4 * e + 2] = bswap32(v.z);
             w[4 * e + 3] = bswap32(v.w);
         }
-        w[rem / 4] = 0x80000000u;
-        const uint64_t bitlen = bytes * 8;
-        if (rem + 9 > 64) {
-            sha256_compress(st, w);
+        if (log_lanes == 0) w[4] = 0x80000000u;
+        else w[8] = 0x80000000u;
+        w[15] = 128u << log_lanes;
+        sha256_compress<ROLLED>(st, w);
+    }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) w[i] = 0;
-        }
-        w[14] = (uint32_t)(bitlen >> 32);
-        w[15] = (uint32_t)bitlen;
-        sha256_compress(st, w);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) tree_leaves[leaf * 8 + i] = bswap32(st[i]);
+    for (int i = 0; i < 8; ++i) out[i] = bswap32(st[i]);
+}
+
+// SHA-256 leaves: one thread per leaf, sequential over the row.
+// Body: leaves first, first + step, .. below n_leaves.
+__device__ __forceinline__ void sha_leaves_body(const uint4 *cw, int log_lanes, uint64_t n_leaves,
+                                                uint32_t *tree_leaves, const ShaWords &pad,
+                                                uint64_t first, uint64_t step) {
+    for (uint64_t leaf = first; leaf < n_leaves; leaf += step) {
+        uint32_t o[8];
+        sha_leaf<false>(cw + (leaf << log_lanes), log_lanes, pad, o);
+        uint4 *po = reinterpret_cast<uint4 *>(tree_leaves + leaf * 8);
+        po[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        po[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
 }
 

@@ -68,6 +68,7 @@ struct PStep {
     uint32_t *leaves = nullptr;
     uint64_t count = 0;     // chunks (B3_CHUNKED)
     uint64_t chunk0 = 0;
+    ShaWords pad{};         // SHA: the leaf's padding block
     LevelsArgs lv{};
     const uint32_t *root_src = nullptr;  // last step of a commit: its root node
     uint32_t *root_dst = nullptr;
@@ -201,7 +202,7 @@ __device__ __noinline__ void leaves_item(const PStep *st, uint64_t b, uint64_t e
     } else if (st->kind == PK_B3_SMALL) {
         b3_leaves_small_body(cw, st->log_lanes, e, leaves, b + threadIdx.x, blockDim.x);
     } else {
-        sha_leaves_body(cw, st->log_lanes, e, leaves, b + threadIdx.x, blockDim.x);
+        sha_leaves_body(cw, st->log_lanes, e, leaves, st->pad, b + threadIdx.x, blockDim.x);
     }
 }
 
@@ -491,6 +492,7 @@ int merkle_steps(StepBuilder &sb, const uint4 *cw, uint8_t *d_tree, uint32_t *ro
         st.cw = cw;
         st.leaves = tree;
         st.log_lanes = s.log_lanes;
+        st.pad = sha_pad_kw(s.leaf_bytes() * 8);
         sb.out.push_back(st);
     }
     // parent levels, nine per step (as launch_levels)
