@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "bz_internal.h"
+#include "chain.cuh"
 #include "hash.cuh"
 #include "merkle_kernels.cuh"
 
@@ -25,12 +26,14 @@ __global__ void __launch_bounds__(256) b3_leaves_chunked(const uint4 *cw, uint64
                                                          uint32_t *tree_leaves, int log_c,
                                                          uint64_t chunk0) {
     __shared__ uint32_t cvs[256][9];  // padded rows
+    chain_wait();
     b3_leaves_chunked_body(cw, n_chunks, tree_leaves, log_c, chunk0,
                            (uint64_t)blockIdx.x * blockDim.x, cvs);
 }
 
 __global__ void b3_leaves_small(const uint4 *cw, int log_lanes, uint64_t n_leaves,
                                 uint32_t *tree_leaves) {
+    chain_wait();
     b3_leaves_small_body(cw, log_lanes, n_leaves, tree_leaves,
                          (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                          (uint64_t)gridDim.x * blockDim.x);
@@ -38,12 +41,14 @@ __global__ void b3_leaves_small(const uint4 *cw, int log_lanes, uint64_t n_leave
 
 __global__ void __launch_bounds__(256) merkle_levels(LevelsArgs a) {
     __shared__ uint32_t nodes[256][9];
+    chain_wait();
     merkle_levels_body(a, blockIdx.x, nodes);
 }
 
 __global__ void __launch_bounds__(128) sha_leaves(const uint4 *cw, int log_lanes,
                                                   uint64_t n_leaves, uint32_t *tree_leaves,
                                                   const __grid_constant__ ShaWords pad) {
+    chain_wait();
     sha_leaves_body(cw, log_lanes, n_leaves, tree_leaves, pad,
                     (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
@@ -61,6 +66,7 @@ __global__ void __launch_bounds__(kTreeSmallMax) b3_tree_small(const uint4 *cw, 
                                                                uint32_t n_leaves,
                                                                uint32_t *tree) {
     __shared__ uint32_t nodes[kTreeSmallMax][9];  // padded rows
+    chain_wait();
     const uint32_t t = threadIdx.x;
     uint32_t cv[8];
 #pragma unroll
@@ -117,6 +123,7 @@ __global__ void __launch_bounds__(kShaTreeSmallMax) sha_tree_small(
     const uint4 *cw, int log_lanes, uint32_t n_leaves, uint32_t *tree,
     const __grid_constant__ ShaWords pad) {
     __shared__ uint32_t nodes[kShaTreeSmallMax][9];  // padded rows
+    chain_wait();
     const uint32_t t = threadIdx.x;
     uint32_t o[8];
     sha_leaf<true>(cw + ((uint64_t)t << log_lanes), log_lanes, pad, o);
@@ -140,6 +147,7 @@ __global__ void __launch_bounds__(kShaTreeSmallMax) sha_tree_small(
 // Generic BLAKE3 chunk CVs into scratch (leaves longer than 256 chunks).
 __global__ void b3_chunk_cvs(const uint4 *cw, uint64_t n_chunks, int log_c, uint32_t *out,
                              uint64_t chunk0) {
+    chain_wait();
     const uint64_t chunk = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (chunk >= n_chunks) return;
     const uint64_t c_in_leaf = chunk0 + (chunk & ((1ull << log_c) - 1));
@@ -196,18 +204,18 @@ int launch_leaves_range(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint
     uint32_t *leaves = tree + p0 * 8;
     if (s.hash_kind == 1) {
         if (s.log_lanes < 6) {
-            b3_leaves_small<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(cw, s.log_lanes, n,
-                                                                      leaves);
+            launch_chained(b3_leaves_small, (unsigned)((n + 255) / 256), 256, 0, st, cw,
+                           s.log_lanes, n, leaves);
         } else {
             const int log_c = s.log_lanes - 6;
             const uint64_t n_chunks = n << log_c;
             const unsigned t = leaf_threads(n_chunks, log_c, num_sms);
-            b3_leaves_chunked<<<(unsigned)((n_chunks + t - 1) / t), t, 0, st>>>(
-                cw, n_chunks, leaves, log_c, s.chunk0);
+            launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, cw,
+                           n_chunks, leaves, log_c, s.chunk0);
         }
     } else {
-        sha_leaves<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(cw, s.log_lanes, n, leaves,
-                                                                sha_pad_kw(s.leaf_bytes() * 8));
+        launch_chained(sha_leaves, (unsigned)((n + 127) / 128), 128, 0, st, cw, s.log_lanes, n,
+                       leaves, sha_pad_kw(s.leaf_bytes() * 8));
     }
     return 1;
 }
@@ -240,7 +248,7 @@ static int launch_levels(uint32_t *tree, uint64_t n_leaves, int kind, cudaStream
             cnt >>= 1;
         }
         const uint64_t ctas = (n_in + 511) / 512;
-        merkle_levels<<<(unsigned)ctas, 256, 0, st>>>(a);
+        launch_chained(merkle_levels, (unsigned)ctas, 256, 0, st, a);
         if (log) log->mark("merkle_levels");
         ++launches;
         // advance: the last produced level becomes the next input
@@ -265,30 +273,30 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
     int launches = 0;
     if (s.hash_kind == 1) {
         if (s.log_lanes < 6 && n_leaves <= (uint64_t)kTreeSmallMax && n_leaves >= 2) {
-            b3_tree_small<<<1, (unsigned)n_leaves, 0, st>>>(d_cw, s.log_lanes,
-                                                            (uint32_t)n_leaves, tree);
+            launch_chained(b3_tree_small, 1, (unsigned)n_leaves, 0, st, d_cw, s.log_lanes,
+                           (uint32_t)n_leaves, tree);
             mark("b3_tree_small");
             return 1;
         }
         if (s.log_lanes < 6) {
-            b3_leaves_small<<<(unsigned)((n_leaves + 255) / 256), 256, 0, st>>>(d_cw, s.log_lanes,
-                                                                             n_leaves, tree);
+            launch_chained(b3_leaves_small, (unsigned)((n_leaves + 255) / 256), 256, 0, st, d_cw,
+                           s.log_lanes, n_leaves, tree);
             mark("b3_leaves_small");
             ++launches;
         } else if (s.log_lanes <= 14) {
             const int log_c = s.log_lanes - 6;
             const uint64_t n_chunks = n_leaves << log_c;
             const unsigned t = leaf_threads(n_chunks, log_c, num_sms);
-            b3_leaves_chunked<<<(unsigned)((n_chunks + t - 1) / t), t, 0, st>>>(
-                d_cw, n_chunks, tree, log_c, s.chunk0);
+            launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, d_cw,
+                           n_chunks, tree, log_c, s.chunk0);
             mark("b3_leaves_chunked");
             ++launches;
         } else {
             const int log_c = s.log_lanes - 6;
             const uint64_t n_chunks = n_leaves << log_c;
             uint32_t *cvs = reinterpret_cast<uint32_t *>(d_scratch);
-            b3_chunk_cvs<<<(unsigned)((n_chunks + 255) / 256), 256, 0, st>>>(d_cw, n_chunks,
-                                                                           log_c, cvs, s.chunk0);
+            launch_chained(b3_chunk_cvs, (unsigned)((n_chunks + 255) / 256), 256, 0, st, d_cw,
+                           n_chunks, log_c, cvs, s.chunk0);
             mark("b3_chunk_cvs");
             ++launches;
             // reduce chunk CVs to leaf CVs: levels inside the scratch area,
@@ -303,7 +311,7 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
                 a.k = 1;
                 a.kind = 1;
                 a.out[0] = (lv == log_c - 1) ? tree : bufs[cur ^ 1];
-                merkle_levels<<<(unsigned)((n + 511) / 512), 256, 0, st>>>(a);
+                launch_chained(merkle_levels, (unsigned)((n + 511) / 512), 256, 0, st, a);
                 mark("merkle_levels");
                 ++launches;
                 n >>= 1;
@@ -313,13 +321,13 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
     } else {
         const ShaWords pad = sha_pad_kw(s.leaf_bytes() * 8);
         if (n_leaves <= (uint64_t)kShaTreeSmallMax) {
-            sha_tree_small<<<1, (unsigned)n_leaves, 0, st>>>(d_cw, s.log_lanes,
-                                                             (uint32_t)n_leaves, tree, pad);
+            launch_chained(sha_tree_small, 1, (unsigned)n_leaves, 0, st, d_cw, s.log_lanes,
+                           (uint32_t)n_leaves, tree, pad);
             mark("sha_tree_small");
             return 1;
         }
-        sha_leaves<<<(unsigned)((n_leaves + 127) / 128), 128, 0, st>>>(d_cw, s.log_lanes,
-                                                                       n_leaves, tree, pad);
+        launch_chained(sha_leaves, (unsigned)((n_leaves + 127) / 128), 128, 0, st, d_cw,
+                       s.log_lanes, n_leaves, tree, pad);
         mark("sha_leaves");
         ++launches;
     }

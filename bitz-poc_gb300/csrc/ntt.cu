@@ -40,6 +40,7 @@
 #include <string>
 
 #include "bz_internal.h"
+#include "chain.cuh"
 #include "gf128.cuh"
 #include "t16.cuh"
 #include "t8.cuh"
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(THREADS, 1) ntt_table_pass(TablePassArgs a) {
     __shared__ uint4 tw_buf[kTwWindow * (LAYERS == 2 ? 3 : 1)];
     __shared__ uint64_t win[2];
     __shared__ int tz[3];
+    chain_wait();
     uint64_t c_beg, c_end;
     cta_chunks(a.n_tasks, c_beg, c_end);
     table_pass_body<LAYERS>(a, c_beg, c_end, smem, tw_buf, win, tz);
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(THREADS, MINB) ntt_table_pass2_pf(TablePassArg
     extern __shared__ uint4 smem[];
     __shared__ uint4 tw_buf[kTwWindow * 3];
     __shared__ uint64_t win[2];
+    chain_wait();
     uint64_t c_beg, c_end;
     cta_chunks(a.n_tasks, c_beg, c_end);
     table_pass2_pf_body<WO, WAB>(a, c_beg, c_end, smem, tw_buf, win);
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(512, 1) ntt_pass8(TablePassArgs a) {
     extern __shared__ uint4 smem[];
     __shared__ uint4 tw_buf[kTw8Window * 7];
     __shared__ uint64_t win[2];
+    chain_wait();
     uint64_t c_beg, c_end;
     cta_chunks(a.n_tasks, c_beg, c_end);
     pass8_body<W0, W1, W2>(a, c_beg, c_end, reinterpret_cast<char *>(smem), tw_buf, win);
@@ -201,18 +205,21 @@ __global__ void __launch_bounds__(512, 1) ntt_pass8_first(TablePassArgs a) {
     extern __shared__ uint4 smem[];
     __shared__ uint4 tw_buf[kTw8Window * 7];
     __shared__ uint64_t win[2];
+    chain_wait();
     pass8_body<4, 4, 4>(a, blockIdx.x, a.n_tasks / blockDim.x, reinterpret_cast<char *>(smem),
                         tw_buf, win, gridDim.x);
 }
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(256) ntt_deep_pass(DeepArgs a) {
+    chain_wait();
     deep_pass_body<D, MODE>(a, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, a.n_tasks,
                             (uint64_t)gridDim.x * blockDim.x);
 }
 
 __global__ void ntt_generic_layer(const uint4 *src, uint4 *dst, const uint4 *tw, int ell,
                                   int layer, int log_lanes, int src_pos_bits, uint64_t n_tasks) {
+    chain_wait();
     generic_layer_body(src, dst, tw, ell, layer, log_lanes, src_pos_bits,
                        (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n_tasks,
                        (uint64_t)gridDim.x * blockDim.x);
@@ -227,6 +234,7 @@ __global__ void ntt_generic_layer(const uint4 *src, uint4 *dst, const uint4 *tw,
 template <int DT, int DN, int MODE>
 __global__ void __launch_bounds__(512, 1) ntt_tail_pass(DeepArgs a) {
     extern __shared__ uint4 smem[];
+    chain_wait();
     constexpr int NT = DT == 2 ? 3 : 1;
     constexpr int P = 1 << (DT + DN);
     uint4 *tbl = smem;
@@ -311,6 +319,7 @@ __global__ void __launch_bounds__(512) ntt_small_kernel(const uint4 *msg, uint4 
     const uint32_t P = 1u << ell;
     const uint64_t lane = blockIdx.x;
     const uint32_t msg_mask = (1u << msg_pos_bits) - 1;
+    chain_wait();
     for (uint32_t p = threadIdx.x; p < P; p += blockDim.x)
         col[p] = msg[((uint64_t)(p & msg_mask) << log_lanes) | lane];
     for (int layer = r; layer < ell; ++layer) {
@@ -343,6 +352,7 @@ bool small_ntt_ok(const Shape &s) {
 
 // cw[rep * N + i] = msg[i] for every replica (commit.rs:239-258).
 __global__ void replicate_fill(const uint4 *msg, uint4 *cw, uint64_t msg_words, int reps) {
+    chain_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < msg_words;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint4 v = __ldcs(msg + i);
@@ -427,16 +437,17 @@ static bool launch_pass8(const Shape &s, int layer, const uint4 *src, int src_bi
     const uint64_t nb = (uint64_t)1 << layer;
     if (layer == s.log_inv_rate && key == 444 && waves == 1 &&
         4 * (a.n_tasks / 512) >= 3 * nb * (nb - 1) * grid) {
-        ntt_pass8_first<<<grid, 512, kPass8Smem, st>>>(a);
+        launch_chained(ntt_pass8_first, grid, 512, kPass8Smem, st, a);
         return false;
     }
-#define BZ_P8_CASE(A, B, C) \
-    case A * 100 + B * 10 + C: ntt_pass8<A, B, C><<<grid, 512, kPass8Smem, st>>>(a); break
+#define BZ_P8_CASE(A, B, C)                                                    \
+    case A * 100 + B * 10 + C:                                                 \
+        launch_chained(ntt_pass8<A, B, C>, grid, 512, kPass8Smem, st, a); break
     switch (key) {
         BZ_P8_CASE(4, 4, 2); BZ_P8_CASE(4, 4, 1); BZ_P8_CASE(4, 2, 2); BZ_P8_CASE(4, 2, 1);
         BZ_P8_CASE(4, 1, 1); BZ_P8_CASE(2, 2, 2); BZ_P8_CASE(2, 2, 1); BZ_P8_CASE(2, 1, 1);
         BZ_P8_CASE(1, 1, 1);
-        default: ntt_pass8<4, 4, 4><<<grid, 512, kPass8Smem, st>>>(a); break;
+        default: launch_chained(ntt_pass8<4, 4, 4>, grid, 512, kPass8Smem, st, a); break;
     }
 #undef BZ_P8_CASE
     return w2 < 4;
@@ -444,17 +455,17 @@ static bool launch_pass8(const Shape &s, int layer, const uint4 *src, int src_bi
 
 template <int D>
 static void launch_deep(const DeepArgs &a, int mode, unsigned grid, cudaStream_t st) {
-    if (mode == 1) ntt_deep_pass<D, 1><<<grid, 256, 0, st>>>(a);
-    else if (mode == 2) ntt_deep_pass<D, 2><<<grid, 256, 0, st>>>(a);
-    else ntt_deep_pass<D, 0><<<grid, 256, 0, st>>>(a);
+    if (mode == 1) launch_chained(ntt_deep_pass<D, 1>, grid, 256, 0, st, a);
+    else if (mode == 2) launch_chained(ntt_deep_pass<D, 2>, grid, 256, 0, st, a);
+    else launch_chained(ntt_deep_pass<D, 0>, grid, 256, 0, st, a);
 }
 
 template <int DT, int DN>
 static void launch_tail(const DeepArgs &a, int mode, unsigned grid, cudaStream_t st) {
     const size_t sm = table_smem(DT);
-    if (mode == 1) ntt_tail_pass<DT, DN, 1><<<grid, 512, sm, st>>>(a);
-    else if (mode == 2) ntt_tail_pass<DT, DN, 2><<<grid, 512, sm, st>>>(a);
-    else ntt_tail_pass<DT, DN, 0><<<grid, 512, sm, st>>>(a);
+    if (mode == 1) launch_chained(ntt_tail_pass<DT, DN, 1>, grid, 512, sm, st, a);
+    else if (mode == 2) launch_chained(ntt_tail_pass<DT, DN, 2>, grid, 512, sm, st, a);
+    else launch_chained(ntt_tail_pass<DT, DN, 0>, grid, 512, sm, st, a);
 }
 
 // Whether a table pass runs with compact tables (ntt_table_pass2_pf with
@@ -490,25 +501,27 @@ int launch_table_pass(const Shape &s, int layer, int layers, const uint4 *src, i
         const int wo = narrow_class(twiddle_bits(ell, layer));
         const int wab = narrow_class(twiddle_bits(ell, layer + 1));
         const size_t sm = pf_smem(wo, wab);
-        if (wab == 1 && wo == 1) ntt_table_pass2_pf<512, 1, 1, 1><<<grid, 512, sm, st>>>(a);
-        else if (wab == 1 && wo == 2) ntt_table_pass2_pf<512, 1, 2, 1><<<grid, 512, sm, st>>>(a);
-        else if (wab == 1) ntt_table_pass2_pf<512, 1, 4, 1><<<grid, 512, sm, st>>>(a);
-        else if (wo == 2) ntt_table_pass2_pf<512, 1, 2, 2><<<grid, 512, sm, st>>>(a);
-        else ntt_table_pass2_pf<512, 1, 4, 2><<<grid, 512, sm, st>>>(a);
+        if (wab == 1 && wo == 1) launch_chained(ntt_table_pass2_pf<512, 1, 1, 1>, grid, 512, sm,
+                                                st, a);
+        else if (wab == 1 && wo == 2) launch_chained(ntt_table_pass2_pf<512, 1, 2, 1>, grid, 512,
+                                                     sm, st, a);
+        else if (wab == 1) launch_chained(ntt_table_pass2_pf<512, 1, 4, 1>, grid, 512, sm, st, a);
+        else if (wo == 2) launch_chained(ntt_table_pass2_pf<512, 1, 2, 2>, grid, 512, sm, st, a);
+        else launch_chained(ntt_table_pass2_pf<512, 1, 4, 2>, grid, 512, sm, st, a);
     } else if (prefetch && layers == 2) {
         const size_t sm = pf_smem(4, 4);
         if (threads == 256 && lean)
-            ntt_table_pass2_pf<256, 2, 4, 4><<<grid, 256, sm, st>>>(a);
+            launch_chained(ntt_table_pass2_pf<256, 2, 4, 4>, grid, 256, sm, st, a);
         else if (threads == 256)
-            ntt_table_pass2_pf<256, 1, 4, 4><<<grid, 256, sm, st>>>(a);
+            launch_chained(ntt_table_pass2_pf<256, 1, 4, 4>, grid, 256, sm, st, a);
         else
-            ntt_table_pass2_pf<512, 1, 4, 4><<<grid, 512, sm, st>>>(a);
+            launch_chained(ntt_table_pass2_pf<512, 1, 4, 4>, grid, 512, sm, st, a);
     } else if (threads == 256) {
-        if (layers == 2) ntt_table_pass<2, 256><<<grid, 256, table_smem(2), st>>>(a);
-        else ntt_table_pass<1, 256><<<grid, 256, table_smem(1), st>>>(a);
+        if (layers == 2) launch_chained(ntt_table_pass<2, 256>, grid, 256, table_smem(2), st, a);
+        else launch_chained(ntt_table_pass<1, 256>, grid, 256, table_smem(1), st, a);
     } else {
-        if (layers == 2) ntt_table_pass<2, 512><<<grid, 512, table_smem(2), st>>>(a);
-        else ntt_table_pass<1, 512><<<grid, 512, table_smem(1), st>>>(a);
+        if (layers == 2) launch_chained(ntt_table_pass<2, 512>, grid, 512, table_smem(2), st, a);
+        else launch_chained(ntt_table_pass<1, 512>, grid, 512, table_smem(1), st, a);
     }
     return 1;
 }
@@ -546,24 +559,24 @@ int launch_ntt(const Shape &s, uint32_t schedule, const uint4 *d_msg, uint4 *d_c
     const uint4 *src = d_msg;
     int src_bits = b;  // message positions are the low b bits of a codeword position
     if (b == 0) {
-        replicate_fill<<<grid_for(s.msg_words(), 256, num_sms, 8), 256, 0, st>>>(
-            d_msg, d_cw, s.msg_words(), 1 << r);
+        launch_chained(replicate_fill, grid_for(s.msg_words(), 256, num_sms, 8), 256, 0, st, d_msg,
+                       d_cw, s.msg_words(), 1 << r);
         mark("replicate_fill");
         return 1;
     }
     const bool generic = (schedule & SCHED_GENERIC) != 0;
     if (!generic && small_ntt_ok(s)) {
         const unsigned threads = (unsigned)std::min<uint64_t>(P / 2, 512);
-        ntt_small_kernel<<<1u << L, threads, P * sizeof(uint4), st>>>(d_msg, d_cw, d_tw, ell, r,
-                                                                      L, b);
+        launch_chained(ntt_small_kernel, 1u << L, threads, P * sizeof(uint4), st, d_msg, d_cw,
+                       d_tw, ell, r, L, b);
         mark("ntt_small");
         return 1;
     }
     if (generic) {
         for (int layer = r; layer < ell; ++layer) {
             const uint64_t n_tasks = ((uint64_t)1 << (ell - 1)) << L;
-            ntt_generic_layer<<<grid_for(n_tasks, 256, num_sms, 8), 256, 0, st>>>(
-                src, d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
+            launch_chained(ntt_generic_layer, grid_for(n_tasks, 256, num_sms, 8), 256, 0, st, src,
+                           d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
             mark("ntt_generic_layer");
             ++launches;
             src = d_cw;
@@ -595,8 +608,8 @@ int launch_ntt(const Shape &s, uint32_t schedule, const uint4 *d_msg, uint4 *d_c
         auto generic_layers = [&](int layers) {
             const uint64_t n_tasks = ((uint64_t)1 << (ell - 1)) << L;
             for (int k = 0; k < layers; ++k) {
-                ntt_generic_layer<<<grid_for(n_tasks, 256, num_sms, 8), 256, 0, st>>>(
-                    src, d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
+                launch_chained(ntt_generic_layer, grid_for(n_tasks, 256, num_sms, 8), 256, 0, st,
+                               src, d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
                 done("ntt_generic_layer", 1);
             }
         };
@@ -703,8 +716,8 @@ int launch_ntt(const Shape &s, uint32_t schedule, const uint4 *d_msg, uint4 *d_c
         if (!table_pass_ok(ell, layer, layers, L, log_threads)) {
             // too few tasks per block for table passes: generic single layers
             const uint64_t n_tasks = ((uint64_t)1 << (ell - 1)) << L;
-            ntt_generic_layer<<<grid_for(n_tasks, 256, num_sms, 8), 256, 0, st>>>(
-                src, d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
+            launch_chained(ntt_generic_layer, grid_for(n_tasks, 256, num_sms, 8), 256, 0, st, src,
+                           d_cw, d_tw, ell, layer, L, src_bits, n_tasks);
             mark("ntt_generic_layer");
             ++launches;
             src = d_cw;

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "bz_internal.h"
+#include "chain.cuh"
 #include "gf128.cuh"
 #include "ntt_group.cuh"
 
@@ -77,7 +78,8 @@ int launch_group16(const Shape &s, const uint4 *src, int src_bits, uint4 *dst, c
     const int w3 = narrow_class(twiddle_bits(ell, ell - 4));
     const int w2 = narrow_class(twiddle_bits(ell, ell - 3));
     const int w1 = narrow_class(twiddle_bits(ell, ell - 2));
-#define BZ_G_RUN(A, B, C, D) ntt_group16<A, B, C, D><<<grid, 1u << t, kGroup16Smem, st>>>(a)
+#define BZ_G_RUN(A, B, C, D) \
+    launch_chained(ntt_group16<A, B, C, D>, grid, 1u << t, kGroup16Smem, st, a)
     if (w3 <= 2) BZ_G_RUN(2, 2, 1, 1);
     else if (w2 <= 2 && w1 == 1) BZ_G_RUN(4, 2, 1, 1);
     else if (w2 <= 2) BZ_G_RUN(4, 2, 2, 1);
@@ -100,7 +102,7 @@ int launch_group8(const Shape &s, int depth, const uint4 *src, int src_bits, uin
     const unsigned grid =
         (unsigned)std::min<uint64_t>(a.n_tasks >> t, (uint64_t)num_sms * 2 * waves);
     if (depth > 0) {
-        ntt_group8<4, 4, 4, 4><<<grid, 1u << t, kGroup8Smem, st>>>(a);
+        launch_chained(ntt_group8<4, 4, 4, 4>, grid, 1u << t, kGroup8Smem, st, a);
         return 1;
     }
     const int w2 = narrow_class(twiddle_bits(ell, ell - 3));
@@ -109,8 +111,8 @@ int launch_group8(const Shape &s, int depth, const uint4 *src, int src_bits, uin
     // 4 (t - L) <= 32 bits at depth 2, which the 64-bit product holds
 #define BZ_G_RUN(A, B, C)                                                                     \
     {                                                                                         \
-        if (L >= t) ntt_group8<A, B, C, 0><<<grid, 1u << t, kGroup8Smem, st>>>(a);            \
-        else ntt_group8<A, B, C, 2><<<grid, 1u << t, kGroup8Smem, st>>>(a);                   \
+        if (L >= t) launch_chained(ntt_group8<A, B, C, 0>, grid, 1u << t, kGroup8Smem, st, a);\
+        else launch_chained(ntt_group8<A, B, C, 2>, grid, 1u << t, kGroup8Smem, st, a);       \
     }
     if (w2 <= 2 && w1 == 1) BZ_G_RUN(2, 1, 1)
     else if (w2 <= 2) BZ_G_RUN(2, 2, 1)

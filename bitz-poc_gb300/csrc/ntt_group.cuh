@@ -327,7 +327,6 @@ __device__ __forceinline__ void group_pass_body(const GroupPassArgs &a, uint64_t
             }
         }
     }
-    int64_t cur = -1;
     auto load = [&](uint64_t c, uint4 (&v)[1 << K]) {
         const uint64_t task = c * blockDim.x + threadIdx.x;
         const uint64_t pbase = ((task >> log_task_per_b) << (depth + K)) +
@@ -338,6 +337,27 @@ __device__ __forceinline__ void group_pass_body(const GroupPassArgs &a, uint64_t
             v[i] = __ldcs(a.src + (((p & src_mask) << a.log_lanes) | (task & lanes_mask)));
         }
     };
+    auto build = [&](uint64_t B0) {
+        constexpr int n0 = build_items<W0>(), n1 = build_items<W1>(), n2 = build_items<W2>();
+        constexpr int n3 = K > 3 ? build_items<W3>() : 0;
+        for (int u = threadIdx.x; u < n0 + n1 + n2 + n3; u += blockDim.x) {
+            const int j = u < n0 ? 0 : u < n0 + n1 ? 1 : u < n0 + n1 + n2 ? 2 : 3;
+            const uint4 t = __ldg(a.tw + ((uint64_t)1 << (top + j)) + (B0 << j));
+            if (j == 0) group_build_item<W0, group_pitch<K>(0)>(tbl + group_slot(0), t, u);
+            else if (j == 1)
+                group_build_item<W1, group_pitch<K>(1)>(tbl + group_slot(1), t, u - n0);
+            else if (j == 2)
+                group_build_item<W2, group_pitch<K>(2)>(tbl + group_slot(2), t, u - n0 - n1);
+            else if constexpr (K > 3)
+                group_build_item<W3, group_pitch<K>(3)>(tbl + group_slot(3), t,
+                                                        u - n0 - n1 - n2);
+        }
+    };
+    // the first chunk's tables are built ahead of the wait; its barrier below
+    build((c_beg * blockDim.x) >> log_task_per_b);
+    chain_wait();
+    uint64_t cur = (c_beg * blockDim.x) >> log_task_per_b;
+    bool built = true;  // since the last barrier
     uint4 nxt[1 << K];
     if (PF && c_beg < c_end) load(c_beg, nxt);
     for (uint64_t c = c_beg; c < c_end; ++c) {
@@ -354,22 +374,14 @@ __device__ __forceinline__ void group_pass_body(const GroupPassArgs &a, uint64_t
             load(c, v);
         }
         const uint64_t B0 = (c * blockDim.x) >> log_task_per_b;  // uniform
-        if ((int64_t)B0 != cur) {
+        if (B0 != cur) {
             __syncthreads();  // every lookup into the previous tables is done
-            constexpr int n0 = build_items<W0>(), n1 = build_items<W1>(), n2 = build_items<W2>();
-            constexpr int n3 = K > 3 ? build_items<W3>() : 0;
-            for (int u = threadIdx.x; u < n0 + n1 + n2 + n3; u += blockDim.x) {
-                const int j = u < n0 ? 0 : u < n0 + n1 ? 1 : u < n0 + n1 + n2 ? 2 : 3;
-                const uint4 t = __ldg(a.tw + ((uint64_t)1 << (top + j)) + (B0 << j));
-                if (j == 0) group_build_item<W0, group_pitch<K>(0)>(tbl + group_slot(0), t, u);
-                else if (j == 1) group_build_item<W1, group_pitch<K>(1)>(tbl + group_slot(1), t, u - n0);
-                else if (j == 2) group_build_item<W2, group_pitch<K>(2)>(tbl + group_slot(2), t, u - n0 - n1);
-                else if constexpr (K > 3)
-                    group_build_item<W3, group_pitch<K>(3)>(tbl + group_slot(3), t, u - n0 - n1 - n2);
-            }
-            __syncthreads();
-            cur = (int64_t)B0;
+            build(B0);
+            built = true;
+            cur = B0;
         }
+        if (built) __syncthreads();
+        built = false;
         group_layer<K, 0, W0, EW>(v, lc, tbl + group_slot(0), eb[0],
                                   a.tw + ((uint64_t)1 << top));
         group_layer<K, 1, W1, EW>(v, lc, tbl + group_slot(1), eb[1],

@@ -168,7 +168,9 @@ int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out) {
     std::vector<uint64_t> heap = twiddle_heap(ell);
     void *d = nullptr;
     BZ_CUDA(ctx, cudaMalloc(&d, heap.size() * 8));
+    // (the copy of a pageable buffer may still be in flight when it returns)
     BZ_CUDA(ctx, cudaMemcpy(d, heap.data(), heap.size() * 8, cudaMemcpyHostToDevice));
+    BZ_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
     ctx->twiddles[ell] = (const uint4 *)d;
     *out = (const uint4 *)d;
     return BZ_OK;
