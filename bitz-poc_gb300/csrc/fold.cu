@@ -11,8 +11,10 @@
 #include <algorithm>
 
 #include "bz_internal.h"
+#include "chain.cuh"
 #include "gf128.cuh"
 #include "t16.cuh"
+#include "t8.cuh"
 
 namespace bz {
 
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(256) round_msg_kernel(const uint4 *f, const ui
 // Final XOR of per-CTA partials and the single reduction: out = {u0, u2}.
 __global__ void __launch_bounds__(kFinishThreads) finish_msg_kernel(const uint64_t *partials,
                                                                     int n, uint64_t *out) {
+    chain_wait();
     finish_msg_body(partials, n, out);
 }
 
@@ -299,7 +302,7 @@ int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, u
         fold_and_msg_kernel<false><<<grid, 256, kRTableSmem, st>>>(d_f, d_b, half, r, d_nf, d_nb,
                                                                    d_partials, mb, RGate{});
     if (post) return 1;
-    finish_msg_kernel<<<1, kFinishThreads, 0, st>>>(d_partials, grid, d_msg_out);
+    launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
 }
 
@@ -311,7 +314,7 @@ int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_p
     if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
     round_msg_kernel<<<grid, 256, 0, st>>>(d_f, d_b, pairs, d_partials, mb);
     if (post) return 1;
-    finish_msg_kernel<<<1, kFinishThreads, 0, st>>>(d_partials, grid, d_msg_out);
+    launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
 }
 
@@ -406,6 +409,62 @@ __global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *p
         eq[j] = gf_mul(lo[j & mask], hi[j >> a]);
 }
 
+// The same entries from kEqRowsK variables on.  A CTA takes rows of 2^a entries
+// with the same hi and multiplies lo by its byte tables: 2 clocks per SM a
+// product instead of 7, for a build of 2048 table entries a row.  The half
+// tables' rounds (a launch's latency) are split once more: lo and the CTA's
+// own hi are products of quarter tables of at most 6 rounds.  2^18 entries: 24
+// us against 30 us, 2^20: 34 against 56, 2^22: 67 against 142 (below, the extra
+// products make it 2 to 8 us slower).
+constexpr int kEqRowsK = 18;
+constexpr int kEqThreads = 512;
+constexpr int kEqHeadRows = 64;  // rows whose hi a CTA forms at a time
+__global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq, const uint4 *point, int k,
+                                                             int a) {
+    extern __shared__ uint4 lo[];  // 2^a, then the row's byte tables
+    __shared__ uint4 quarter[4][1 << ((kEqSplitMaxK + 3) / 4)];
+    __shared__ uint4 head[kEqHeadRows];
+    const int b = k - a, a0 = a / 2, b0 = b / 2;
+    {
+        const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
+        const int first = g == 0 ? 0 : g == 1 ? a0 : g == 2 ? a : a + b0;
+        const int nv = g == 0 ? a0 : g == 1 ? a - a0 : g == 2 ? b0 : b - b0;
+        const int rounds = max(a - a0, b - b0);
+        if (t == 0) quarter[g][0] = make_uint4(1, 0, 0, 0);
+        __syncthreads();
+        for (int i = 0; i < rounds; ++i) {
+            if (i < nv && t < (1 << i)) {
+                const uint4 p = quarter[g][t];
+                const uint4 one = gf_mul(p, point[first + i]);
+                quarter[g][(1 << i) + t] = one;
+                quarter[g][t] = gf_add(p, one);
+            }
+            __syncthreads();
+        }
+    }
+    char *tbl = reinterpret_cast<char *>(lo + ((size_t)1 << a));
+    T8Lane lc;
+    lc.init();
+    for (uint32_t j = threadIdx.x; j < (1u << a); j += kEqThreads)
+        lo[j] = gf_mul(quarter[0][j & ((1u << a0) - 1)], quarter[1][j >> a0]);
+    const uint32_t rows = 1u << b;
+    uint32_t at = kEqHeadRows;  // rows of head[] taken
+    for (uint32_t h = blockIdx.x; h < rows; h += gridDim.x, ++at) {
+        if (at == kEqHeadRows) {
+            __syncthreads();
+            const uint64_t hh = h + (uint64_t)threadIdx.x * gridDim.x;
+            if (threadIdx.x < kEqHeadRows && hh < rows)
+                head[threadIdx.x] = gf_mul(quarter[2][hh & ((1u << b0) - 1)], quarter[3][hh >> b0]);
+            at = 0;
+        }
+        __syncthreads();  // head, lo; the previous row's lookups are done
+        t8_build_item<4>(tbl, head[at], threadIdx.x);
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < (1u << a); j += kEqThreads)
+            eq[((uint64_t)h << a) | j] = lc.mul(tbl, lo[j]);
+    }
+}
+
 constexpr size_t kEqSmallRounds = 12;
 
 // Up to 6 variables: the doubling rounds in one CTA.  Up to 22: one split
@@ -416,6 +475,12 @@ int launch_build_eq(const uint4 *d_point, size_t k, uint4 *d_out, cudaStream_t s
                     int num_sms) {
     if (k > 6 && k <= (size_t)kEqSplitMaxK) {
         const int a = (int)k / 2;
+        if ((int)k >= kEqRowsK) {
+            const unsigned grid = std::min(1u << (k - a), 2u * (unsigned)num_sms);
+            eq_rows_kernel<<<grid, kEqThreads, (sizeof(uint4) << a) + kT8Bytes, st>>>(
+                d_out, d_point, (int)k, a);
+            return 1;
+        }
         const size_t smem = (((size_t)1 << a) + ((size_t)1 << (k - a))) * sizeof(uint4);
         const uint64_t n = (uint64_t)1 << k;
         const unsigned grid = (unsigned)std::max<uint64_t>(
@@ -434,92 +499,113 @@ int launch_build_eq(const uint4 *d_point, size_t k, uint4 *d_out, cudaStream_t s
 }
 
 // sv[j] = sum_y eq[y] * bit_j(P[y]) (src/ligerito.rs:317-375).  128 threads
-// per CTA, one per output bit j.  For each tile of 256 y the CTA stages P in
-// shared memory and, per group of 4 consecutive y, the 16 XORs of eq over
-// every subset of the group.  Thread j gathers bit j of the group's 4 P words
-// into a 4-bit index and adds that subset's sum: one lookup per 4 y instead
-// of 4 masked additions.
-constexpr int kSvTile = 256;
-__global__ void __launch_bounds__(128) sv_fold_kernel(const uint4 *packed, const uint4 *eq,
-                                                      uint64_t n, uint4 *partials) {
-    __shared__ uint32_t sp[kSvTile][4];
-    __shared__ uint4 sub[kSvTile / 4][16];
-    const int j = threadIdx.x;
-    const int wsel = j >> 5;
-    const uint32_t bit = j & 31;
-    uint4 acc = make_uint4(0, 0, 0, 0);
-    for (uint64_t base = (uint64_t)blockIdx.x * kSvTile; base < n;
-         base += (uint64_t)gridDim.x * kSvTile) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < kSvTile; i += blockDim.x) {
-            const uint64_t y = base + i;
-            const uint4 v = y < n ? packed[y] : make_uint4(0, 0, 0, 0);
-            sp[i][0] = v.x;
-            sp[i][1] = v.y;
-            sp[i][2] = v.z;
-            sp[i][3] = v.w;
-        }
-        {
-            // thread t builds subsets 8h .. 8h+7 of group g = t / 2 (h = t mod 2)
-            const int g = threadIdx.x >> 1, h = threadIdx.x & 1;
-            uint4 e[4];
+// per CTA, one per output bit j, over tiles of 128 y.  Warp w transposes the
+// 32 P words of its y by shuffles, so thread j has bit j of 32 words in one
+// register and takes four of them as an index into the 16 subset sums of
+// their eq entries.  The sums of the 8 groups of 4 of a warp's y stand side by
+// side (row x: subset x of each group), and thread j walks the groups in an
+// order rotated by j mod 8, so a quarter-warp's lookups fall in 8 bank groups
+// as those of the byte tables do: 4 clocks per SM and y, against 17 for lookups
+// of one group by every thread.  A CTA runs four such tiles side by side and
+// stores its sums; a CTA per output adds them (2^20 words: 80 us before).
+constexpr int kSvTile = 128;
+__device__ __forceinline__ uint32_t transpose32(uint32_t x) {
+    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint64_t y = base + 4 * g + k;
-                e[k] = y < n ? eq[y] : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int m = 8 * h + q;
-                uint4 t = make_uint4(0, 0, 0, 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if ((m >> k) & 1) t = gf_add(t, e[k]);
-                sub[g][m] = t;
-            }
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int g = 0; g < kSvTile / 4; ++g) {
-            uint32_t idx = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) idx |= ((sp[4 * g + k][wsel] >> bit) & 1u) << k;
-            acc = gf_add(acc, sub[g][idx]);
-        }
+    for (int j = 16; j > 0; j >>= 1) {
+        const uint32_t m = j == 16 ? 0x0000FFFFu : j == 8 ? 0x00FF00FFu : j == 4 ? 0x0F0F0F0Fu
+                         : j == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
     }
-    partials[(uint64_t)blockIdx.x * 128 + j] = acc;
+    return x;
 }
 
-// 1024 threads: thread (g, j) XORs output j of partials g, g + 8, ...; the 8
-// groups then combine in shared memory.
-constexpr int kSvFinishGroups = 8;
-__global__ void __launch_bounds__(128 * kSvFinishGroups) sv_finish_kernel(const uint4 *partials,
-                                                                          int n_ctas, uint4 *sv) {
-    __shared__ uint4 red[kSvFinishGroups][128];
-    const int j = threadIdx.x & 127, g = threadIdx.x >> 7;
+constexpr int kSvGroups = 4;  // groups of 128 threads, each with a tile of its own
+__global__ void __launch_bounds__(kSvTile *kSvGroups, 2) sv_fold_kernel(const uint4 *packed,
+                                                                         const uint4 *eq,
+                                                                         uint64_t n,
+                                                                         uint4 *partials) {
+    __shared__ uint32_t bits[kSvGroups][4][128];
+    __shared__ uint4 sub[kSvGroups][4][16][8];
+    const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, w = t >> 5, r = t & 7;
+    auto sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(kSvTile) : "memory"); };
     uint4 acc = make_uint4(0, 0, 0, 0);
-    for (int c = g; c < n_ctas; c += kSvFinishGroups)
-        acc = gf_add(acc, partials[(uint64_t)c * 128 + j]);
-    red[g][j] = acc;
+    for (uint64_t base = ((uint64_t)blockIdx.x * kSvGroups + grp) * kSvTile; base < n;
+         base += (uint64_t)gridDim.x * kSvGroups * kSvTile) {
+        const uint64_t y = base + t;
+        const uint4 p = y < n ? packed[y] : make_uint4(0, 0, 0, 0);
+        // thread (w, q, g) sums subsets 4q .. 4q + 3 of group g of warp w's y
+        const int g = t & 7, q = (t >> 3) & 3;
+        uint4 e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t ye = base + 32 * w + 4 * g + k;
+            e[k] = ye < n ? eq[ye] : make_uint4(0, 0, 0, 0);
+        }
+        sync();  // the previous tile's lookups are done
+        bits[grp][w][t & 31] = transpose32(p.x);
+        bits[grp][w][32 + (t & 31)] = transpose32(p.y);
+        bits[grp][w][64 + (t & 31)] = transpose32(p.z);
+        bits[grp][w][96 + (t & 31)] = transpose32(p.w);
+        uint4 H = make_uint4(0, 0, 0, 0);
+        if (q & 1) H = gf_add(H, e[2]);
+        if (q & 2) H = gf_add(H, e[3]);
+        sub[grp][w][4 * q][g] = H;
+        sub[grp][w][4 * q + 1][g] = gf_add(H, e[0]);
+        sub[grp][w][4 * q + 2][g] = gf_add(H, e[1]);
+        sub[grp][w][4 * q + 3][g] = gf_add(gf_add(H, e[0]), e[1]);
+        sync();
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t b = bits[grp][s][t];
+            const uint32_t x = __funnelshift_r(b, b, 4 * r);  // nibble m: group (m + r) mod 8
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                acc = gf_add(acc, sub[grp][s][(x >> (4 * m)) & 15][(m + r) & 7]);
+        }
+    }
     __syncthreads();
-    if (g == 0) {
-        for (int k = 1; k < kSvFinishGroups; ++k) acc = gf_add(acc, red[k][j]);
-        sv[j] = acc;
+    uint4 *red = &sub[0][0][0][0];
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    if (grp == 0) {
+#pragma unroll
+        for (int k = 1; k < kSvGroups; ++k) acc = gf_add(acc, red[k * kSvTile + t]);
+        partials[(uint64_t)blockIdx.x * 128 + t] = acc;
     }
 }
 
-size_t sv_partials_bytes(size_t n, int num_sms) {
-    (void)n;
-    return (size_t)num_sms * 4 * 128 * 16;
+// CTA j XORs output j of every partial.
+__global__ void __launch_bounds__(128) sv_finish_kernel(const uint4 *partials, int n_ctas,
+                                                        uint4 *sv) {
+    __shared__ uint4 red[4];
+    chain_wait();
+    uint4 acc = make_uint4(0, 0, 0, 0);
+    for (int c = threadIdx.x; c < n_ctas; c += 128)
+        acc = gf_add(acc, partials[(uint64_t)c * 128 + blockIdx.x]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        acc.x ^= __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y ^= __shfl_xor_sync(0xffffffffu, acc.y, o);
+        acc.z ^= __shfl_xor_sync(0xffffffffu, acc.z, o);
+        acc.w ^= __shfl_xor_sync(0xffffffffu, acc.w, o);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        sv[blockIdx.x] = gf_add(gf_add(red[0], red[1]), gf_add(red[2], red[3]));
 }
 
-int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint64_t *d_partials,
+size_t sv_partials_bytes(int num_sms) { return (size_t)num_sms * 2 * 128 * sizeof(uint4); }
+
+int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_partials,
                    uint4 *d_sv, cudaStream_t st, int num_sms) {
     const uint64_t tiles = (n + kSvTile - 1) / kSvTile;
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)num_sms * 4));
-    uint4 *parts = reinterpret_cast<uint4 *>(d_partials);
-    sv_fold_kernel<<<grid, 128, 0, st>>>(d_packed, d_eq, n, parts);
-    sv_finish_kernel<<<1, 128 * kSvFinishGroups, 0, st>>>(parts, grid, d_sv);
+    const int grid = (int)std::max<uint64_t>(
+        1, std::min<uint64_t>((tiles + kSvGroups - 1) / kSvGroups, (uint64_t)num_sms * 2));
+    sv_fold_kernel<<<grid, kSvTile * kSvGroups, 0, st>>>(d_packed, d_eq, n, d_partials);
+    launch_chained(sv_finish_kernel, 128, 128, 0, st, d_partials, grid, d_sv);
     return 2;
 }
 
@@ -551,8 +637,8 @@ void init_fold_kernels() {
     init_gkr_kernels();
     cudaFuncSetAttribute(phi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kRTableSmem);
-    cudaFuncSetAttribute(eq_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)((2u << (kEqSplitMaxK / 2)) * sizeof(uint4)));
+    cudaFuncSetAttribute(eq_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(uint4) << (kEqSplitMaxK / 2)) + kT8Bytes);
     cudaFuncSetAttribute(fold_and_msg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kRTableSmem);
     cudaFuncSetAttribute(fold_and_msg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -627,6 +713,7 @@ int launch_chacha(uint64_t seed, uint64_t first_word, uint4 *d_out, size_t n_wor
 // batched_eval, gkr.rs:93-108: the top index bit pairs the factors).
 __global__ void __launch_bounds__(256) gkr_product_kernel(const uint4 *in, uint64_t half,
                                                           uint4 *out) {
+    chain_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < half;
          i += (uint64_t)gridDim.x * blockDim.x)
         out[i] = gf_mul(in[i], in[half + i]);
@@ -704,7 +791,7 @@ int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_
                        int num_sms) {
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((half + 255) / 256, (uint64_t)num_sms * 8));
-    gkr_product_kernel<<<grid, 256, 0, st>>>(d_in, half, d_out);
+    launch_chained(gkr_product_kernel, grid, 256, 0, st, d_in, half, d_out);
     return 1;
 }
 
@@ -723,7 +810,7 @@ int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fo
         gkr_round_kernel<false><<<grid, 256, 0, st>>>(d_l, d_r, d_w, h, rho, send_one,
                                                       d_partials, mb, d_w_next);
     if (post) return 1;
-    finish_msg_kernel<<<1, kFinishThreads, 0, st>>>(d_partials, grid, d_out);
+    launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_out);
     return 2;
 }
 

@@ -1079,11 +1079,11 @@ int bz_build_eq_lsb(bz_ctx *ctx, const uint64_t *point, size_t k, uint64_t *d_ou
 int bz_sv_fold(bz_ctx *ctx, const uint64_t *d_packed, const uint64_t *d_eq, size_t n,
                uint64_t *sv) {
     if (!ctx || !d_packed || !d_eq || !sv) return BZ_ERR_ARG;
-    int rc = ensure_scratch(ctx, sv_partials_bytes(n, ctx->num_sms) + 128 * 16);
+    int rc = ensure_scratch(ctx, sv_partials_bytes(ctx->num_sms) + 128 * 16);
     if (rc) return rc;
-    uint4 *d_sv = (uint4 *)(ctx->scratch + sv_partials_bytes(n, ctx->num_sms));
+    uint4 *d_sv = (uint4 *)(ctx->scratch + sv_partials_bytes(ctx->num_sms));
     ctx->launches += launch_sv_fold((const uint4 *)d_packed, (const uint4 *)d_eq, n,
-                                    (uint64_t *)ctx->scratch, d_sv, ctx->stream, ctx->num_sms);
+                                    (uint4 *)ctx->scratch, d_sv, ctx->stream, ctx->num_sms);
     BZ_CUDA(ctx, cudaGetLastError());
     BZ_CUDA(ctx, cudaMemcpyAsync(sv, d_sv, 128 * 16, cudaMemcpyDeviceToHost, ctx->stream));
     BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

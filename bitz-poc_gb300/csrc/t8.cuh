@@ -32,12 +32,15 @@ BZ_HD uint4 gf_mul_x(uint4 t) {
     return r;
 }
 
-// Work item u (0 .. 127) of the table of t: byte position s = u mod 8 and the
-// high nibble hi = u / 8 of the byte value; writes the 16 entries
-// (hi * 16 + lo, s).  The 8 threads of a quarter-warp take 8 different byte
-// positions, so their stores fall in 8 different bank groups.
+// Work item u (0 .. 128 * PARTS - 1) of the table of t: byte position
+// s = u mod 8, the high nibble hi = u / 8 mod 16 of the byte value and a part
+// u / 128 of the low nibbles; writes the 16 / PARTS entries (hi * 16 + lo, s).
+// The 8 threads of a quarter-warp take 8 different byte positions, so their
+// stores fall in 8 different bank groups.
+template <int PARTS = 1>
 __device__ __forceinline__ void t8_build_item(char *tb, uint4 t, int u) {
     const int s = u & 7, hi = (u >> 3) & 15;
+    const int lo0 = PARTS == 1 ? 0 : (u >> 7) * (16 / PARTS);
     uint4 b[8];
     b[0] = gf_mul_xpow(t, (uint32_t)(8 * s));
 #pragma unroll
@@ -46,17 +49,23 @@ __device__ __forceinline__ void t8_build_item(char *tb, uint4 t, int u) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
         if ((hi >> q) & 1) H = gf_add(H, b[4 + q]);
-    uint4 L[16];
+    if constexpr (PARTS > 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if ((lo0 >> q) & 1) H = gf_add(H, b[q]);
+    }
+    uint4 L[16 / PARTS];
     L[0] = make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int x = 1; x < 16; ++x) {
+    for (int x = 1; x < 16 / PARTS; ++x) {
         const int low = x & -x;
         const uint4 bb = low == 1 ? b[0] : low == 2 ? b[1] : low == 4 ? b[2] : b[3];
         L[x] = gf_add(L[x & (x - 1)], bb);
     }
 #pragma unroll
-    for (int lo = 0; lo < 16; ++lo)
-        *reinterpret_cast<uint4 *>(tb + ((hi << 4) | lo) * 128 + s * 16) = gf_add(H, L[lo]);
+    for (int lo = 0; lo < 16 / PARTS; ++lo)
+        *reinterpret_cast<uint4 *>(tb + ((hi << 4) | (lo0 + lo)) * 128 + s * 16) =
+            gf_add(H, L[lo]);
 }
 
 // Per-thread lookup order: step m reads byte position (m + r) mod 8, r =
