@@ -24,13 +24,13 @@ __device__ __forceinline__ void chain_wait() {
 }
 
 template <typename... P, typename... A>
-inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
                            cudaStream_t st, A &&...args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;

@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(256, 2) fold_and_msg_kernel(const uint4 *f, co
                                                            uint64_t half, uint4 r, uint4 *nf,
                                                            uint4 *nb, uint64_t *partials,
                                                            MsgMailbox mb, RGate gate) {
+    chain_wait();
     extern __shared__ uint4 smem[];
     if constexpr (GATED) {
         if (!gate_wait(gate, r)) return;
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(256, 2) fold_and_msg_kernel(const uint4 *f, co
 __global__ void __launch_bounds__(256) round_msg_kernel(const uint4 *f, const uint4 *b,
                                                         uint64_t pairs, uint64_t *partials,
                                                         MsgMailbox mb) {
+    chain_wait();
     gf_wide u0 = gf_wide_zero(), u2 = gf_wide_zero();
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < pairs;
          j += (uint64_t)gridDim.x * blockDim.x) {
@@ -296,11 +298,11 @@ int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, u
     MsgMailbox mb;
     if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
     if (gate)
-        fold_and_msg_kernel<true><<<grid, 256, kRTableSmem, st>>>(d_f, d_b, half, r, d_nf, d_nb,
-                                                                  d_partials, mb, *gate);
+        launch_chained(fold_and_msg_kernel<true>, grid, 256, kRTableSmem, st, d_f, d_b, half, r,
+                       d_nf, d_nb, d_partials, mb, *gate);
     else
-        fold_and_msg_kernel<false><<<grid, 256, kRTableSmem, st>>>(d_f, d_b, half, r, d_nf, d_nb,
-                                                                   d_partials, mb, RGate{});
+        launch_chained(fold_and_msg_kernel<false>, grid, 256, kRTableSmem, st, d_f, d_b, half, r,
+                       d_nf, d_nb, d_partials, mb, RGate{});
     if (post) return 1;
     launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
@@ -312,7 +314,7 @@ int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_p
     const int grid = std::min(msg_grid(pairs, num_sms), 1024);
     MsgMailbox mb;
     if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
-    round_msg_kernel<<<grid, 256, 0, st>>>(d_f, d_b, pairs, d_partials, mb);
+    launch_chained(round_msg_kernel, grid, 256, 0, st, d_f, d_b, pairs, d_partials, mb);
     if (post) return 1;
     launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
@@ -322,6 +324,7 @@ int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_p
 // (= in[2i]*(1+r) + in[2i+1]*r exactly, ligerito.rs:1686-1691).
 __global__ void __launch_bounds__(256) partial_eval_round_kernel(const uint4 *in, uint64_t half,
                                                                  uint4 r, uint4 *out) {
+    chain_wait();
     extern __shared__ uint4 smem[];
     const char *T = build_r_table(smem, r);
     T16Lane8 lc;
@@ -337,12 +340,14 @@ int launch_partial_eval_round(const uint4 *d_in, size_t n, uint4 r, uint4 *d_out
                               cudaStream_t st) {
     const uint64_t half = n / 2;
     const unsigned grid = (unsigned)std::min<uint64_t>((half + 255) / 256, 152 * 3);
-    partial_eval_round_kernel<<<std::max(grid, 1u), 256, kRTableSmem, st>>>(d_in, half, r, d_out);
+    launch_chained(partial_eval_round_kernel, std::max(grid, 1u), 256, kRTableSmem, st, d_in,
+                   half, r, d_out);
     return 1;
 }
 
 // eq table rounds: entries [0, half) double into [0, 2 half).
 __global__ void eq_round_kernel(uint4 *eq, uint64_t half, const uint4 *point, int i) {
+    chain_wait();
     const uint4 r = point[i];
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < half;
          j += (uint64_t)gridDim.x * blockDim.x) {
@@ -356,6 +361,7 @@ __global__ void eq_round_kernel(uint4 *eq, uint64_t half, const uint4 *point, in
 // The first k rounds in one CTA (global writes of a round are visible to the
 // CTA's threads after the barrier).
 __global__ void __launch_bounds__(512) eq_small_kernel(uint4 *eq, const uint4 *point, int k) {
+    chain_wait();
     if (threadIdx.x == 0) eq[0] = make_uint4(1, 0, 0, 0);
     __syncthreads();
     for (int i = 0; i < k; ++i) {
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(512) eq_small_kernel(uint4 *eq, const uint4 *p
 constexpr int kEqSplitMaxK = 22;
 __global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *point, int k,
                                                        int a) {
+    chain_wait();
     extern __shared__ uint4 halves[];
     const int b = k - a;
     uint4 *lo = halves, *hi = halves + ((size_t)1 << a);
@@ -421,6 +428,7 @@ constexpr int kEqThreads = 512;
 constexpr int kEqHeadRows = 64;  // rows whose hi a CTA forms at a time
 __global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq, const uint4 *point, int k,
                                                              int a) {
+    chain_wait();
     extern __shared__ uint4 lo[];  // 2^a, then the row's byte tables
     __shared__ uint4 quarter[4][1 << ((kEqSplitMaxK + 3) / 4)];
     __shared__ uint4 head[kEqHeadRows];
@@ -477,23 +485,24 @@ int launch_build_eq(const uint4 *d_point, size_t k, uint4 *d_out, cudaStream_t s
         const int a = (int)k / 2;
         if ((int)k >= kEqRowsK) {
             const unsigned grid = std::min(1u << (k - a), 2u * (unsigned)num_sms);
-            eq_rows_kernel<<<grid, kEqThreads, (sizeof(uint4) << a) + kT8Bytes, st>>>(
-                d_out, d_point, (int)k, a);
+            launch_chained(eq_rows_kernel, grid, kEqThreads, (sizeof(uint4) << a) + kT8Bytes, st,
+                           d_out, d_point, (int)k, a);
             return 1;
         }
         const size_t smem = (((size_t)1 << a) + ((size_t)1 << (k - a))) * sizeof(uint4);
         const uint64_t n = (uint64_t)1 << k;
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((n + 511) / 512, (uint64_t)2 * num_sms));
-        eq_split_kernel<<<grid, 512, smem, st>>>(d_out, d_point, (int)k, a);
+        launch_chained(eq_split_kernel, grid, 512, smem, st, d_out, d_point, (int)k, a);
         return 1;
     }
     const size_t k0 = std::min(k, kEqSmallRounds);
-    eq_small_kernel<<<1, 512, 0, st>>>(d_out, d_point, (int)k0);
+    launch_chained(eq_small_kernel, 1, 512, 0, st, d_out, d_point, (int)k0);
     for (size_t i = k0; i < k; ++i) {
         const uint64_t half = (uint64_t)1 << i;
         const unsigned grid = (unsigned)std::min<uint64_t>((half + 255) / 256, 8192);
-        eq_round_kernel<<<std::max(grid, 1u), 256, 0, st>>>(d_out, half, d_point, (int)i);
+        launch_chained(eq_round_kernel, std::max(grid, 1u), 256, 0, st, d_out, half, d_point,
+                       (int)i);
     }
     return (int)(k - k0) + 1;
 }
@@ -526,6 +535,7 @@ __global__ void __launch_bounds__(kSvTile *kSvGroups, 2) sv_fold_kernel(const ui
                                                                          const uint4 *eq,
                                                                          uint64_t n,
                                                                          uint4 *partials) {
+    chain_wait();
     __shared__ uint32_t bits[kSvGroups][4][128];
     __shared__ uint4 sub[kSvGroups][4][16][8];
     const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, w = t >> 5, r = t & 7;
@@ -604,7 +614,8 @@ int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_
     const uint64_t tiles = (n + kSvTile - 1) / kSvTile;
     const int grid = (int)std::max<uint64_t>(
         1, std::min<uint64_t>((tiles + kSvGroups - 1) / kSvGroups, (uint64_t)num_sms * 2));
-    sv_fold_kernel<<<grid, kSvTile * kSvGroups, 0, st>>>(d_packed, d_eq, n, d_partials);
+    launch_chained(sv_fold_kernel, grid, kSvTile * kSvGroups, 0, st, d_packed, d_eq, n,
+                   d_partials);
     launch_chained(sv_finish_kernel, 128, 128, 0, st, d_partials, grid, d_sv);
     return 2;
 }
@@ -617,6 +628,7 @@ int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_
 // table multiply.
 __global__ void __launch_bounds__(256) phi_kernel(const uint4 *eq_hi, uint64_t n,
                                                   const uint4 *eq_r2, uint4 *out) {
+    chain_wait();
     extern __shared__ uint4 smem[];
     uint4 *bases = smem + kT16Entries;
     for (int e = threadIdx.x; e < 128; e += blockDim.x)
@@ -653,7 +665,7 @@ int launch_phi(const uint4 *d_eq_hi, size_t n, const uint4 *d_eq_r2, uint4 *d_ou
                cudaStream_t st, int num_sms) {
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((n + 255) / 256, (uint64_t)2 * num_sms));
-    phi_kernel<<<grid, 256, kRTableSmem, st>>>(d_eq_hi, n, d_eq_r2, d_out);
+    launch_chained(phi_kernel, grid, 256, kRTableSmem, st, d_eq_hi, n, d_eq_r2, d_out);
     return 1;
 }
 
@@ -735,6 +747,7 @@ __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, c
                                                            uint64_t h, uint4 rho, int send_one,
                                                            uint64_t *partials, MsgMailbox mb,
                                                            uint4 *w_next) {
+    chain_wait();
     extern __shared__ uint4 smem[];
     const char *T = nullptr;
     T16Lane8 lc;
@@ -778,6 +791,7 @@ __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, c
 __global__ void __launch_bounds__(256) gkr_forest_leaves_kernel(const uint64_t *packed,
                                                                 const uint4 *images, int t,
                                                                 int s, uint4 *out) {
+    chain_wait();
     const uint64_t n = (uint64_t)1 << (t + s), rows = (uint64_t)1 << t;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -804,11 +818,11 @@ int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fo
     MsgMailbox mb;
     if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
     if (fold)
-        gkr_round_kernel<true><<<grid, 256, kRTableSmem, st>>>(d_l, d_r, d_w, h, rho, send_one,
-                                                               d_partials, mb, d_w_next);
+        launch_chained(gkr_round_kernel<true>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h, rho,
+                       send_one, d_partials, mb, d_w_next);
     else
-        gkr_round_kernel<false><<<grid, 256, 0, st>>>(d_l, d_r, d_w, h, rho, send_one,
-                                                      d_partials, mb, d_w_next);
+        launch_chained(gkr_round_kernel<false>, grid, 256, 0, st, d_l, d_r, d_w, h, rho, send_one,
+                       d_partials, mb, d_w_next);
     if (post) return 1;
     launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_out);
     return 2;
@@ -824,7 +838,7 @@ int launch_gkr_forest_leaves(const uint64_t *d_packed, const uint4 *d_images, in
     const uint64_t n = (uint64_t)1 << (t + s);
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((n + 255) / 256, (uint64_t)num_sms * 8));
-    gkr_forest_leaves_kernel<<<grid, 256, 0, st>>>(d_packed, d_images, t, s, d_out);
+    launch_chained(gkr_forest_leaves_kernel, grid, 256, 0, st, d_packed, d_images, t, s, d_out);
     return 1;
 }
 

@@ -135,6 +135,7 @@ __global__ void glue_kernel(uint4 *b, const uint4 *nb, uint64_t n, uint4 beta) {
 // per-CTA partials of sum_j f[j] * b[j]
 __global__ void __launch_bounds__(kThreads) dot_kernel(const uint4 *f, const uint4 *b, uint64_t n,
                                                        uint4 *partial) {
+    chain_wait();
     uint4 acc = make_uint4(0, 0, 0, 0);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(kThreads) split_dot_rows_kernel(const uint4 *p
                                                                   const uint4 *head,
                                                                   uint64_t n_blocks,
                                                                   uint4 *partial) {
+    chain_wait();
     __shared__ __align__(16) char tbl[kT8Bytes];
     T8Lane lc;
     lc.init();
@@ -188,6 +190,7 @@ __global__ void __launch_bounds__(kThreads) split_dot_rows_kernel(const uint4 *p
 __global__ void __launch_bounds__(kThreads) split_dot_kernel(const uint4 *p, const uint4 *tail,
                                                              int lo, const uint4 *head,
                                                              uint64_t n_blocks, uint4 *partial) {
+    chain_wait();
     const uint64_t bl = (uint64_t)1 << lo;
     uint4 acc = make_uint4(0, 0, 0, 0);
     for (uint64_t h = blockIdx.x; h < n_blocks; h += gridDim.x) {
@@ -208,6 +211,7 @@ constexpr int kAxpyLog = 11;
 __global__ void __launch_bounds__(kThreads) eq_axpy_rows_kernel(uint4 *b, const uint4 *tail,
                                                                 int lo, const uint4 *head,
                                                                 uint4 eta) {
+    chain_wait();
     __shared__ __align__(16) char tbl[kT8Bytes];
     T8Lane lc;
     lc.init();
@@ -233,6 +237,7 @@ static_assert((1 << kLogThreads) == kThreads, "eq_axpy assumes 256-thread CTAs")
 __global__ void __launch_bounds__(kThreads) eq_axpy_kernel(uint4 *b, const uint4 *tail, int lo,
                                                            const uint4 *head, uint4 eta,
                                                            uint64_t n) {
+    chain_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint4 s;
     if (lo >= kLogThreads) {
@@ -272,12 +277,12 @@ int launch_split_dot(const uint4 *d_p, const uint4 *d_tail, int lo, const uint4 
     size_t ctas = std::max<size_t>(1, std::min(n_blocks, cap));
     const dim3 grid(lo >= kDotCols ? 1u << (lo - kDotCols) : 1u, dot_row_splits(n_blocks, num_sms));
     if (lo >= kDotCols && n_blocks >= 8 && (size_t)grid.x * grid.y <= cap) {
-        split_dot_rows_kernel<<<grid, kThreads, 0, st>>>(d_p, d_tail, lo, d_head, n_blocks,
-                                                         d_partial);
+        launch_chained(split_dot_rows_kernel, grid, kThreads, 0, st, d_p, d_tail, lo, d_head,
+                       n_blocks, d_partial);
         ctas = (size_t)grid.x * grid.y;
     } else {
-        split_dot_kernel<<<(unsigned)ctas, kThreads, 0, st>>>(d_p, d_tail, lo, d_head, n_blocks,
-                                                              d_partial);
+        launch_chained(split_dot_kernel, (unsigned)ctas, kThreads, 0, st, d_p, d_tail, lo, d_head,
+                       n_blocks, d_partial);
     }
     launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, d_out);
     return 2;
@@ -286,10 +291,11 @@ int launch_split_dot(const uint4 *d_p, const uint4 *d_tail, int lo, const uint4 
 int launch_eq_axpy(uint4 *d_b, const uint4 *d_tail, int lo, const uint4 *d_head, uint4 eta,
                    size_t n, cudaStream_t st) {
     if (lo >= kAxpyLog && n >> kAxpyLog)
-        eq_axpy_rows_kernel<<<(unsigned)(n >> kAxpyLog), kThreads, 0, st>>>(d_b, d_tail, lo,
-                                                                            d_head, eta);
+        launch_chained(eq_axpy_rows_kernel, (unsigned)(n >> kAxpyLog), kThreads, 0, st, d_b,
+                       d_tail, lo, d_head, eta);
     else
-        eq_axpy_kernel<<<grid_for(n), kThreads, 0, st>>>(d_b, d_tail, lo, d_head, eta, n);
+        launch_chained(eq_axpy_kernel, grid_for(n), kThreads, 0, st, d_b, d_tail, lo, d_head, eta,
+                       n);
     return 1;
 }
 
@@ -330,7 +336,7 @@ size_t dot_partials_count(size_t n, int num_sms) {
 int launch_dot(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 *d_partial, uint4 *d_out,
                cudaStream_t st, int num_sms) {
     const size_t ctas = dot_partials_count(n, num_sms);
-    dot_kernel<<<(unsigned)ctas, kThreads, 0, st>>>(d_f, d_b, n, d_partial);
+    launch_chained(dot_kernel, (unsigned)ctas, kThreads, 0, st, d_f, d_b, n, d_partial);
     launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, d_out);
     return 2;
 }

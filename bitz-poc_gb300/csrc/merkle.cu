@@ -383,6 +383,7 @@ int launch_combine_shard_cvs(const uint8_t *d_cvs, uint32_t world, uint64_t n_le
 // ---------------------------------------------------------------------------
 __global__ void gather_rows(const uint4 *cw, int log_lanes, const uint64_t *pos, size_t q,
                             uint4 *out) {
+    chain_wait();
     const uint64_t L = (uint64_t)1 << log_lanes;
     const uint64_t total = q * L;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -393,6 +394,7 @@ __global__ void gather_rows(const uint4 *cw, int log_lanes, const uint64_t *pos,
 }
 
 __global__ void gather_nodes(const uint4 *tree, const uint64_t *idx, size_t n, uint4 *out) {
+    chain_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2 * n) return;
     out[i] = tree[idx[i >> 1] * 2 + (i & 1)];
@@ -403,15 +405,16 @@ int launch_gather_rows(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, 
     if (q == 0) return 0;
     const uint64_t total = (uint64_t)q << log_lanes;
     const unsigned grid = (unsigned)std::min<uint64_t>((total + 255) / 256, 4096);
-    gather_rows<<<grid, 256, 0, st>>>(d_cw, log_lanes, d_pos, q, d_out);
+    launch_chained(gather_rows, grid, 256, 0, st, d_cw, log_lanes, d_pos, q, d_out);
     return 1;
 }
 
 int launch_gather_nodes(const uint8_t *d_tree, const uint64_t *d_idx, size_t n, uint8_t *d_out,
                         cudaStream_t st) {
     if (n == 0) return 0;
-    gather_nodes<<<(unsigned)((2 * n + 255) / 256), 256, 0, st>>>(
-        reinterpret_cast<const uint4 *>(d_tree), d_idx, n, reinterpret_cast<uint4 *>(d_out));
+    launch_chained(gather_nodes, (unsigned)((2 * n + 255) / 256), 256, 0, st,
+                   reinterpret_cast<const uint4 *>(d_tree), d_idx, n,
+                   reinterpret_cast<uint4 *>(d_out));
     return 1;
 }
 
