@@ -128,12 +128,26 @@ uint32_t log2_exact(size_t n) {
     return k;
 }
 
+// 64 x 64 bits: out[u] bit v = in[v] bit u, by swapping blocks of halving size
+void transpose_bits_64(uint64_t x[64]) {
+    uint64_t m = 0x00000000FFFFFFFFull;
+    for (int j = 32; j; j >>= 1, m ^= m << j)
+        for (int k = 0; k < 64; k = (k + j + 1) & ~j) {
+            const uint64_t t = ((x[k] >> j) ^ x[k + j]) & m;
+            x[k] ^= t << j;
+            x[k + j] ^= t;
+        }
+}
+
 // the 128 x 128 bit transpose of s (src/ligerito.rs:108-120)
 void transpose_bits_128(const uint64_t *s, uint64_t *out) {
-    memset(out, 0, 256 * 8);
-    for (int v = 0; v < 128; ++v)
-        for (int u = 0; u < 128; ++u)
-            if ((s[2 * v + (u >> 6)] >> (u & 63)) & 1) out[2 * u + (v >> 6)] |= 1ull << (v & 63);
+    for (int r = 0; r < 2; ++r)
+        for (int c = 0; c < 2; ++c) {
+            uint64_t x[64];
+            for (int i = 0; i < 64; ++i) x[i] = s[2 * (64 * r + i) + c];
+            transpose_bits_64(x);
+            for (int i = 0; i < 64; ++i) out[2 * (64 * c + i) + r] = x[i];
+        }
 }
 
 }  // namespace
