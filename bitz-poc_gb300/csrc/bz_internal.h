@@ -124,10 +124,18 @@ int launch_commit_pipelined(const Shape &s, uint32_t schedule, const uint4 *d_ms
 int launch_combine_shard_cvs(const uint8_t *d_cvs, uint32_t world, uint64_t n_leaves,
                              uint8_t *d_tree, cudaStream_t st);
 // Merkle tree over the codeword rows (leaves = positions).  d_scratch must hold
-// merkle_scratch_bytes(s).  Returns kernels launched.
+// merkle_scratch_bytes(s).  Returns kernels launched.  With `post`, the kernel
+// that writes the root of a tree of at least two leaves also posts it to mapped
+// host memory: four 64-bit words, then the sequence number.
+struct RootPost {
+    uint64_t *words = nullptr;  // device view of mapped host memory
+    uint32_t *seq = nullptr;    // device view of mapped host memory
+    uint32_t seq_val = 0;
+};
 size_t merkle_scratch_bytes(const Shape &s);
 int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d_scratch,
-                  cudaStream_t st, int num_sms, LaunchLog *log = nullptr);
+                  cudaStream_t st, int num_sms, LaunchLog *log = nullptr,
+                  const RootPost *post = nullptr);
 
 // Gathers: rows of the codeword and arbitrary tree nodes.
 int launch_gather_rows(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, size_t q,

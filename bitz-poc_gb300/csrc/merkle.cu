@@ -24,11 +24,12 @@ namespace bz {
 // ---- kernels around the bodies of merkle_kernels.cuh -----------------------
 __global__ void __launch_bounds__(256) b3_leaves_chunked(const uint4 *cw, uint64_t n_chunks,
                                                          uint32_t *tree_leaves, int log_c,
-                                                         uint64_t chunk0) {
+                                                         uint64_t chunk0, int levels,
+                                                         uint64_t n_leaves) {
     __shared__ uint32_t cvs[256][9];  // padded rows
     chain_wait();
     b3_leaves_chunked_body(cw, n_chunks, tree_leaves, log_c, chunk0,
-                           (uint64_t)blockIdx.x * blockDim.x, cvs);
+                           (uint64_t)blockIdx.x * blockDim.x, cvs, levels, n_leaves);
 }
 
 __global__ void b3_leaves_small(const uint4 *cw, int log_lanes, uint64_t n_leaves,
@@ -37,6 +38,38 @@ __global__ void b3_leaves_small(const uint4 *cw, int log_lanes, uint64_t n_leave
     b3_leaves_small_body(cw, log_lanes, n_leaves, tree_leaves,
                          (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                          (uint64_t)gridDim.x * blockDim.x);
+}
+
+// Short leaves (one per thread, a power of two of them) and the `levels` tree
+// levels above the CTA's blockDim.x leaves, level l stored at tree + the sizes
+// of the levels below it.
+__global__ void __launch_bounds__(256) b3_leaves_small_levels(const uint4 *cw, int log_lanes,
+                                                              uint64_t n_leaves, uint32_t *tree,
+                                                              int levels) {
+    __shared__ uint32_t nodes[256][9];  // padded rows
+    chain_wait();
+    const uint32_t t = threadIdx.x;
+    const uint64_t leaf = (uint64_t)blockIdx.x * blockDim.x + t;
+    uint32_t o[8];
+    b3_leaf_small(cw + (leaf << log_lanes), log_lanes, o);
+    uint64_t off = 0;
+    for (int lv = 0;; ++lv) {
+        const uint32_t n = blockDim.x >> lv;  // the CTA's nodes of this level
+        if (t < n) {
+            uint4 *po = reinterpret_cast<uint4 *>(tree + (off + (uint64_t)blockIdx.x * n + t) * 8);
+            po[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            po[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+        if (lv == levels) break;
+        if (t < n) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
+        }
+        __syncthreads();
+        if (t < n / 2) b3_parent(nodes[2 * t], nodes[2 * t + 1], o);
+        __syncthreads();  // every read of this level precedes the overwrite
+        off += n_leaves >> lv;
+    }
 }
 
 __global__ void __launch_bounds__(256) merkle_levels(LevelsArgs a) {
@@ -64,55 +97,28 @@ __global__ void __launch_bounds__(128) sha_leaves(const uint4 *cw, int log_lanes
 constexpr int kTreeSmallMax = 1024;  // leaves (threads)
 __global__ void __launch_bounds__(kTreeSmallMax) b3_tree_small(const uint4 *cw, int log_lanes,
                                                                uint32_t n_leaves,
-                                                               uint32_t *tree) {
+                                                               uint32_t *tree, RootPost post) {
     __shared__ uint32_t nodes[kTreeSmallMax][9];  // padded rows
     chain_wait();
     const uint32_t t = threadIdx.x;
-    uint32_t cv[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) cv[i] = kIV[i];
-    const uint32_t elems = 1u << log_lanes, bytes = elems * 16, nblk = (bytes + 63) / 64;
-    const uint4 *p = cw + (uint64_t)t * elems;
-#pragma unroll 1
-    for (uint32_t blk = 0; blk < nblk; ++blk) {
-        uint32_t m[16];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t e = blk * 4 + q;
-            const uint4 v = e < elems ? p[e] : make_uint4(0, 0, 0, 0);
-            m[4 * q] = v.x;
-            m[4 * q + 1] = v.y;
-            m[4 * q + 2] = v.z;
-            m[4 * q + 3] = v.w;
-        }
-        const uint32_t len = min(64u, bytes - blk * 64);
-        const uint32_t flags =
-            (blk == 0 ? B3_CHUNK_START : 0) | (blk == nblk - 1 ? B3_CHUNK_END : 0);
-        b3_compress_cv(cv, m, 0, len, flags);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        nodes[t][i] = cv[i];
-        tree[(uint64_t)t * 8 + i] = cv[i];
-    }
-    __syncthreads();
-    uint64_t off = n_leaves;
-    for (uint32_t n = n_leaves; n > 1; n >>= 1) {
-        const uint32_t half = n >> 1;
-        uint32_t o[8];
-        if (t < half) {
-            b3_parent(nodes[2 * t], nodes[2 * t + 1], o);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) tree[(off + t) * 8 + i] = o[i];
-        }
-        __syncthreads();  // every read of this level precedes the overwrite
-        if (t < half) {
+    uint32_t o[8];
+    b3_leaf_small(cw + ((uint64_t)t << log_lanes), log_lanes, o);
+    uint64_t off = 0;
+    for (uint32_t n = n_leaves;; n >>= 1) {
+        if (t < n) {
+            uint4 *po = reinterpret_cast<uint4 *>(tree + (off + t) * 8);
+            po[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            po[1] = make_uint4(o[4], o[5], o[6], o[7]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
         }
         __syncthreads();
-        off += half;
+        if (n == 1) break;
+        if (t < n / 2) b3_parent(nodes[2 * t], nodes[2 * t + 1], o);
+        __syncthreads();  // every read of this level precedes the overwrite
+        off += n;
     }
+    if (t == 0) post_root(post, o);
 }
 
 // A small SHA-256 tree in one CTA: thread i hashes leaf i, then the CTA builds
@@ -121,7 +127,7 @@ __global__ void __launch_bounds__(kTreeSmallMax) b3_tree_small(const uint4 *cw, 
 constexpr int kShaTreeSmallMax = 128;  // leaves (threads)
 __global__ void __launch_bounds__(kShaTreeSmallMax) sha_tree_small(
     const uint4 *cw, int log_lanes, uint32_t n_leaves, uint32_t *tree,
-    const __grid_constant__ ShaWords pad) {
+    const __grid_constant__ ShaWords pad, RootPost post) {
     __shared__ uint32_t nodes[kShaTreeSmallMax][9];  // padded rows
     chain_wait();
     const uint32_t t = threadIdx.x;
@@ -136,12 +142,13 @@ __global__ void __launch_bounds__(kShaTreeSmallMax) sha_tree_small(
 #pragma unroll
             for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];
         }
-        if (n == 1) break;
         __syncthreads();
+        if (n == 1) break;
         if (t < n / 2) sha256_pair(nodes[2 * t], nodes[2 * t + 1], o);
         __syncthreads();  // every read of this level precedes the overwrite
         off += n;
     }
+    if (t == 0 && n_leaves > 1) post_root(post, o);
 }
 
 // Generic BLAKE3 chunk CVs into scratch (leaves longer than 256 chunks).
@@ -182,8 +189,25 @@ size_t merkle_scratch_bytes(const Shape &s) {
 }
 
 // Build all parent levels above `n_leaves` leaves stored at tree[0..).
+// (or above level `from`, whose nodes are stored).
 static int launch_levels(uint32_t *tree, uint64_t n_leaves, int kind, cudaStream_t st,
-                         LaunchLog *log);
+                         LaunchLog *log, int from = 0, const RootPost *post = nullptr);
+
+// Tree levels that the leaf kernel builds, of at most `most` that its CTAs can:
+// the fewest that save a launch of nine levels, below the root, else none.  A
+// level costs a CTA more than 1 us behind its leaves, and a launch 4 us or more
+// (2^17 leaves of 256 bytes, 17 levels: 49 us with 8 levels and one launch, 51
+// with two launches; 2^14 leaves of 64 KiB with the 2 levels that its CTAs
+// reach and still two launches: 569 + 20 us against 551 + 20).  For commits that
+// a caller waits for (those that post their root): many at once are bound by
+// issue slots, of which half-empty levels waste some (16 commits in one plan:
+// 1431 us against 1411).
+static int leaf_levels(uint64_t n_leaves, int most) {
+    int lg = 0;
+    while (n_leaves >> (lg + 1)) ++lg;
+    const int need = lg % 9 == 0 ? 9 : lg % 9;
+    return lg > 9 && need <= most ? need : 0;
+}
 
 // CTA size of b3_leaves_chunked: 256 threads, halved (down to 32 and to the
 // chunks per leaf) while that leaves fewer than two CTAs per SM.
@@ -211,7 +235,7 @@ int launch_leaves_range(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint
             const uint64_t n_chunks = n << log_c;
             const unsigned t = leaf_threads(n_chunks, log_c, num_sms);
             launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, cw,
-                           n_chunks, leaves, log_c, s.chunk0);
+                           n_chunks, leaves, log_c, s.chunk0, 0, n);
         }
     } else {
         launch_chained(sha_leaves, (unsigned)((n + 127) / 128), 128, 0, st, cw, s.log_lanes, n,
@@ -226,9 +250,9 @@ int launch_merkle_levels(const Shape &s, uint8_t *d_tree, cudaStream_t st, Launc
 }
 
 static int launch_levels(uint32_t *tree, uint64_t n_leaves, int kind, cudaStream_t st,
-                         LaunchLog *log) {
+                         LaunchLog *log, int from, const RootPost *post) {
     int launches = 0;
-    uint64_t in_off = 0, n_in = n_leaves;
+    uint64_t in_off = 2 * n_leaves - (2 * n_leaves >> from), n_in = n_leaves >> from;
     while (n_in > 1) {
         int k = 0;
         uint64_t n = n_in;
@@ -241,6 +265,7 @@ static int launch_levels(uint32_t *tree, uint64_t n_leaves, int kind, cudaStream
         a.n_in = n_in;
         a.k = k;
         a.kind = kind;
+        if (post && n_in >> k == 1) a.post = *post;
         uint64_t off = in_off + n_in, cnt = n_in >> 1;
         for (int j = 0; j < k; ++j) {
             a.out[j] = tree + off * 8;
@@ -264,7 +289,8 @@ static int launch_levels(uint32_t *tree, uint64_t n_leaves, int kind, cudaStream
 }
 
 int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d_scratch,
-                  cudaStream_t st, int num_sms, LaunchLog *log) {
+                  cudaStream_t st, int num_sms, LaunchLog *log, const RootPost *post) {
+    int from = 0;  // tree levels the leaf kernel has built
     auto mark = [&](const char *n) {
         if (log) log->mark(n);
     };
@@ -274,21 +300,31 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
     if (s.hash_kind == 1) {
         if (s.log_lanes < 6 && n_leaves <= (uint64_t)kTreeSmallMax && n_leaves >= 2) {
             launch_chained(b3_tree_small, 1, (unsigned)n_leaves, 0, st, d_cw, s.log_lanes,
-                           (uint32_t)n_leaves, tree);
+                           (uint32_t)n_leaves, tree, post ? *post : RootPost{});
             mark("b3_tree_small");
             return 1;
         }
         if (s.log_lanes < 6) {
-            launch_chained(b3_leaves_small, (unsigned)((n_leaves + 255) / 256), 256, 0, st, d_cw,
-                           s.log_lanes, n_leaves, tree);
+            // more than kTreeSmallMax leaves: a multiple of the CTA's 256
+            from = post ? leaf_levels(n_leaves, 8) : 0;
+            if (from)
+                launch_chained(b3_leaves_small_levels, (unsigned)(n_leaves / 256), 256, 0, st,
+                               d_cw, s.log_lanes, n_leaves, tree, from);
+            else
+                launch_chained(b3_leaves_small, (unsigned)((n_leaves + 255) / 256), 256, 0, st,
+                               d_cw, s.log_lanes, n_leaves, tree);
             mark("b3_leaves_small");
             ++launches;
         } else if (s.log_lanes <= 14) {
             const int log_c = s.log_lanes - 6;
             const uint64_t n_chunks = n_leaves << log_c;
             const unsigned t = leaf_threads(n_chunks, log_c, num_sms);
+            // a CTA that is full of chunks has t >> log_c whole leaves
+            int most = 0;
+            while (n_chunks >= t && (t >> log_c) >> (most + 1)) ++most;
+            from = post ? leaf_levels(n_leaves, most) : 0;
             launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, d_cw,
-                           n_chunks, tree, log_c, s.chunk0);
+                           n_chunks, tree, log_c, s.chunk0, from, n_leaves);
             mark("b3_leaves_chunked");
             ++launches;
         } else {
@@ -322,7 +358,7 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
         const ShaWords pad = sha_pad_kw(s.leaf_bytes() * 8);
         if (n_leaves <= (uint64_t)kShaTreeSmallMax) {
             launch_chained(sha_tree_small, 1, (unsigned)n_leaves, 0, st, d_cw, s.log_lanes,
-                           (uint32_t)n_leaves, tree, pad);
+                           (uint32_t)n_leaves, tree, pad, post ? *post : RootPost{});
             mark("sha_tree_small");
             return 1;
         }
@@ -331,7 +367,7 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
         mark("sha_leaves");
         ++launches;
     }
-    launches += launch_levels(tree, n_leaves, s.hash_kind, st, log);
+    launches += launch_levels(tree, n_leaves, s.hash_kind, st, log, from, post);
     return launches;
 }
 

@@ -5,9 +5,21 @@
 #pragma once
 #include <stdint.h>
 
+#include "bz_internal.h"
 #include "hash.cuh"
 
 namespace bz {
+
+// The root o to mapped host memory, by the thread that the CTA's barrier has
+// ordered behind every write of the tree.  The host reads the words once it sees
+// the sequence number, instead of copying the root and waiting for the stream.
+__device__ __forceinline__ void post_root(const RootPost &p, const uint32_t o[8]) {
+    if (!p.seq) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        p.words[i] = (uint64_t)o[2 * i] | ((uint64_t)o[2 * i + 1] << 32);
+    asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p.seq), "r"(p.seq_val) : "memory");
+}
 
 // ---------------------------------------------------------------------------
 // BLAKE3 leaves, C >= 1 chunks per leaf, C <= 256.
@@ -19,10 +31,15 @@ namespace bz {
 //
 // Body: the CTA's blockDim.x chunks from chunk_base (a multiple of blockDim.x,
 // blockDim.x a multiple of C); cvs holds blockDim.x padded rows of 9 words.
+//
+// levels > 0 (at most log2 of the CTA's leaves): the CTA goes on merging its
+// leaves into that many levels of the tree above them (n_leaves leaves), whose
+// parents are the same PARENT merge as those inside a leaf.
 __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t n_chunks,
                                                        uint32_t *tree_leaves, int log_c,
                                                        uint64_t chunk0, uint64_t chunk_base,
-                                                       uint32_t (*cvs)[9]) {
+                                                       uint32_t (*cvs)[9], int levels = 0,
+                                                       uint64_t n_leaves = 0) {
     const uint64_t chunk = chunk_base + threadIdx.x;
     const uint64_t c_in_leaf = chunk0 + (chunk & ((1u << log_c) - 1));
     uint32_t cv[8];
@@ -48,10 +65,22 @@ __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t
 #pragma unroll
     for (int i = 0; i < 8; ++i) cvs[threadIdx.x][i] = cv[i];
     __syncthreads();
-    // In-leaf reduction: level s merges nodes (2j, 2j+1) within groups of C.
-    for (int s = 0; s < log_c; ++s) {
-        const int stride = 1 << s;
+    // Step s merges nodes (2j, 2j+1): inside the leaf below log_c, then the
+    // levels above.  The level of step s is stored when it is one of the tree.
+    uint64_t off = 0, cnt = n_leaves;  // the tree level's first node and size
+    for (int s = 0;; ++s) {
         const int t = threadIdx.x;
+        if (s >= log_c) {
+            if ((t & ((1 << s) - 1)) == 0 && chunk < n_chunks) {
+                const uint64_t node = off + (chunk >> s);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) tree_leaves[node * 8 + i] = cvs[t][i];
+            }
+            off += cnt;
+            cnt >>= 1;
+        }
+        if (s == log_c + levels) break;
+        const int stride = 1 << s;
         if ((t & ((stride << 1) - 1)) == 0 && t + stride < (int)blockDim.x) {
             uint32_t out[8];
             b3_parent(cvs[t], cvs[t + stride], out);
@@ -60,42 +89,41 @@ __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t
         }
         __syncthreads();
     }
-    if ((threadIdx.x & ((1 << log_c) - 1)) == 0 && chunk < n_chunks) {
-        const uint64_t leaf = chunk >> log_c;
+}
+
+// One BLAKE3 leaf of at most one chunk (leaf_bytes = 16 * 2^log_lanes <= 1024).
+__device__ __forceinline__ void b3_leaf_small(const uint4 *p, int log_lanes, uint32_t cv[8]) {
+    const uint32_t elems = 1u << log_lanes;  // 16-byte elements
+    const uint32_t bytes = elems * 16;
+    const uint32_t nblk = (bytes + 63) / 64;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) tree_leaves[leaf * 8 + i] = cvs[threadIdx.x][i];
+    for (int i = 0; i < 8; ++i) cv[i] = kIV[i];
+#pragma unroll 1
+    for (uint32_t blk = 0; blk < nblk; ++blk) {
+        uint32_t m[16];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t e = blk * 4 + q;
+            const uint4 v = e < elems ? p[e] : make_uint4(0, 0, 0, 0);
+            m[4 * q] = v.x;
+            m[4 * q + 1] = v.y;
+            m[4 * q + 2] = v.z;
+            m[4 * q + 3] = v.w;
+        }
+        const uint32_t len = min(64u, bytes - blk * 64);
+        const uint32_t flags =
+            (blk == 0 ? B3_CHUNK_START : 0) | (blk == nblk - 1 ? B3_CHUNK_END : 0);
+        b3_compress_cv(cv, m, 0, len, flags);
     }
 }
 
-// BLAKE3 leaves of at most one chunk (leaf_bytes = 16 * 2^log_lanes <= 1024).
 // Body: leaves first, first + step, .. below n_leaves.
 __device__ __forceinline__ void b3_leaves_small_body(const uint4 *cw, int log_lanes,
                                                      uint64_t n_leaves, uint32_t *tree_leaves,
                                                      uint64_t first, uint64_t step) {
     for (uint64_t leaf = first; leaf < n_leaves; leaf += step) {
-        const uint32_t elems = 1u << log_lanes;  // 16-byte elements
-        const uint32_t bytes = elems * 16;
-        const uint32_t nblk = (bytes + 63) / 64;
-        const uint4 *p = cw + leaf * elems;
         uint32_t cv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) cv[i] = kIV[i];
-        for (uint32_t blk = 0; blk < nblk; ++blk) {
-            uint32_t m[16];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t e = blk * 4 + q;
-                const uint4 v = e < elems ? p[e] : make_uint4(0, 0, 0, 0);
-                m[4 * q] = v.x;
-                m[4 * q + 1] = v.y;
-                m[4 * q + 2] = v.z;
-                m[4 * q + 3] = v.w;
-            }
-            const uint32_t len = min(64u, bytes - blk * 64);
-            const uint32_t flags =
-                (blk == 0 ? B3_CHUNK_START : 0) | (blk == nblk - 1 ? B3_CHUNK_END : 0);
-            b3_compress_cv(cv, m, 0, len, flags);
-        }
+        b3_leaf_small(cw + (leaf << log_lanes), log_lanes, cv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) tree_leaves[leaf * 8 + i] = cv[i];
     }
@@ -138,6 +166,7 @@ struct LevelsArgs {
     uint64_t n_in;
     int k;  // levels to produce (<= 9)
     int kind;
+    RootPost post;  // when the last level is the root
 };
 
 // Body: unit u (512 input nodes) with threads 0..255; any further threads of
@@ -174,6 +203,10 @@ __device__ __forceinline__ void merkle_levels_body(const LevelsArgs &a, uint64_t
             po[1] = make_uint4(o[4], o[5], o[6], o[7]);
         }
         __syncthreads();  // every read of this level precedes the overwrite
+        if (lv == a.k - 1) {
+            if (t == 0) post_root(a.post, o);
+            break;
+        }
         if (active) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) nodes[t][i] = o[i];

@@ -229,7 +229,7 @@ int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out, bool with
 
 // Enqueue NTT + Merkle for a commitment whose buffers exist.
 int enqueue_commit(bz_ctx *ctx, const Shape &s, const uint4 *d_msg, bz_commitment *c,
-                   cudaStream_t st, uint32_t schedule) {
+                   cudaStream_t st, uint32_t schedule, RootPost *post) {
     const uint4 *d_tw = nullptr;
     int rc = get_twiddles(ctx, s.k_code(), &d_tw);
     if (rc) return rc;
@@ -238,7 +238,8 @@ int enqueue_commit(bz_ctx *ctx, const Shape &s, const uint4 *d_msg, bz_commitmen
         rc = ensure_scratch(ctx, need);
         if (rc) return rc;
     }
-    int n = launch_commit_kernels(ctx, s, schedule, d_msg, c->d_cw, c->d_tree, d_tw, st, nullptr);
+    int n = launch_commit_kernels(ctx, s, schedule, d_msg, c->d_cw, c->d_tree, d_tw, st, nullptr,
+                                  post);
     ctx->launches += (uint64_t)n;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_err(ctx, BZ_ERR_CUDA, "kernel launch", e);
@@ -261,17 +262,20 @@ bz_aux_stream *get_aux(bz_ctx *ctx, cudaStream_t st) {
 
 int launch_commit_kernels(bz_ctx *ctx, const Shape &s, uint32_t schedule, const uint4 *d_msg,
                           uint4 *d_cw, uint8_t *d_tree, const uint4 *d_tw, cudaStream_t st,
-                          LaunchLog *log) {
+                          LaunchLog *log, RootPost *post) {
     if ((schedule >> SCHED_PIPE_SHIFT) & 3) {
         bz_aux_stream *ax = get_aux(ctx, st);
         if (ax) {
             const int n = launch_commit_pipelined(s, schedule, d_msg, d_cw, d_tree, d_tw, st, ax->s,
                                                   ax->ev, ctx->num_sms, log);
-            if (n >= 0) return n;
+            if (n >= 0) {
+                if (post) post->seq = nullptr;
+                return n;
+            }
         }
     }
     int n = launch_ntt(s, schedule, d_msg, d_cw, d_tw, st, ctx->num_sms, log);
-    n += launch_merkle(s, d_cw, d_tree, ctx->scratch, st, ctx->num_sms, log);
+    n += launch_merkle(s, d_cw, d_tree, ctx->scratch, st, ctx->num_sms, log, post);
     return n;
 }
 
@@ -587,8 +591,13 @@ int bz_timer_end(bz_ctx *ctx, float *ms) {
 uint64_t bz_kernel_launches(const bz_ctx *ctx) { return ctx ? ctx->launches.load() : 0; }
 
 // ---- commit ---------------------------------------------------------------
-int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
-                           const bz_params *params, bz_commitment **out) {
+// Roots of synchronous commits: 16 slots of the mapped mailbox from byte 1024
+// (32 bytes of root, the sequence number at byte 64), taken in turn.
+constexpr size_t kRootMbox = 1024, kRootSlotBytes = 128;
+constexpr uint32_t kRootSlots = 16;
+
+static int commit_device_enqueue(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
+                                 const bz_params *params, bz_commitment **out, RootPost *post) {
     if (!ctx || !d_msg || !out) return BZ_ERR_ARG;
     *out = nullptr;
     Shape s;
@@ -598,7 +607,7 @@ int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
     bz_commitment *c = nullptr;
     rc = alloc_commitment(ctx, s, &c);
     if (rc) return rc;
-    rc = enqueue_commit(ctx, s, (const uint4 *)d_msg, c, ctx->stream, schedule_for(ctx, s));
+    rc = enqueue_commit(ctx, s, (const uint4 *)d_msg, c, ctx->stream, schedule_for(ctx, s), post);
     if (rc) {
         bz_commitment_free(c);
         return rc;
@@ -607,11 +616,31 @@ int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
     return BZ_OK;
 }
 
+int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
+                           const bz_params *params, bz_commitment **out) {
+    return commit_device_enqueue(ctx, d_msg, n_words, params, out, nullptr);
+}
+
 int bz_commit_device(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words, const bz_params *params,
                      bz_commitment **out, uint8_t root[32]) {
-    int rc = bz_commit_device_async(ctx, d_msg, n_words, params, out);
+    if (!ctx) return BZ_ERR_ARG;
+    const uint32_t seq = ++ctx->root_seq;
+    const size_t slot = kRootMbox + (seq % kRootSlots) * kRootSlotBytes;
+    RootPost post;
+    post.words = (uint64_t *)((uint8_t *)ctx->d_mbox + slot);
+    post.seq = (uint32_t *)((uint8_t *)ctx->d_mbox + slot + 64);
+    post.seq_val = seq;
+    int rc = commit_device_enqueue(ctx, d_msg, n_words, params, out, &post);
     if (rc) return rc;
-    rc = fetch_root(*out);
+    if (post.seq) {
+        rc = mapped_wait(ctx, slot + 64, seq, "commit");
+        if (!rc) {
+            memcpy((*out)->root, (const uint8_t *)ctx->h_mbox + slot, 32);
+            (*out)->root_ready = true;
+        }
+    } else {
+        rc = fetch_root(*out);
+    }
     if (rc) {
         bz_commitment_free(*out);
         *out = nullptr;

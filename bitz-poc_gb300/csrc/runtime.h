@@ -56,6 +56,7 @@ struct bz_ctx {
     void *h_mbox = nullptr;   // 4 KiB mapped pinned: sumcheck message mailbox
     void *d_mbox = nullptr;   // its device view
     uint32_t mbox_seq = 0;    // last posted sequence number
+    std::atomic<uint32_t> root_seq{0};  // commits whose root the mailbox was offered to
     uint32_t gate_seq = 0;    // last armed fold's gate number
     bool arm_folds = true;    // cleared after a gate ran out (the prover stops arming)
     uint32_t pow_seq = 0;     // last proof-of-work search's mailbox number
@@ -128,8 +129,10 @@ int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out);
 uint32_t schedule_for(bz_ctx *ctx, const Shape &s);
 int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out,
                      bool with_codeword = true);
+// With `post`, the commit's last kernel posts the root; post->seq is null on
+// return when it does not (the two-stream pipeline).
 int enqueue_commit(bz_ctx *ctx, const Shape &s, const uint4 *d_msg, bz_commitment *c,
-                   cudaStream_t st, uint32_t schedule);
+                   cudaStream_t st, uint32_t schedule, RootPost *post = nullptr);
 int fetch_root(bz_commitment *c);
 // The auxiliary stream paired with `st` (created on first use; call before a
 // stream capture that will use it).
@@ -138,7 +141,7 @@ bz_aux_stream *get_aux(bz_ctx *ctx, cudaStream_t st);
 // schedule asks for it and the shape allows it, else the plain sequence.
 int launch_commit_kernels(bz_ctx *ctx, const Shape &s, uint32_t schedule, const uint4 *d_msg,
                           uint4 *d_cw, uint8_t *d_tree, const uint4 *d_tw, cudaStream_t st,
-                          LaunchLog *log);
+                          LaunchLog *log, RootPost *post = nullptr);
 
 // Sumcheck rounds on the context stream.  fold_launch enqueues one
 // fold-and-message round with a known challenge; msg_wait returns its
