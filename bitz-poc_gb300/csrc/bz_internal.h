@@ -179,8 +179,8 @@ int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_p
                      const MsgPost *post = nullptr);
 int launch_partial_eval_round(const uint4 *d_in, size_t n, uint4 r, uint4 *d_out,
                               cudaStream_t st);
-int launch_build_eq(const uint4 *d_point_dev, size_t k, uint4 *d_out, cudaStream_t st,
-                    int num_sms);
+// eq over the k coordinates of `point` (host memory, 2 words each)
+int launch_build_eq(const uint64_t *point, size_t k, uint4 *d_out, cudaStream_t st, int num_sms);
 int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_partials,
                    uint4 *d_sv, cudaStream_t st, int num_sms);
 size_t sv_partials_bytes(int num_sms);
@@ -193,16 +193,18 @@ int launch_chacha(uint64_t seed, uint64_t first_word, uint4 *d_out, size_t n_wor
 // Batched grand-product GKR (BitZ src/bitz/gkr.rs; fold.cu): one product
 // layer (out[i] = in[i] * in[half + i]), one dense round over h slots of the
 // two half tables (with the previous round's fold by rho first when `fold`;
-// the reduced (sum_end, sum_inf) land in d_out[0..3]; d_w_next, when not
-// null, gets the next round's weights), and the forest's leaf grid.
-// d_partials holds fold_partials_bytes(0) bytes.  With `post` the round's
-// last CTA posts the sums to the mapped mailbox (as the sumcheck rounds do)
-// and d_out is unused.
+// d_w_next, when not null, gets the next round's weights), and the forest's
+// leaf grid.  d_partials holds fold_partials_bytes(0) bytes.  The round posts
+// (sum_end, sum_inf) to the mapped mailbox as the sumcheck rounds do and, when
+// h = 1, first the four entries it leaves to d_tail (mapped, 8 words).  With
+// `gate` (rounds of one CTA, folding) rho comes through the gate.
 int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_t st,
                        int num_sms);
+int gkr_round_grid(size_t h, int num_sms);
 int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fold, uint4 rho,
-                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, uint64_t *d_out,
-                     cudaStream_t st, int num_sms, const MsgPost *post = nullptr);
+                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, cudaStream_t st,
+                     int num_sms, const MsgPost &post, uint64_t *d_tail,
+                     const RGate *gate = nullptr);
 int launch_gkr_forest_leaves(const uint64_t *d_packed, const uint4 *d_images, int t, int s,
                              uint4 *d_out, cudaStream_t st, int num_sms);
 

@@ -345,10 +345,16 @@ int launch_partial_eval_round(const uint4 *d_in, size_t n, uint4 r, uint4 *d_out
     return 1;
 }
 
+// The point of an eq table is a kernel argument: no upload and no buffer, and
+// the small tables are built while the previous kernel still runs.
+constexpr int kEqSplitMaxK = 22;
+struct EqPoint {
+    uint4 r[kEqSplitMaxK];
+};
+
 // eq table rounds: entries [0, half) double into [0, 2 half).
-__global__ void eq_round_kernel(uint4 *eq, uint64_t half, const uint4 *point, int i) {
+__global__ void eq_round_kernel(uint4 *eq, uint64_t half, uint4 r) {
     chain_wait();
-    const uint4 r = point[i];
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < half;
          j += (uint64_t)gridDim.x * blockDim.x) {
         const uint4 p = eq[j];
@@ -360,12 +366,13 @@ __global__ void eq_round_kernel(uint4 *eq, uint64_t half, const uint4 *point, in
 
 // The first k rounds in one CTA (global writes of a round are visible to the
 // CTA's threads after the barrier).
-__global__ void __launch_bounds__(512) eq_small_kernel(uint4 *eq, const uint4 *point, int k) {
+__global__ void __launch_bounds__(512) eq_small_kernel(uint4 *eq, const __grid_constant__ EqPoint point,
+                                                       int k) {
     chain_wait();
     if (threadIdx.x == 0) eq[0] = make_uint4(1, 0, 0, 0);
     __syncthreads();
     for (int i = 0; i < k; ++i) {
-        const uint4 r = point[i];
+        const uint4 r = point.r[i];
         const uint32_t half = 1u << i;
         for (uint32_t j = threadIdx.x; j < half; j += blockDim.x) {
             const uint4 p = eq[j];
@@ -383,10 +390,9 @@ __global__ void __launch_bounds__(512) eq_small_kernel(uint4 *eq, const uint4 *p
 // doubling rounds (bit i of j picks r_i or 1 + r_i), so the entries are
 // identical.  Each CTA builds both halves in shared memory (their rounds side
 // by side), then writes its share of the products.
-constexpr int kEqSplitMaxK = 22;
-__global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *point, int k,
-                                                       int a) {
-    chain_wait();
+__global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq,
+                                                       const __grid_constant__ EqPoint point,
+                                                       int k, int a) {
     extern __shared__ uint4 halves[];
     const int b = k - a;
     uint4 *lo = halves, *hi = halves + ((size_t)1 << a);
@@ -401,7 +407,7 @@ __global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *p
             const bool in_lo = j < nlo;
             uint4 *t = in_lo ? lo : hi;
             const uint32_t jj = in_lo ? j : j - nlo;
-            const uint4 r = point[in_lo ? i : a + i];
+            const uint4 r = point.r[in_lo ? i : a + i];
             const uint4 p = t[jj];
             const uint4 one = gf_mul(p, r);
             t[(1u << i) + jj] = one;
@@ -409,6 +415,7 @@ __global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *p
         }
         __syncthreads();
     }
+    chain_wait();
     const uint64_t n = (uint64_t)1 << k;
     const uint64_t mask = ((uint64_t)1 << a) - 1;
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
@@ -426,13 +433,15 @@ __global__ void __launch_bounds__(512) eq_split_kernel(uint4 *eq, const uint4 *p
 constexpr int kEqRowsK = 18;
 constexpr int kEqThreads = 512;
 constexpr int kEqHeadRows = 64;  // rows whose hi a CTA forms at a time
-__global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq, const uint4 *point, int k,
-                                                             int a) {
-    chain_wait();
+__global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq,
+                                                             const __grid_constant__ EqPoint point,
+                                                             int k, int a) {
     extern __shared__ uint4 lo[];  // 2^a, then the row's byte tables
     __shared__ uint4 quarter[4][1 << ((kEqSplitMaxK + 3) / 4)];
     __shared__ uint4 head[kEqHeadRows];
+    __shared__ uint4 pt[kEqSplitMaxK];
     const int b = k - a, a0 = a / 2, b0 = b / 2;
+    if (threadIdx.x < kEqSplitMaxK) pt[threadIdx.x] = point.r[threadIdx.x];
     {
         const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
         const int first = g == 0 ? 0 : g == 1 ? a0 : g == 2 ? a : a + b0;
@@ -443,7 +452,7 @@ __global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq, const ui
         for (int i = 0; i < rounds; ++i) {
             if (i < nv && t < (1 << i)) {
                 const uint4 p = quarter[g][t];
-                const uint4 one = gf_mul(p, point[first + i]);
+                const uint4 one = gf_mul(p, pt[first + i]);
                 quarter[g][(1 << i) + t] = one;
                 quarter[g][t] = gf_add(p, one);
             }
@@ -455,6 +464,7 @@ __global__ void __launch_bounds__(kEqThreads) eq_rows_kernel(uint4 *eq, const ui
     lc.init();
     for (uint32_t j = threadIdx.x; j < (1u << a); j += kEqThreads)
         lo[j] = gf_mul(quarter[0][j & ((1u << a0) - 1)], quarter[1][j >> a0]);
+    chain_wait();
     const uint32_t rows = 1u << b;
     uint32_t at = kEqHeadRows;  // rows of head[] taken
     for (uint32_t h = blockIdx.x; h < rows; h += gridDim.x, ++at) {
@@ -479,30 +489,35 @@ constexpr size_t kEqSmallRounds = 12;
 // launch (2^12 entries: 3 to 4 us of products after 6 half-table rounds,
 // against 12 rounds in one CTA; 2^20: one launch instead of nine).  Above:
 // 12 rounds in one CTA, then one launch per further round.
-int launch_build_eq(const uint4 *d_point, size_t k, uint4 *d_out, cudaStream_t st,
+int launch_build_eq(const uint64_t *point, size_t k, uint4 *d_out, cudaStream_t st,
                     int num_sms) {
+    auto r = [&](size_t i) {
+        return make_uint4((uint32_t)point[2 * i], (uint32_t)(point[2 * i] >> 32),
+                          (uint32_t)point[2 * i + 1], (uint32_t)(point[2 * i + 1] >> 32));
+    };
+    EqPoint pt{};
+    for (size_t i = 0; i < std::min(k, (size_t)kEqSplitMaxK); ++i) pt.r[i] = r(i);
     if (k > 6 && k <= (size_t)kEqSplitMaxK) {
         const int a = (int)k / 2;
         if ((int)k >= kEqRowsK) {
             const unsigned grid = std::min(1u << (k - a), 2u * (unsigned)num_sms);
             launch_chained(eq_rows_kernel, grid, kEqThreads, (sizeof(uint4) << a) + kT8Bytes, st,
-                           d_out, d_point, (int)k, a);
+                           d_out, pt, (int)k, a);
             return 1;
         }
         const size_t smem = (((size_t)1 << a) + ((size_t)1 << (k - a))) * sizeof(uint4);
         const uint64_t n = (uint64_t)1 << k;
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((n + 511) / 512, (uint64_t)2 * num_sms));
-        launch_chained(eq_split_kernel, grid, 512, smem, st, d_out, d_point, (int)k, a);
+        launch_chained(eq_split_kernel, grid, 512, smem, st, d_out, pt, (int)k, a);
         return 1;
     }
     const size_t k0 = std::min(k, kEqSmallRounds);
-    launch_chained(eq_small_kernel, 1, 512, 0, st, d_out, d_point, (int)k0);
+    launch_chained(eq_small_kernel, 1, 512, 0, st, d_out, pt, (int)k0);
     for (size_t i = k0; i < k; ++i) {
         const uint64_t half = (uint64_t)1 << i;
         const unsigned grid = (unsigned)std::min<uint64_t>((half + 255) / 256, 8192);
-        launch_chained(eq_round_kernel, std::max(grid, 1u), 256, 0, st, d_out, half, d_point,
-                       (int)i);
+        launch_chained(eq_round_kernel, std::max(grid, 1u), 256, 0, st, d_out, half, r(i));
     }
     return (int)(k - k0) + 1;
 }
@@ -742,13 +757,23 @@ __global__ void __launch_bounds__(256) gkr_product_kernel(const uint4 *in, uint6
 // finish kernel reduces them.  With w_next, the next round's weights
 // w_next[c] = w[c] + w[c + h/2] (eq over one coordinate fewer: the two
 // values of the dropped coordinate's factor sum to 1) are written too.
-template <bool FOLD>
+//
+// A round of one slot also posts the four entries it leaves (l[0], l[1], r[0],
+// r[1]) to `tail`, ahead of its sums, so the layer's close needs no copy.
+// GATED: launched before rho is known, as the sumcheck's armed folds; for
+// launches of one CTA, because the fold is in place and a gate that runs out
+// must leave the whole round undone.
+template <bool FOLD, bool GATED>
 __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, const uint4 *w,
                                                            uint64_t h, uint4 rho, int send_one,
                                                            uint64_t *partials, MsgMailbox mb,
-                                                           uint4 *w_next) {
+                                                           uint4 *w_next, uint64_t *tail,
+                                                           RGate gate) {
     chain_wait();
     extern __shared__ uint4 smem[];
+    if constexpr (GATED) {
+        if (!gate_wait(gate, rho)) return;
+    }
     const char *T = nullptr;
     T16Lane8 lc;
     if constexpr (FOLD) {
@@ -781,6 +806,14 @@ __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, c
         const uint4 le = send_one ? l1 : l0, re = send_one ? r1 : r0;
         gf_wide_xor(e, gf_mul_wide(gf_mul(wc, le), re));
         gf_wide_xor(f, gf_mul_wide(gf_mul(wc, gf_add(l1, l0)), gf_add(r1, r0)));
+        if (tail && h == 1) {
+            const uint4 v[4] = {l0, l1, r0, r1};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                tail[2 * i] = lo64(v[i]);
+                tail[2 * i + 1] = hi64(v[i]);
+            }
+        }
     }
     msg_finish_call(e, f, partials, mb);
 }
@@ -812,24 +845,26 @@ int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_
 int gkr_round_grid(size_t h, int num_sms) { return std::min(msg_grid(h, num_sms), 1024); }
 
 int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fold, uint4 rho,
-                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, uint64_t *d_out,
-                     cudaStream_t st, int num_sms, const MsgPost *post) {
+                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, cudaStream_t st,
+                     int num_sms, const MsgPost &post, uint64_t *d_tail, const RGate *gate) {
     const int grid = gkr_round_grid(h, num_sms);
-    MsgMailbox mb;
-    if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
-    if (fold)
-        launch_chained(gkr_round_kernel<true>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h, rho,
-                       send_one, d_partials, mb, d_w_next);
+    const MsgMailbox mb = {post.ticket, post.words, post.seq, post.seq_val};
+    if (gate)
+        launch_chained(gkr_round_kernel<true, true>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h,
+                       rho, send_one, d_partials, mb, d_w_next, d_tail, *gate);
+    else if (fold)
+        launch_chained(gkr_round_kernel<true, false>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h,
+                       rho, send_one, d_partials, mb, d_w_next, d_tail, RGate{});
     else
-        launch_chained(gkr_round_kernel<false>, grid, 256, 0, st, d_l, d_r, d_w, h, rho, send_one,
-                       d_partials, mb, d_w_next);
-    if (post) return 1;
-    launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_out);
-    return 2;
+        launch_chained(gkr_round_kernel<false, false>, grid, 256, 0, st, d_l, d_r, d_w, h, rho,
+                       send_one, d_partials, mb, d_w_next, d_tail, RGate{});
+    return 1;
 }
 
 void init_gkr_kernels() {
-    cudaFuncSetAttribute(gkr_round_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(gkr_round_kernel<true, false>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRTableSmem);
+    cudaFuncSetAttribute(gkr_round_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kRTableSmem);
 }
 

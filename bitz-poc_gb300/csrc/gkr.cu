@@ -75,6 +75,23 @@ struct DevBuf {
     }
 };
 
+// A GKR round's gate waits for the caller's transcript.  A transcript that
+// takes longer (or waits on the context's stream, which the armed round holds)
+// costs this once per context; the round then runs unarmed.
+constexpr uint64_t kGkrGateLimitNs = 2000000ull;
+
+// The armed round, withdrawn when the proof ends early.
+struct Armed {
+    bz_ctx *ctx;
+    ArmedFold fold;
+    MsgPost post{};
+    explicit Armed(bz_ctx *c) : ctx(c) {}
+    void cancel() {
+        if (fold.live) fold_cancel(ctx, &fold);
+    }
+    ~Armed() { cancel(); }
+};
+
 // The whole proof from device leaves (n of them, overwritten: the leaf layer
 // is folded in place as the rounds go).
 int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_t *point,
@@ -88,11 +105,13 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
     if (!rc) rc = dev_alloc(ctx, std::max<size_t>(n / 4, 1) * 16, &eqa.p, false);
     if (!rc) rc = dev_alloc(ctx, std::max<size_t>(n / 4, 1) * 16, &eqb.p, false);
     const size_t part_bytes = fold_partials_bytes(0);
-    if (!rc) rc = dev_alloc(ctx, part_bytes + 64 * 16 + 64, &scratch.p, false);
+    if (!rc) rc = dev_alloc(ctx, part_bytes, &scratch.p, false);
     if (rc) return rc;
     uint64_t *d_partials = (uint64_t *)scratch.p;
-    uint4 *d_point = (uint4 *)((uint8_t *)scratch.p + part_bytes);
-    uint64_t *d_msg = (uint64_t *)((uint8_t *)scratch.p + part_bytes + 64 * 16);
+    // the last round's four entries, at byte 512 of the mapped mailbox
+    uint64_t *d_tail = (uint64_t *)((uint8_t *)ctx->d_mbox + 512);
+    const volatile uint64_t *h_tail = (const volatile uint64_t *)((uint8_t *)ctx->h_mbox + 512);
+    Armed armed{ctx};
     std::vector<uint4 *> layer(layers + 1);
     layer[0] = d_leaves;
     size_t off = 0;
@@ -125,26 +144,63 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                 ext[2 * i] = p[k - 1 - i].w[0];
                 ext[2 * i + 1] = p[k - 1 - i].w[1];
             }
-            if (k > 1)
-                BZ_CUDA(ctx, cudaMemcpyAsync(d_point, ext.data(), (size_t)(k - 1) * 16,
-                                             cudaMemcpyHostToDevice, st));
-            ctx->launches += launch_build_eq(d_point, (size_t)(k - 1), (uint4 *)eqa.p, st,
+            ctx->launches += launch_build_eq(ext.data(), (size_t)(k - 1), (uint4 *)eqa.p, st,
                                              ctx->num_sms);
             uint4 *w = (uint4 *)eqa.p, *w_next = (uint4 *)eqb.p;
-            for (int rnd = 0; rnd < k; ++rnd) {
+            // enqueue round rnd; with a gate its rho is not known yet
+            auto launch = [&](int rnd, const MsgPost &post, const RGate *gate) -> int {
                 const int remaining = k - 1 - rnd;
-                const size_t h = (size_t)1 << remaining;
+                ctx->launches += launch_gkr_round(
+                    l, r, w, (size_t)1 << remaining, rnd > 0, to_u4(rho), gzero(p[rnd]),
+                    remaining ? w_next : nullptr, d_partials, st, ctx->num_sms, post, d_tail, gate);
+                BZ_CUDA(ctx, cudaGetLastError());
+                return BZ_OK;
+            };
+            for (int rnd = 0; rnd < k; ++rnd) {
                 const Gf &z = p[rnd];
                 // the round's last CTA posts the two sums to the mapped
                 // mailbox: no finish kernel, copy or stream synchronisation
-                const MsgPost post = next_msg_post(ctx);
-                ctx->launches += launch_gkr_round(l, r, w, h, pending, to_u4(rho), gzero(z),
-                                                  remaining ? w_next : nullptr, d_partials,
-                                                  d_msg, st, ctx->num_sms, &post);
-                BZ_CUDA(ctx, cudaGetLastError());
+                const bool was_armed = armed.fold.live;
+                MsgPost post = armed.post;
+                if (was_armed) {
+                    fold_open(ctx, &armed.fold, rho.w);
+                } else {
+                    post = next_msg_post(ctx);
+                    if ((rc = launch(rnd, post, nullptr))) return rc;
+                }
+                std::swap(w, w_next);
+                // The next round of one CTA is enqueued behind this one, and
+                // waits on the device for the challenge: its launch overlaps
+                // the wait, the sums' host work and the transcript.
+                if (rnd + 1 < k && ctx->arm_gkr &&
+                    gkr_round_grid((size_t)1 << (k - 2 - rnd), ctx->num_sms) == 1) {
+                    const RGate g = next_gate(ctx, kGkrGateLimitNs);
+                    armed.post = next_msg_post(ctx);
+                    if ((rc = launch(rnd + 1, armed.post, &g))) return rc;
+                    armed.fold.gate_seq = g.seq;
+                    armed.fold.live = true;
+                }
                 Gf se, si;
                 rc = msg_wait(ctx, post.seq_val, se.w, si.w);
+                if (rc && was_armed) {
+                    // the gate ran out before the challenge came (a transcript
+                    // that took long or used the context's stream): the round
+                    // was left undone, so run it unarmed and arm no further
+                    if (armed.fold.live) fold_cancel(ctx, &armed.fold);
+                    const bool arm_folds = ctx->arm_folds;
+                    const bool gave_up = gate_gave_up(ctx);
+                    ctx->arm_folds = arm_folds;
+                    if (gave_up) {
+                        ctx->arm_gkr = false;
+                        std::swap(w, w_next);
+                        post = next_msg_post(ctx);
+                        if ((rc = launch(rnd, post, nullptr))) return rc;
+                        std::swap(w, w_next);
+                        rc = msg_wait(ctx, post.seq_val, se.w, si.w);
+                    }
+                }
                 if (rc) {
+                    armed.cancel();
                     reset_msg_ticket(ctx);
                     return rc;
                 }
@@ -158,16 +214,19 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                 rho = ch;
                 pending = true;
                 factor = gmul(factor, eq_factor(ch, z));
-                std::swap(w, w_next);
             }
         }
         // the close (gkr.rs:270-281): the last fold of the two-entry halves
-        // two entries per half still to fold, or (a layer without rounds) one
+        // two entries per half still to fold, posted by the last round, or (a
+        // layer without rounds) one
         uint64_t lr[8] = {0};
-        const size_t take = pending ? 32 : 16;
-        BZ_CUDA(ctx, cudaMemcpyAsync(lr, l, take, cudaMemcpyDeviceToHost, st));
-        BZ_CUDA(ctx, cudaMemcpyAsync(lr + 4, r, take, cudaMemcpyDeviceToHost, st));
-        BZ_CUDA(ctx, cudaStreamSynchronize(st));
+        if (pending) {
+            for (int i = 0; i < 8; ++i) lr[i] = h_tail[i];
+        } else {
+            BZ_CUDA(ctx, cudaMemcpyAsync(lr, l, 16, cudaMemcpyDeviceToHost, st));
+            BZ_CUDA(ctx, cudaMemcpyAsync(lr + 4, r, 16, cudaMemcpyDeviceToHost, st));
+            BZ_CUDA(ctx, cudaStreamSynchronize(st));
+        }
         Gf l0, l1, r0, r1;
         l0.w[0] = lr[0], l0.w[1] = lr[1], l1.w[0] = lr[2], l1.w[1] = lr[3];
         r0.w[0] = lr[4], r0.w[1] = lr[5], r1.w[0] = lr[6], r1.w[1] = lr[7];

@@ -203,17 +203,14 @@ struct Sumcheck {
         while (((size_t)1 << n) < len) ++n;
         const size_t parts = bz::dot_partials_count(len, ctx->num_sms);
         void *scratch = nullptr;
-        const size_t bytes = (len + n + 1 + parts) * 16;
+        const size_t bytes = (len + 1 + parts) * 16;
         int rc = bz::dev_alloc(ctx, bytes, &scratch, false);
         if (rc) return rc;
-        uint4 *d_eq = (uint4 *)scratch, *d_z = d_eq + len, *d_y = d_z + n,
-              *d_part = d_y + 1;
+        uint4 *d_eq = (uint4 *)scratch, *d_y = d_eq + len, *d_part = d_y + 1;
         std::vector<uint64_t> z(2 * (size_t)n);
         for (uint32_t s = 0; s < count && !rc; ++s) {
             for (uint32_t i = 0; i < n; ++i) tr->sample_f128(&z[2 * i]);
-            if (n) cudaMemcpyAsync(d_z, z.data(), 16 * (size_t)n, cudaMemcpyHostToDevice,
-                                   ctx->stream);
-            ctx->launches += bz::launch_build_eq(d_z, n, d_eq, ctx->stream, ctx->num_sms);
+            ctx->launches += bz::launch_build_eq(z.data(), n, d_eq, ctx->stream, ctx->num_sms);
             uint64_t u0[2], u2[2], y[2];
             rc = bz_round_msg_lsb(ctx, f, (const uint64_t *)d_eq, len, u0, u2);
             if (rc) break;
@@ -311,22 +308,20 @@ int induce_basis(bz_ctx *ctx, uint32_t log_msg_cols, uint32_t rate,
     const size_t q = queries.size();
     const size_t n_alpha = alpha.size() / 2;
     const size_t n_w = (size_t)1 << n_alpha;  // eq(alpha) has 2^n_alpha >= q entries
-    const size_t bytes = (((size_t)1 << log_d) + n_w + n_alpha) * 16 + q * 8 + 16;
+    const size_t bytes = (((size_t)1 << log_d) + n_w) * 16 + q * 8 + 16;
     void *mem = nullptr;
     int rc = bz::dev_alloc(ctx, bytes, &mem, false);
     if (rc) return rc;
-    uint4 *d_dom = (uint4 *)mem, *d_w = d_dom + ((size_t)1 << log_d), *d_alpha = d_w + n_w;
-    uint64_t *d_pos = (uint64_t *)(d_alpha + n_alpha);
+    uint4 *d_dom = (uint4 *)mem, *d_w = d_dom + ((size_t)1 << log_d);
+    uint64_t *d_pos = (uint64_t *)(d_w + n_w);
     const uint4 *d_tw = nullptr;
     rc = bz::get_twiddles(ctx, log_d, &d_tw);
     if (rc) {
         bz::dev_free(ctx, mem, bytes, false);
         return rc;
     }
-    if (n_alpha)
-        cudaMemcpyAsync(d_alpha, alpha.data(), 16 * n_alpha, cudaMemcpyHostToDevice, ctx->stream);
     if (q) cudaMemcpyAsync(d_pos, queries.data(), 8 * q, cudaMemcpyHostToDevice, ctx->stream);
-    ctx->launches += bz::launch_build_eq(d_alpha, n_alpha, d_w, ctx->stream, ctx->num_sms);
+    ctx->launches += bz::launch_build_eq(alpha.data(), n_alpha, d_w, ctx->stream, ctx->num_sms);
     ctx->launches += bz::launch_induce_basis(d_dom, log_d, d_pos, d_w, (int)q, d_tw, ctx->stream);
     if (cudaGetLastError() != cudaSuccess) {
         bz::dev_free(ctx, mem, bytes, false);

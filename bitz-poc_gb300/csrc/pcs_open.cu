@@ -100,17 +100,15 @@ struct EqSplit {
         lo = (int)(vars < (uint32_t)kOodBlockLog ? vars : kOodBlockLog);
         const uint32_t hi_vars = vars - (uint32_t)lo;
         n_head = (size_t)1 << hi_vars;
-        bytes = (((size_t)1 << lo) + n_head + vars + 1) * 16;
+        bytes = (((size_t)1 << lo) + n_head) * 16;
         int rc = bz::dev_alloc(ctx, bytes, &mem, false);
         if (rc) return rc;
         tail = (uint4 *)mem;
         head = tail + ((size_t)1 << lo);
-        uint4 *d_pt = head + n_head;
-        if (vars)
-            cudaMemcpyAsync(d_pt, point.data(), 16 * (size_t)vars, cudaMemcpyHostToDevice,
-                            ctx->stream);
-        ctx->launches += bz::launch_build_eq(d_pt, (size_t)lo, tail, ctx->stream, ctx->num_sms);
-        ctx->launches += bz::launch_build_eq(d_pt + lo, hi_vars, head, ctx->stream, ctx->num_sms);
+        ctx->launches += bz::launch_build_eq(point.data(), (size_t)lo, tail, ctx->stream,
+                                             ctx->num_sms);
+        ctx->launches += bz::launch_build_eq(point.data() + 2 * lo, hi_vars, head, ctx->stream,
+                                             ctx->num_sms);
         return cudaGetLastError() == cudaSuccess ? BZ_OK
                                                  : bz::set_msg(ctx, BZ_ERR_CUDA, "eq tables");
     }

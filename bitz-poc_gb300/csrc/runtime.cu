@@ -960,11 +960,7 @@ bool gate_gave_up(bz_ctx *ctx) {
     return true;
 }
 
-int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, uint64_t *d_nf,
-             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns) {
-    if (a->live) return set_msg(ctx, BZ_ERR_STATE, "a fold is already armed");
-    int rc = ensure_scratch(ctx, fold_partials_bytes(n));
-    if (rc) return rc;
+RGate next_gate(bz_ctx *ctx, uint64_t limit_ns) {
     if (++ctx->gate_seq >= kGateCancel) ctx->gate_seq = 1;
     RGate g;
     g.r = (const uint64_t *)((uint8_t *)ctx->d_mbox + 128);
@@ -972,6 +968,15 @@ int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, ui
     g.seq = ctx->gate_seq;
     g.err = (uint32_t *)((uint8_t *)ctx->d_small + 832);
     g.limit_ns = limit_ns;
+    return g;
+}
+
+int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, uint64_t *d_nf,
+             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns) {
+    if (a->live) return set_msg(ctx, BZ_ERR_STATE, "a fold is already armed");
+    int rc = ensure_scratch(ctx, fold_partials_bytes(n));
+    if (rc) return rc;
+    const RGate g = next_gate(ctx, limit_ns);
     const MsgPost post = next_post(ctx);
     ctx->launches += launch_fold_and_msg((const uint4 *)d_f, (const uint4 *)d_b, n,
                                          make_uint4(0, 0, 0, 0), (uint4 *)d_nf, (uint4 *)d_nb,
@@ -1098,13 +1103,7 @@ int bz_partial_eval_lsb(bz_ctx *ctx, const uint64_t *d_in, size_t n, const uint6
 int bz_build_eq_lsb(bz_ctx *ctx, const uint64_t *point, size_t k, uint64_t *d_out) {
     if (!ctx || !d_out || (k && !point)) return BZ_ERR_ARG;
     if (k > 40) return set_msg(ctx, BZ_ERR_SHAPE, "k too large");
-    void *d_pt = nullptr;
-    int rc = dev_alloc(ctx, (k ? k : 1) * 16, &d_pt, false);
-    if (rc) return rc;
-    if (k) cudaMemcpyAsync(d_pt, point, k * 16, cudaMemcpyHostToDevice, ctx->stream);
-    ctx->launches +=
-        launch_build_eq((const uint4 *)d_pt, k, (uint4 *)d_out, ctx->stream, ctx->num_sms);
-    dev_free(ctx, d_pt, 0, false);
+    ctx->launches += launch_build_eq(point, k, (uint4 *)d_out, ctx->stream, ctx->num_sms);
     BZ_CUDA(ctx, cudaGetLastError());
     BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return BZ_OK;

@@ -59,6 +59,7 @@ struct bz_ctx {
     std::atomic<uint32_t> root_seq{0};  // commits whose root the mailbox was offered to
     uint32_t gate_seq = 0;    // last armed fold's gate number
     bool arm_folds = true;    // cleared after a gate ran out (the prover stops arming)
+    bool arm_gkr = true;      // the same for GKR rounds, whose transcript is the caller's
     uint32_t pow_seq = 0;     // last proof-of-work search's mailbox number
     bool pow_ready = false;   // the search's device counters hold their idle values
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -163,6 +164,8 @@ int fold_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
 bool fold_armable(const bz_ctx *ctx, size_t n);
 int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, uint64_t *d_nf,
              uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns = kGateLimitNs);
+// The gate of the next armed launch (its number is what fold_open posts).
+RGate next_gate(bz_ctx *ctx, uint64_t limit_ns);
 void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]);
 int fold_cancel(bz_ctx *ctx, ArmedFold *a);
 // After a gated round's message failed to arrive: drains the stream and
