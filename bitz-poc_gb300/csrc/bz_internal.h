@@ -149,27 +149,31 @@ int launch_gather_nodes(const uint8_t *d_tree, const uint64_t *d_idx, size_t n, 
 // kernel, no copy); without it a finish kernel writes d_msg_out.
 struct MsgPost {
     unsigned int *ticket;  // device counter, 0 between launches
-    uint64_t *words;       // device view of mapped host memory (4 words)
-    uint32_t *seq;         // device view of mapped host memory
+    uint64_t *words;       // device view of mapped host memory (6 tagged words a post)
     uint32_t seq_val;
 };
+// Posts of a message kernel of `grid` CTAs: one by each CTA, whose sum is the
+// message, or one by the last.
+constexpr int kMsgPosts = 16;
+__host__ __device__ inline int msg_posts(int grid) { return grid <= kMsgPosts ? grid : 1; }
 // Challenge gate of a fold launched ahead of its challenge: the host writes r
-// to mapped memory, then the sequence number to `go` (or seq | kGateCancel to
-// cancel).  The kernel waits at most limit_ns, then sets bit 0 of *err.  The
+// to mapped memory as three words of 44 bits tagged with the gate's number
+// (or the first word tagged seq | kGateCancel to cancel).  The kernel waits at most limit_ns, then sets bit 0 of *err.  The
 // host posts r within microseconds; the limit only bounds a gate that nothing
 // opens (an error path, or a tool that runs each launch to completion before
 // returning), and the prover then runs the round again unarmed.
-constexpr uint32_t kGateCancel = 0x80000000u;
+constexpr uint32_t kGateCancel = 0x80000u;  // of a 20-bit tag
 constexpr uint64_t kGateLimitNs = 100000000ull;  // 100 ms
 struct RGate {
-    const uint32_t *go = nullptr;  // device view of mapped host memory
-    const uint64_t *r = nullptr;   // device view of mapped host memory: r.lo, r.hi
-    uint32_t seq = 0;              // 1 .. kGateCancel - 1
+    const uint64_t *words = nullptr;  // device view of mapped host memory
+    uint32_t seq = 0;                 // 1 .. kGateCancel - 1
     uint32_t *err = nullptr;       // device memory
     uint64_t limit_ns = kGateLimitNs;
 };
 size_t fold_partials_bytes(size_t n);
 int fold_grid(size_t n, int num_sms);
+int fold_posts(size_t n, int num_sms);
+int round_msg_posts(size_t n, int num_sms);
 int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, uint4 *d_nf,
                         uint4 *d_nb, uint64_t *d_partials, uint64_t *d_msg_out, cudaStream_t st,
                         int num_sms, const MsgPost *post = nullptr,
@@ -195,15 +199,17 @@ int launch_chacha(uint64_t seed, uint64_t first_word, uint4 *d_out, size_t n_wor
 // two half tables (with the previous round's fold by rho first when `fold`;
 // d_w_next, when not null, gets the next round's weights), and the forest's
 // leaf grid.  d_partials holds fold_partials_bytes(0) bytes.  The round posts
-// (sum_end, sum_inf) to the mapped mailbox as the sumcheck rounds do and, when
-// h = 1, first the four entries it leaves to d_tail (mapped, 8 words).  With
-// `gate` (rounds of one CTA, folding) rho comes through the gate.
+// (sum_end, sum_inf) to the mapped mailbox as the sumcheck rounds do.
+// A small round's fold writes d_nl, d_nr (2 h entries each) and not in place,
+// its rho may come through `gate`, and the round of h = 1 posts the four
+// entries it leaves to d_tail (mapped, 12 tagged words).
 int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_t st,
                        int num_sms);
-int gkr_round_grid(size_t h, int num_sms);
-int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fold, uint4 rho,
-                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, cudaStream_t st,
-                     int num_sms, const MsgPost &post, uint64_t *d_tail,
+bool gkr_small_round(size_t h);
+int gkr_round_posts(size_t h, int num_sms);
+int launch_gkr_round(uint4 *d_l, uint4 *d_r, uint4 *d_nl, uint4 *d_nr, const uint4 *d_w, size_t h,
+                     bool fold, uint4 rho, bool send_one, uint4 *d_w_next, uint64_t *d_partials,
+                     cudaStream_t st, int num_sms, const MsgPost &post, uint64_t *d_tail,
                      const RGate *gate = nullptr);
 int launch_gkr_forest_leaves(const uint64_t *d_packed, const uint4 *d_images, int t, int s,
                              uint4 *d_out, cudaStream_t st, int num_sms);

@@ -18,34 +18,39 @@
 
 namespace bz {
 
-__device__ __forceinline__ void warp_xor_wide(gf_wide &a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a.w[i] ^= __shfl_xor_sync(0xffffffffu, a.w[i], o);
-    }
+__device__ __forceinline__ uint64_t warp_xor64(uint64_t v) {
+    const uint32_t lo = __reduce_xor_sync(0xffffffffu, (uint32_t)v);
+    const uint32_t hi = __reduce_xor_sync(0xffffffffu, (uint32_t)(v >> 32));
+    return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
-// Reduce two wide accumulators over the CTA and store 8 words at out.
-__device__ void cta_store_pair(gf_wide u0, gf_wide u2, uint64_t *out) {
+// Word w = lane mod 8 of the XOR of n rows of 8 words (one warp; every lane
+// returns its word).
+template <typename Load>
+__device__ __forceinline__ uint64_t rows_xor(int n, Load row_word) {
+    const int ln = threadIdx.x & 31, w = ln & 7;
+    uint64_t a = 0;
+    for (int i = ln >> 3; i < n; i += 4) a ^= row_word(i, w);
+    a ^= __shfl_xor_sync(0xffffffffu, a, 8);
+    return a ^ __shfl_xor_sync(0xffffffffu, a, 16);
+}
+
+// XOR of two wide accumulators over the CTA: lanes of warp 0 return word
+// (lane mod 8) of {u0, u2}.
+__device__ __forceinline__ uint64_t cta_xor_pair(const gf_wide &u0, const gf_wide &u2) {
     __shared__ uint64_t red[32][8];
-    warp_xor_wide(u0);
-    warp_xor_wide(u2);
     const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
-    if (ln == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            red[w][i] = u0.w[i];
-            red[w][4 + i] = u2.w[i];
+    for (int i = 0; i < 4; ++i) {
+        const uint64_t x = warp_xor64(u0.w[i]), y = warp_xor64(u2.w[i]);
+        if (ln == 0) {
+            red[w][i] = x;
+            red[w][4 + i] = y;
         }
     }
     __syncthreads();
-    if (threadIdx.x < 8) {
-        uint64_t acc = 0;
-        const int nw = blockDim.x >> 5;
-        for (int k = 0; k < nw; ++k) acc ^= red[k][threadIdx.x];
-        out[threadIdx.x] = acc;
-    }
+    if (w != 0) return 0;
+    return rows_xor((int)(blockDim.x >> 5), [&](int i, int k) { return red[i][k]; });
 }
 
 // Dynamic shared memory of the kernels that multiply by one challenge r
@@ -62,97 +67,93 @@ __device__ __forceinline__ const char *build_r_table(uint4 *smem, uint4 r) {
     return reinterpret_cast<const char *>(smem);
 }
 
-// XOR of the per-CTA partials (8 words each) of n CTAs and the single
-// reduction: out = {u0, u2}.  256 threads: thread t XORs word t mod 8 of
-// partials t / 8, t / 8 + 32, ...; lanes holding the same word then combine
-// by shuffles and across warps.  Partials are read from L2 (other CTAs wrote
-// them in this launch or the previous one).
-constexpr int kFinishThreads = 256;
-
-// out = {u0, u2}: the two unreduced sums acc[0..3], acc[4..7], reduced.
-__device__ __forceinline__ void store_msg(const uint64_t *acc, uint64_t *out) {
-    gf_wide w0, w2;
-    for (int i = 0; i < 4; ++i) {
-        w0.w[i] = acc[i];
-        w2.w[i] = acc[4 + i];
-    }
-    const uint4 u0 = gf_reduce(w0), u2 = gf_reduce(w2);
-    out[0] = lo64(u0);
-    out[1] = hi64(u0);
-    out[2] = lo64(u2);
-    out[3] = hi64(u2);
+// {u0, u2} from the eight words of their unreduced sums, word i in lane i of
+// the calling warp: lane 0 returns u0 and lane 1 u2, reduced.
+__device__ __forceinline__ uint4 reduce_pair(uint64_t word) {
+    gf_wide x;
+    const int t = threadIdx.x & 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x.w[i] = __shfl_sync(0xffffffffu, word, 4 * t + i);
+    return gf_reduce(x);
 }
 
-__device__ __forceinline__ void st_release_sys(uint32_t *p, uint32_t v) {
-    asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ void finish_msg_body(const uint64_t *partials, int n, uint64_t *out) {
-    __shared__ uint64_t red[kFinishThreads / 32][8];
-    __shared__ uint64_t acc[8];
-    const int w = threadIdx.x & 7;
-    uint64_t a = 0;
-    for (int i = threadIdx.x >> 3; i < n; i += kFinishThreads / 8)
-        a ^= __ldcg(partials + (uint64_t)i * 8 + w);
-    a ^= __shfl_xor_sync(0xffffffffu, a, 8);
-    a ^= __shfl_xor_sync(0xffffffffu, a, 16);
-    if ((threadIdx.x & 31) < 8) red[threadIdx.x >> 5][w] = a;
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        uint64_t x = 0;
-        for (int k = 0; k < kFinishThreads / 32; ++k) x ^= red[k][threadIdx.x];
-        acc[threadIdx.x] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) store_msg(acc, out);
-}
-
-// The last CTA of a launch (the one whose ticket completes the count)
-// reduces every CTA's partials and posts {u0, u2} to a mailbox in mapped host
-// memory: the four words, then (a system-scope release store by the same
-// thread) the sequence number the host waits for.  It resets the ticket for
-// the next launch.  Without a mailbox (ticket null) the caller launches
-// finish_msg_kernel.
+// Where a message goes: a mailbox in mapped host memory.  A field element is
+// posted as three words of 44 bits, each with the low 20 bits of the message's
+// number above them.  A 64-bit store is one access, so a word whose tag is
+// right holds this message's bits and the host needs no flag that is ordered
+// behind them.  With a system-scope release store of a flag (and the sums
+// reduced by shuffles) the end of a one-CTA round took 1.74 us, now 0.45.
+// Without a mailbox (ticket null) the caller launches finish_msg_kernel.
 struct MsgMailbox {
     unsigned int *ticket = nullptr;  // device counter, 0 between launches
     uint64_t *words = nullptr;       // mapped host memory: u0, u2
-    uint32_t *seq = nullptr;         // mapped host memory
     uint32_t seq_val = 0;
 };
 
-__device__ void msg_epilogue(const uint64_t *partials, const MsgMailbox &mb) {
+__device__ __forceinline__ void post_element(uint64_t *words, uint32_t seq, uint4 v) {
+    const uint64_t lo = lo64(v), hi = hi64(v), tag = (uint64_t)seq << 44;
+    const uint64_t m = ((uint64_t)1 << 44) - 1;
+    volatile uint64_t *o = words;
+    o[0] = (lo & m) | tag;
+    o[1] = (((lo >> 44) | (hi << 20)) & m) | tag;
+    o[2] = (hi >> 24) | tag;
+}
+
+// Lanes 0 and 1 of the calling warp post u0 and u2.
+__device__ __forceinline__ void post_pair(uint64_t word, const MsgMailbox &mb) {
+    const uint4 v = reduce_pair(word);
+    const int ln = threadIdx.x & 31;
+    if (ln < 2) post_element(mb.words + 3 * ln, mb.seq_val, v);
+}
+
+// XOR of the partials (8 words each) of n CTAs, by all threads; lanes of warp
+// 0 return word (lane mod 8).  Partials are read from L2 (other CTAs wrote
+// them in this launch or the previous one).
+constexpr int kFinishThreads = 256;
+__device__ uint64_t partials_xor(const uint64_t *partials, int n) {
+    __shared__ uint64_t red[32][8];
+    const int nw = blockDim.x >> 5, wp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+    const int rows = n > wp * 4 ? (n - wp * 4 + 4 * nw - 1) / (4 * nw) * 4 : 0;
+    const uint64_t a = rows_xor(rows, [&](int i, int k) {
+        const int row = (i >> 2) * 4 * nw + wp * 4 + (i & 3);
+        return row < n ? __ldcg(partials + (uint64_t)row * 8 + k) : 0;
+    });
+    if (ln < 8) red[wp][ln] = a;
+    __syncthreads();
+    if (wp != 0) return 0;
+    return rows_xor(nw, [&](int i, int k) { return red[i][k]; });
+}
+
+// The CTA's sums (word (lane mod 8) in the lanes of warp 0).  With a mailbox
+// and up to kMsgPosts CTAs, each posts its own and the host adds them (0.2 us;
+// the ticket takes 0.9 to 2.1).  Otherwise every CTA stores its partial, and
+// with a mailbox the last one (whose ticket completes the count) reduces them
+// all, posts and resets the ticket for the next launch.
+__device__ __forceinline__ void msg_out(uint64_t word, uint64_t *partials, MsgMailbox mb) {
+    if (mb.ticket && msg_posts(gridDim.x) == (int)gridDim.x) {
+        mb.words += 6 * blockIdx.x;
+        if (threadIdx.x < 32) post_pair(word, mb);
+        return;
+    }
+    if (threadIdx.x < 8) partials[(uint64_t)blockIdx.x * 8 + threadIdx.x] = word;
     if (!mb.ticket) return;
     __shared__ int last;
-    __threadfence();  // this CTA's partial (written before the barrier below)
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(mb.ticket, 1u) == gridDim.x - 1;
+    if (threadIdx.x < 32) {
+        __threadfence();  // this CTA's partial, by the lanes that wrote it
+        __syncwarp();
+        if (threadIdx.x == 0) last = atomicAdd(mb.ticket, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    finish_msg_body(partials, (int)gridDim.x, mb.words);
-    if (threadIdx.x == 0) {
-        st_release_sys(mb.seq, mb.seq_val);
-        *mb.ticket = 0;
-    }
+    const uint64_t sum = partials_xor(partials, (int)gridDim.x);
+    if (threadIdx.x < 32) post_pair(sum, mb);
+    if (threadIdx.x == 0) *mb.ticket = 0;
 }
 
-// A single-CTA launch with a mailbox reduces its terms in shared memory and
-// posts them itself (no partials, no ticket); otherwise every CTA stores its
-// partial and the last one posts.
-__device__ __forceinline__ void msg_finish(gf_wide u0, gf_wide u2, uint64_t *partials,
-                                           const MsgMailbox &mb) {
-    if (mb.ticket && gridDim.x == 1) {
-        __shared__ uint64_t acc[8];
-        cta_store_pair(u0, u2, acc);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            store_msg(acc, mb.words);
-            st_release_sys(mb.seq, mb.seq_val);
-        }
-        return;
-    }
-    cta_store_pair(u0, u2, partials + (uint64_t)blockIdx.x * 8);
-    msg_epilogue(partials, mb);
+__device__ __forceinline__ void msg_finish(const gf_wide &u0, const gf_wide &u2,
+                                           uint64_t *partials, const MsgMailbox &mb) {
+    msg_out(cta_xor_pair(u0, u2), partials, mb);
 }
 
 // Out of line for the fold kernel: its loop runs at the 128-register cap, and
@@ -162,9 +163,9 @@ __device__ __noinline__ void msg_finish_call(gf_wide u0, gf_wide u2, uint64_t *p
     msg_finish(u0, u2, partials, mb);
 }
 
-__device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ uint64_t ld_relaxed_sys(const uint64_t *p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -174,36 +175,42 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
-// Thread 0 of each CTA polls the gate word, sleeping between polls, until it
-// reads the round's sequence number (open: r is read behind it), the number
-// with bit 31 set (cancelled) or the time limit passes (bit 0 of *err is
-// set).  Returns whether the gate opened; r is then the posted challenge.
+// Warp 0 of each CTA polls the gate's three words, sleeping between polls,
+// until all carry the round's number (open: together they hold r, as
+// post_element lays it out, so one access brings both), the first carries the
+// number with its top bit set (cancelled) or the time limit passes (bit 0 of
+// *err is set).  Returns whether the gate opened; r is then the posted
+// challenge.
 __device__ bool gate_wait(const RGate &g, uint4 &r) {
     __shared__ uint4 rs;
     __shared__ int open;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         const uint64_t t0 = globaltimer_ns();
+        const int ln = threadIdx.x;
         int st = 0;
+        uint64_t v = 0;
         for (;;) {
-            const uint32_t v = ld_acquire_sys(g.go);
-            if (v == g.seq) {
+            if (ln < 3) v = ld_relaxed_sys(g.words + ln);
+            const uint32_t tag = (uint32_t)(v >> 44);
+            if (__all_sync(0xffffffffu, ln >= 3 || tag == g.seq)) {
                 st = 1;
                 break;
             }
-            if (v == (g.seq | kGateCancel)) break;
-            if (globaltimer_ns() - t0 > g.limit_ns) {
-                atomicOr(g.err, 1u);
+            if (__any_sync(0xffffffffu, ln == 0 && tag == (g.seq | kGateCancel))) break;
+            if (__any_sync(0xffffffffu, ln == 0 && globaltimer_ns() - t0 > g.limit_ns)) {
+                if (ln == 0) atomicOr(g.err, 1u);
                 break;
             }
             __nanosleep(128);
         }
-        if (st) {
-            const volatile uint64_t *rp = g.r;
-            const uint64_t lo = rp[0], hi = rp[1];
-            rs = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi,
-                            (uint32_t)(hi >> 32));
+        const uint64_t m = ((uint64_t)1 << 44) - 1;
+        const uint64_t v0 = __shfl_sync(0xffffffffu, v, 0) & m;
+        const uint64_t v1 = __shfl_sync(0xffffffffu, v, 1) & m;
+        const uint64_t v2 = __shfl_sync(0xffffffffu, v, 2) & m;
+        if (ln == 0) {
+            rs = mk(v0 | (v1 << 44), (v1 >> 20) | (v2 << 24));
+            open = st;
         }
-        open = st;
     }
     __syncthreads();
     r = rs;
@@ -250,10 +257,6 @@ __global__ void __launch_bounds__(256, 2) fold_and_msg_kernel(const uint4 *f, co
         gf_wide_xor(u0, gf_mul_wide(x0, y0));
         gf_wide_xor(u2, gf_mul_wide(gf_add(x0, x1), gf_add(y0, y1)));
     }
-    if (half == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-        nf[0] = gf_add(f[0], gf_mul(gf_add(f[0], f[1]), r));
-        nb[0] = gf_add(b[0], gf_mul(gf_add(b[0], b[1]), r));
-    }
     msg_finish_call(u0, u2, partials, mb);
 }
 
@@ -275,7 +278,229 @@ __global__ void __launch_bounds__(256) round_msg_kernel(const uint4 *f, const ui
 __global__ void __launch_bounds__(kFinishThreads) finish_msg_kernel(const uint64_t *partials,
                                                                     int n, uint64_t *out) {
     chain_wait();
-    finish_msg_body(partials, n, out);
+    const uint64_t sum = partials_xor(partials, n);
+    if (threadIdx.x >= 32) return;
+    const uint4 v = reduce_pair(sum);
+    if (threadIdx.x < 2) {
+        out[2 * threadIdx.x] = lo64(v);
+        out[2 * threadIdx.x + 1] = hi64(v);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small rounds.  A round over few slots is the latency of its own chain: the
+// byte tables of the challenge (0.84 us to build), one lookup product and up
+// to three variable products a thread, each of 144 wide multiply-adds one
+// after the other (0.6 us).  Here a CTA has nine warps and warp q computes the
+// q-th 32x32 product of the Karatsuba tree for 32 products at a time, through
+// shared memory: no tables, and a product takes 0.35 to 0.5 us of latency.  The
+// message sums need no recombination per product: each warp sums its own part
+// and the parts of the total are combined once.  A sumcheck round of one CTA
+// takes 1.7 us on the device instead of 4.7, a GKR round 1.6 us behind its
+// challenge instead of 6.7.
+// ---------------------------------------------------------------------------
+constexpr int kCoopThreads = 288;
+constexpr int kCoopSlots = 64;  // slots a CTA takes at a time at most (4 elements each)
+
+// Part q = 3 u + v of the operand: u picks the low or high 64-bit half or
+// their sum, v the same of its 32-bit halves.
+struct CoopPart {
+    uint32_t m[4];
+    __device__ __forceinline__ explicit CoopPart(int q) {
+        const int u = q / 3, v = q - 3 * u;
+        const uint32_t lo = u == 1 ? 0u : ~0u, hi = u == 0 ? 0u : ~0u;
+        const uint32_t even = v == 1 ? 0u : ~0u, odd = v == 0 ? 0u : ~0u;
+        m[0] = lo & even;
+        m[1] = lo & odd;
+        m[2] = hi & even;
+        m[3] = hi & odd;
+    }
+    __device__ __forceinline__ uint32_t of(uint4 a) const {
+        return (a.x & m[0]) ^ (a.y & m[1]) ^ (a.z & m[2]) ^ (a.w & m[3]);
+    }
+};
+
+// The unreduced product from its nine parts.
+template <typename Part>
+__device__ __forceinline__ gf_wide coop_combine(Part part) {
+    uint64_t lo[3], hi[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+        const uint64_t l = part(3 * u), h = part(3 * u + 1), m = part(3 * u + 2) ^ l ^ h;
+        lo[u] = l ^ (m << 32);
+        hi[u] = h ^ (m >> 32);
+    }
+    const uint64_t m0 = lo[2] ^ lo[0] ^ lo[1], m1 = hi[2] ^ hi[0] ^ hi[1];
+    gf_wide r;
+    r.w[0] = lo[0];
+    r.w[1] = hi[0] ^ m0;
+    r.w[2] = lo[1] ^ m1;
+    r.w[3] = hi[1];
+    return r;
+}
+
+// f(p, p < n) for p = lane, lane + 32, .. up to n - 1: U at a time where there
+// is more than one, so that their latencies overlap (p stays below the next
+// multiple of 32 U).
+template <int U, typename F>
+__device__ __forceinline__ void coop_each(int n, F f) {
+    const int ln = threadIdx.x & 31;
+    if (n <= 32) {
+        f(ln, ln < n);
+        return;
+    }
+    for (int p = ln; p - ln < n; p += 32 * U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) f(p + 32 * u, p + 32 * u < n);
+    }
+}
+
+// A round over h slots.  GKR: the tables a, b hold entry i of slot c at c +
+// i h and a fold joins the entries at i h and (i + 2) h; the sums are weighted
+// by w.  Otherwise (the sumcheck): entry i of slot c is at 2 c + i and a fold
+// joins 2 j and 2 j + 1.  Folded tables go to na, nb, which are not the inputs
+// (a gate that runs out in some CTAs leaves the round to be run again).
+struct CoopRound {
+    const uint4 *a, *b;
+    uint4 *na, *nb;
+    const uint4 *w;
+    uint4 *w_next;
+    uint64_t *tail;  // mapped: the round's four entries, 3 tagged words each
+    uint64_t h;
+    int per;  // slots a CTA takes at a time
+    uint4 r;
+    int send_one;
+    int single;  // a sumcheck fold to one element: no message
+    uint64_t *partials;
+    MsgMailbox mb;
+};
+
+template <bool GKR, bool FOLD, bool GATED>
+__global__ void __launch_bounds__(kCoopThreads) coop_round_kernel(
+    const __grid_constant__ CoopRound a, const __grid_constant__ RGate gate) {
+    __shared__ uint4 mul[4 * kCoopSlots];  // multiplicands: differences, then weighted entries
+    __shared__ uint4 ent[4 * kCoopSlots];  // entry 4 slot + 2 table + i
+    __shared__ uint4 wgt[kCoopSlots];
+    __shared__ uint64_t prod[9][4 * kCoopSlots];
+    __shared__ uint64_t sums[9][2];
+    const int tid = threadIdx.x, q = tid >> 5, ln = tid & 31;
+    const CoopPart part(q);
+    const uint64_t h = a.h;
+    uint4 r = a.r;
+    uint32_t rp = 0;
+    uint64_t acc = 0;  // even lanes: the first sum's part, odd lanes: the second's
+    chain_wait();
+    for (uint64_t c0 = (uint64_t)blockIdx.x * a.per; c0 < h;
+         c0 += (uint64_t)gridDim.x * a.per) {
+        const int ns = (int)(h - c0 < a.per ? h - c0 : a.per);
+        // thread 4 slot + 2 table + i loads its entry (GATED: before the challenge)
+        uint64_t dst = 0;
+        const int i = tid & 1;
+        const bool mine = tid < 4 * ns && !(a.single && i);
+        uint4 base = make_uint4(0, 0, 0, 0), diff = base;
+        if (mine) {
+            const uint64_t c = c0 + (tid >> 2);
+            const uint4 *t = (tid & 2) ? a.b : a.a;
+            dst = GKR ? c + i * h : 2 * c + i;
+            if constexpr (FOLD) {
+                base = t[GKR ? dst : 2 * dst];
+                diff = gf_add(base, t[GKR ? dst + 2 * h : 2 * dst + 1]);
+            } else {
+                base = t[dst];
+            }
+        }
+        // the last threads: a slot's weight, and the next round's
+        const int sw = tid - (kCoopThreads - kCoopSlots);
+        const uint64_t cw = c0 + sw;
+        const bool weigh = GKR && sw >= 0 && sw < ns;
+        const bool weigh_next = weigh && a.w_next && cw < h / 2;
+        uint4 wn = base;
+        if (weigh) {
+            const uint4 wc = a.w[cw];
+            wgt[sw] = wc;
+            if (weigh_next) wn = gf_add(wc, a.w[cw + h / 2]);
+        }
+        if constexpr (FOLD) {
+            if (tid < 4 * ns) mul[tid] = diff;
+            if (GATED && c0 == (uint64_t)blockIdx.x * a.per) {
+                if (!gate_wait(gate, r)) return;
+            }
+            __syncthreads();
+            rp = part.of(r);
+            coop_each<4>(4 * ns, [&](int p, bool) { prod[q][p] = clmul32(part.of(mul[p]), rp); });
+            __syncthreads();
+            if (mine) {
+                base = gf_add(base, gf_reduce(coop_combine([&](int k) { return prod[k][tid]; })));
+                ((tid & 2) ? a.nb : a.na)[dst] = base;
+            }
+        }
+        // written after the gate, as all of global memory: the round behind one
+        // whose gate ran out must leave that round's inputs as they are
+        if (weigh_next) a.w_next[cw] = wn;
+        if (tid < 4 * ns) ent[tid] = base;
+        __syncthreads();
+        // products 2 slot + t of the message: t = 0 the end value, 1 the difference
+        auto operand = [&](int p, int table) {
+            const uint4 *e = ent + 4 * (p >> 1) + 2 * table;
+            if (p & 1) return gf_add(e[0], e[1]);
+            return e[GKR && a.send_one];
+        };
+        if constexpr (GKR) {
+            if (a.tail && tid < 4) post_element(a.tail + 3 * tid, a.mb.seq_val, base);
+            coop_each<2>(2 * ns, [&](int p, bool) {
+                prod[q][p] = clmul32(part.of(operand(p, 0)), part.of(wgt[p >> 1]));
+            });
+            __syncthreads();
+            if (tid < 2 * ns)
+                mul[tid] = gf_reduce(coop_combine([&](int k) { return prod[k][tid]; }));
+            __syncthreads();
+        }
+        if (!a.single)
+            coop_each<2>(2 * ns, [&](int p, bool in) {
+                const uint64_t v =
+                    clmul32(part.of(GKR ? mul[p] : operand(p, 0)), part.of(operand(p, 1)));
+                acc ^= in ? v : 0;
+            });
+        __syncthreads();
+    }
+    const uint64_t s0 = warp_xor64((ln & 1) ? 0 : acc), s1 = warp_xor64((ln & 1) ? acc : 0);
+    if (ln == 0) {
+        sums[q][0] = s0;
+        sums[q][1] = s1;
+    }
+    __syncthreads();
+    // word (lane mod 8) of {sum 0, sum 1} in warp 0
+    uint64_t word = 0;
+    if (tid < 8) {
+        const gf_wide x = coop_combine([&](int k) { return sums[k][tid >> 2]; });
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if ((tid & 3) == k) word = x.w[k];
+    }
+    msg_out(word, a.partials, a.mb);
+}
+
+// Up to kMsgPosts CTAs while they take at most kCoopSlots each (the host adds
+// their sums), at least 8 slots (one step of the fold's products) each; above,
+// the ticket is paid for and half the slots a CTA halve its steps.
+static int coop_per(uint64_t slots) {
+    if (slots <= kMsgPosts * kCoopSlots)
+        return (int)std::max<uint64_t>(8, (slots + kMsgPosts - 1) / kMsgPosts);
+    return slots <= 4096 ? kCoopSlots / 2 : kCoopSlots;
+}
+
+// CTAs of a small round over `slots` slots, 0 above `limit`, where the table
+// kernels (or a thread a product) are as fast or faster.  Through the public
+// calls: a fold to 2^13 pairs 18.6 us (tables 19.8) and to 2^14 20.8 (20.2); a
+// message alone over 2^12 pairs 14.9 (15.0) and over 2^14 16.4 (15.3); GKR
+// rounds may be armed below the limit, 2^22 leaves take 2.70 ms at 2^13, 2.65 at
+// 2^14 and 2.68 at 2^15.
+constexpr uint64_t kCoopFoldSlots = 1 << 13, kCoopMsgSlots = 1 << 12, kCoopGkrSlots = 1 << 14;
+static int coop_grid(uint64_t slots, uint64_t limit, int num_sms) {
+    if (slots > limit) return 0;
+    const int per = coop_per(slots);
+    return (int)std::max<uint64_t>(
+        1, std::min<uint64_t>((slots + per - 1) / per, 2 * (uint64_t)num_sms));
 }
 
 static int msg_grid(uint64_t work, int num_sms) {
@@ -288,7 +513,17 @@ size_t fold_partials_bytes(size_t n) {
     return (size_t)1024 * 8 * sizeof(uint64_t);  // up to 1024 CTAs
 }
 
-int fold_grid(size_t n, int num_sms) { return std::min(msg_grid(n / 4, num_sms), 1024); }
+// CTAs of a message kernel over `slots` slots.
+static int round_grid(uint64_t slots, uint64_t limit, int num_sms) {
+    const int cg = coop_grid(slots, limit, num_sms);
+    return cg ? cg : std::min(msg_grid(slots, num_sms), 1024);
+}
+
+int fold_grid(size_t n, int num_sms) { return round_grid(n / 4, kCoopFoldSlots, num_sms); }
+int fold_posts(size_t n, int num_sms) { return msg_posts(fold_grid(n, num_sms)); }
+int round_msg_posts(size_t n, int num_sms) {
+    return msg_posts(round_grid(n / 2, kCoopMsgSlots, num_sms));
+}
 
 int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, uint4 *d_nf,
                         uint4 *d_nb, uint64_t *d_partials, uint64_t *d_msg_out, cudaStream_t st,
@@ -296,13 +531,23 @@ int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, u
     const uint64_t half = n / 2;
     const int grid = fold_grid(n, num_sms);
     MsgMailbox mb;
-    if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
-    if (gate)
+    if (post) mb = {post->ticket, post->words, post->seq_val};
+    if (n / 4 <= kCoopFoldSlots) {
+        const CoopRound a = {d_f, d_b, d_nf, d_nb, nullptr, nullptr, nullptr,
+                             std::max<uint64_t>(n / 4, 1), coop_per(n / 4), r, 0, n == 2, d_partials, mb};
+        if (gate)
+            launch_chained(coop_round_kernel<false, true, true>, grid, kCoopThreads, 0, st, a,
+                           *gate);
+        else
+            launch_chained(coop_round_kernel<false, true, false>, grid, kCoopThreads, 0, st, a,
+                           RGate{});
+    } else if (gate) {
         launch_chained(fold_and_msg_kernel<true>, grid, 256, kRTableSmem, st, d_f, d_b, half, r,
                        d_nf, d_nb, d_partials, mb, *gate);
-    else
+    } else {
         launch_chained(fold_and_msg_kernel<false>, grid, 256, kRTableSmem, st, d_f, d_b, half, r,
                        d_nf, d_nb, d_partials, mb, RGate{});
+    }
     if (post) return 1;
     launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
@@ -311,10 +556,17 @@ int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, u
 int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_partials,
                      uint64_t *d_msg_out, cudaStream_t st, int num_sms, const MsgPost *post) {
     const uint64_t pairs = n / 2;
-    const int grid = std::min(msg_grid(pairs, num_sms), 1024);
+    const int grid = round_grid(pairs, kCoopMsgSlots, num_sms);
     MsgMailbox mb;
-    if (post) mb = {post->ticket, post->words, post->seq, post->seq_val};
-    launch_chained(round_msg_kernel, grid, 256, 0, st, d_f, d_b, pairs, d_partials, mb);
+    if (post) mb = {post->ticket, post->words, post->seq_val};
+    if (pairs <= kCoopMsgSlots) {
+        const CoopRound a = {d_f, d_b, nullptr, nullptr, nullptr, nullptr, nullptr, pairs,
+                             coop_per(pairs), make_uint4(0, 0, 0, 0), 0, 0, d_partials, mb};
+        launch_chained(coop_round_kernel<false, false, false>, grid, kCoopThreads, 0, st, a,
+                       RGate{});
+    } else {
+        launch_chained(round_msg_kernel, grid, 256, 0, st, d_f, d_b, pairs, d_partials, mb);
+    }
     if (post) return 1;
     launch_chained(finish_msg_kernel, 1, kFinishThreads, 0, st, d_partials, grid, d_msg_out);
     return 2;
@@ -757,23 +1009,13 @@ __global__ void __launch_bounds__(256) gkr_product_kernel(const uint4 *in, uint6
 // finish kernel reduces them.  With w_next, the next round's weights
 // w_next[c] = w[c] + w[c + h/2] (eq over one coordinate fewer: the two
 // values of the dropped coordinate's factor sum to 1) are written too.
-//
-// A round of one slot also posts the four entries it leaves (l[0], l[1], r[0],
-// r[1]) to `tail`, ahead of its sums, so the layer's close needs no copy.
-// GATED: launched before rho is known, as the sumcheck's armed folds; for
-// launches of one CTA, because the fold is in place and a gate that runs out
-// must leave the whole round undone.
-template <bool FOLD, bool GATED>
+template <bool FOLD>
 __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, const uint4 *w,
                                                            uint64_t h, uint4 rho, int send_one,
                                                            uint64_t *partials, MsgMailbox mb,
-                                                           uint4 *w_next, uint64_t *tail,
-                                                           RGate gate) {
+                                                           uint4 *w_next) {
     chain_wait();
     extern __shared__ uint4 smem[];
-    if constexpr (GATED) {
-        if (!gate_wait(gate, rho)) return;
-    }
     const char *T = nullptr;
     T16Lane8 lc;
     if constexpr (FOLD) {
@@ -806,14 +1048,6 @@ __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, c
         const uint4 le = send_one ? l1 : l0, re = send_one ? r1 : r0;
         gf_wide_xor(e, gf_mul_wide(gf_mul(wc, le), re));
         gf_wide_xor(f, gf_mul_wide(gf_mul(wc, gf_add(l1, l0)), gf_add(r1, r0)));
-        if (tail && h == 1) {
-            const uint4 v[4] = {l0, l1, r0, r1};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                tail[2 * i] = lo64(v[i]);
-                tail[2 * i + 1] = hi64(v[i]);
-            }
-        }
     }
     msg_finish_call(e, f, partials, mb);
 }
@@ -842,29 +1076,42 @@ int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_
     return 1;
 }
 
-int gkr_round_grid(size_t h, int num_sms) { return std::min(msg_grid(h, num_sms), 1024); }
+bool gkr_small_round(size_t h) { return h <= kCoopGkrSlots; }
 
-int launch_gkr_round(uint4 *d_l, uint4 *d_r, const uint4 *d_w, size_t h, bool fold, uint4 rho,
-                     bool send_one, uint4 *d_w_next, uint64_t *d_partials, cudaStream_t st,
-                     int num_sms, const MsgPost &post, uint64_t *d_tail, const RGate *gate) {
+static int gkr_round_grid(size_t h, int num_sms) { return round_grid(h, kCoopGkrSlots, num_sms); }
+
+int gkr_round_posts(size_t h, int num_sms) { return msg_posts(gkr_round_grid(h, num_sms)); }
+
+int launch_gkr_round(uint4 *d_l, uint4 *d_r, uint4 *d_nl, uint4 *d_nr, const uint4 *d_w, size_t h,
+                     bool fold, uint4 rho, bool send_one, uint4 *d_w_next, uint64_t *d_partials,
+                     cudaStream_t st, int num_sms, const MsgPost &post, uint64_t *d_tail,
+                     const RGate *gate) {
+    const MsgMailbox mb = {post.ticket, post.words, post.seq_val};
     const int grid = gkr_round_grid(h, num_sms);
-    const MsgMailbox mb = {post.ticket, post.words, post.seq, post.seq_val};
-    if (gate)
-        launch_chained(gkr_round_kernel<true, true>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h,
-                       rho, send_one, d_partials, mb, d_w_next, d_tail, *gate);
-    else if (fold)
-        launch_chained(gkr_round_kernel<true, false>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h,
-                       rho, send_one, d_partials, mb, d_w_next, d_tail, RGate{});
+    if (gkr_small_round(h)) {
+        const CoopRound a = {d_l, d_r, d_nl, d_nr, d_w, d_w_next, h == 1 ? d_tail : nullptr, h,
+                             coop_per(h), rho, send_one, 0, d_partials, mb};
+        if (gate)
+            launch_chained(coop_round_kernel<true, true, true>, grid, kCoopThreads, 0, st, a, *gate);
+        else if (fold)
+            launch_chained(coop_round_kernel<true, true, false>, grid, kCoopThreads, 0, st, a,
+                           RGate{});
+        else
+            launch_chained(coop_round_kernel<true, false, false>, grid, kCoopThreads, 0, st, a,
+                           RGate{});
+        return 1;
+    }
+    if (fold)
+        launch_chained(gkr_round_kernel<true>, grid, 256, kRTableSmem, st, d_l, d_r, d_w, h, rho,
+                       send_one, d_partials, mb, d_w_next);
     else
-        launch_chained(gkr_round_kernel<false, false>, grid, 256, 0, st, d_l, d_r, d_w, h, rho,
-                       send_one, d_partials, mb, d_w_next, d_tail, RGate{});
+        launch_chained(gkr_round_kernel<false>, grid, 256, 0, st, d_l, d_r, d_w, h, rho, send_one,
+                       d_partials, mb, d_w_next);
     return 1;
 }
 
 void init_gkr_kernels() {
-    cudaFuncSetAttribute(gkr_round_kernel<true, false>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRTableSmem);
-    cudaFuncSetAttribute(gkr_round_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(gkr_round_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kRTableSmem);
 }
 

@@ -105,12 +105,16 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
     if (!rc) rc = dev_alloc(ctx, std::max<size_t>(n / 4, 1) * 16, &eqa.p, false);
     if (!rc) rc = dev_alloc(ctx, std::max<size_t>(n / 4, 1) * 16, &eqb.p, false);
     const size_t part_bytes = fold_partials_bytes(0);
-    if (!rc) rc = dev_alloc(ctx, part_bytes, &scratch.p, false);
+    // two tables of 2 h entries for the folds of the small rounds, which are
+    // not in place
+    size_t coop = 1;
+    while (2 * coop < n && gkr_small_round(2 * coop)) coop *= 2;
+    if (!rc) rc = dev_alloc(ctx, part_bytes + 4 * coop * 16, &scratch.p, false);
     if (rc) return rc;
     uint64_t *d_partials = (uint64_t *)scratch.p;
     // the last round's four entries, at byte 512 of the mapped mailbox
-    uint64_t *d_tail = (uint64_t *)((uint8_t *)ctx->d_mbox + 512);
-    const volatile uint64_t *h_tail = (const volatile uint64_t *)((uint8_t *)ctx->h_mbox + 512);
+    constexpr size_t kTailOffset = 512;
+    uint64_t *d_tail = (uint64_t *)((uint8_t *)ctx->d_mbox + kTailOffset);
     Armed armed{ctx};
     std::vector<uint4 *> layer(layers + 1);
     layer[0] = d_leaves;
@@ -134,6 +138,8 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
     for (int j = layers - 1; j >= 0; --j) {
         const int k = L - j - 1;  // coordinates of this layer's point
         uint4 *l = layer[j], *r = layer[j] + ((size_t)1 << k);
+        uint4 *nl = (uint4 *)((uint8_t *)scratch.p + part_bytes), *nr = nl + 2 * coop;
+        uint32_t tail_seq = 0;
         Gf factor = gone(), rho;
         std::vector<Gf> next;
         bool pending = false;
@@ -151,10 +157,19 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
             auto launch = [&](int rnd, const MsgPost &post, const RGate *gate) -> int {
                 const int remaining = k - 1 - rnd;
                 ctx->launches += launch_gkr_round(
-                    l, r, w, (size_t)1 << remaining, rnd > 0, to_u4(rho), gzero(p[rnd]),
+                    l, r, nl, nr, w, (size_t)1 << remaining, rnd > 0, to_u4(rho), gzero(p[rnd]),
                     remaining ? w_next : nullptr, d_partials, st, ctx->num_sms, post, d_tail, gate);
                 BZ_CUDA(ctx, cudaGetLastError());
                 return BZ_OK;
+            };
+            auto small = [&](int rnd) { return gkr_small_round((size_t)1 << (k - 1 - rnd)); };
+            // exchange the tables that round rnd reads and those it writes
+            auto flip = [&](int rnd) {
+                std::swap(w, w_next);
+                if (rnd > 0 && small(rnd)) {
+                    std::swap(l, nl);
+                    std::swap(r, nr);
+                }
             };
             for (int rnd = 0; rnd < k; ++rnd) {
                 const Gf &z = p[rnd];
@@ -168,12 +183,11 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                     post = next_msg_post(ctx);
                     if ((rc = launch(rnd, post, nullptr))) return rc;
                 }
-                std::swap(w, w_next);
-                // The next round of one CTA is enqueued behind this one, and
-                // waits on the device for the challenge: its launch overlaps
-                // the wait, the sums' host work and the transcript.
-                if (rnd + 1 < k && ctx->arm_gkr &&
-                    gkr_round_grid((size_t)1 << (k - 2 - rnd), ctx->num_sms) == 1) {
+                flip(rnd);
+                // The next round, if a small one, is enqueued behind this one
+                // and waits on the device for the challenge: its launch
+                // overlaps the wait, the sums' host work and the transcript.
+                if (rnd + 1 < k && ctx->arm_gkr && small(rnd + 1)) {
                     const RGate g = next_gate(ctx, kGkrGateLimitNs);
                     armed.post = next_msg_post(ctx);
                     if ((rc = launch(rnd + 1, armed.post, &g))) return rc;
@@ -181,7 +195,8 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                     armed.fold.live = true;
                 }
                 Gf se, si;
-                rc = msg_wait(ctx, post.seq_val, se.w, si.w);
+                const int posts = gkr_round_posts((size_t)1 << (k - 1 - rnd), ctx->num_sms);
+                rc = msg_wait(ctx, post.seq_val, posts, se.w, si.w);
                 if (rc && was_armed) {
                     // the gate ran out before the challenge came (a transcript
                     // that took long or used the context's stream): the round
@@ -192,11 +207,12 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                     ctx->arm_folds = arm_folds;
                     if (gave_up) {
                         ctx->arm_gkr = false;
-                        std::swap(w, w_next);
+                        reset_msg_ticket(ctx);
+                        flip(rnd);
                         post = next_msg_post(ctx);
                         if ((rc = launch(rnd, post, nullptr))) return rc;
-                        std::swap(w, w_next);
-                        rc = msg_wait(ctx, post.seq_val, se.w, si.w);
+                        flip(rnd);
+                        rc = msg_wait(ctx, post.seq_val, posts, se.w, si.w);
                     }
                 }
                 if (rc) {
@@ -204,6 +220,7 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
                     reset_msg_ticket(ctx);
                     return rc;
                 }
+                tail_seq = post.seq_val;
                 se = gmul(factor, se);
                 si = gmul(factor, si);
                 const uint64_t msg[4] = {se.w[0], se.w[1], si.w[0], si.w[1]};
@@ -221,7 +238,7 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
         // layer without rounds) one
         uint64_t lr[8] = {0};
         if (pending) {
-            for (int i = 0; i < 8; ++i) lr[i] = h_tail[i];
+            if ((rc = elements_wait(ctx, kTailOffset, 4, tail_seq, "layer close", lr))) return rc;
         } else {
             BZ_CUDA(ctx, cudaMemcpyAsync(lr, l, 16, cudaMemcpyDeviceToHost, st));
             BZ_CUDA(ctx, cudaMemcpyAsync(lr + 4, r, 16, cudaMemcpyDeviceToHost, st));

@@ -161,7 +161,8 @@ struct Sumcheck {
             rc = bz::fold_arm(ctx, f, b, len, (uint64_t *)nd, (uint64_t *)(nd + len / 2), &armed);
         }
         uint64_t u0[2], u2[2];
-        int wrc = bz::msg_wait(ctx, seq, u0, u2);
+        const int posts = bz::fold_posts(in_len, ctx->num_sms);
+        int wrc = bz::msg_wait(ctx, seq, posts, u0, u2);
         if (wrc && was_armed && !rc) {
             // the gate ran out before r arrived (a host stall, or a tool that
             // completes each launch before returning): run the round unarmed
@@ -169,7 +170,7 @@ struct Sumcheck {
             if (bz::gate_gave_up(ctx)) {
                 bz::reset_msg_ticket(ctx);
                 wrc = bz::fold_launch(ctx, in_f, in_b, in_len, r_out, nf, nb, &seq);
-                if (!wrc) wrc = bz::msg_wait(ctx, seq, u0, u2);
+                if (!wrc) wrc = bz::msg_wait(ctx, seq, posts, u0, u2);
             }
         }
         if (rc || wrc) {

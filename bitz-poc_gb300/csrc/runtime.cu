@@ -873,12 +873,14 @@ static bool pow2(size_t n) { return n && !(n & (n - 1)); }
 
 namespace bz {
 
+// The messages' posts in the mapped mailbox (kMsgPosts of 48 bytes).
+constexpr size_t kMsgOffset = 3072;
+
 // Mailbox post for the next message kernel on the context stream.
 static MsgPost next_post(bz_ctx *ctx) {
     MsgPost p;
     p.ticket = (unsigned int *)((uint8_t *)ctx->d_small + 768);
-    p.words = (uint64_t *)ctx->d_mbox;
-    p.seq = (uint32_t *)((uint8_t *)ctx->d_mbox + 64);
+    p.words = (uint64_t *)((uint8_t *)ctx->d_mbox + kMsgOffset);
     if (++ctx->mbox_seq == 0) ++ctx->mbox_seq;  // 0 is the initial mailbox value
     p.seq_val = ctx->mbox_seq;
     return p;
@@ -890,18 +892,17 @@ void reset_msg_ticket(bz_ctx *ctx) {
     cudaMemsetAsync((uint8_t *)ctx->d_small + 768, 0, 4, ctx->stream);
 }
 
-// Wait for the message kernel to post sequence number seq, then read
-// {u0, u2}.  The wait spins on the mailbox (no stream synchronisation on the
+// Spin on the mapped mailbox until ready() (no stream synchronisation on the
 // critical path), checking the stream every few hundred spins so that a
-// failed launch returns its error, and gives up after 60 s.
-int mapped_wait(bz_ctx *ctx, size_t offset, uint32_t seq, const char *what) {
-    volatile uint32_t *sp = (volatile uint32_t *)((uint8_t *)ctx->h_mbox + offset);
+// failed launch returns its error, and giving up after 60 s.
+template <typename Ready>
+static int spin_wait(bz_ctx *ctx, const char *what, Ready ready) {
     const auto t0 = std::chrono::steady_clock::now();
-    for (uint64_t spin = 1; *sp != seq; ++spin) {
+    for (uint64_t spin = 1; !ready(); ++spin) {
         if ((spin & 255) == 0) {
             const cudaError_t e = cudaStreamQuery(ctx->stream);
             if (e != cudaSuccess && e != cudaErrorNotReady) return set_err(ctx, BZ_ERR_CUDA, what, e);
-            if (e == cudaSuccess && *sp != seq)
+            if (e == cudaSuccess && !ready())
                 return set_msg(ctx, BZ_ERR_CUDA, std::string(what) + ": result not posted");
             if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60))
                 return set_msg(ctx, BZ_ERR_TIMEOUT, std::string(what) + ": wait");
@@ -911,18 +912,40 @@ int mapped_wait(bz_ctx *ctx, size_t offset, uint32_t seq, const char *what) {
     return BZ_OK;
 }
 
-int msg_wait(bz_ctx *ctx, uint32_t seq, uint64_t u0[2], uint64_t u2[2]) {
-    const int rc = mapped_wait(ctx, 64, seq, "sumcheck message");
+int mapped_wait(bz_ctx *ctx, size_t offset, uint32_t seq, const char *what) {
+    const volatile uint32_t *sp = (const volatile uint32_t *)((uint8_t *)ctx->h_mbox + offset);
+    return spin_wait(ctx, what, [&] { return *sp == seq; });
+}
+
+// An element is three words of 44 bits below the low 20 bits of the message's
+// number; each word is one access, so those that carry the number are final.
+int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
+                  uint64_t *out) {
+    const uint64_t *hp = (const uint64_t *)((uint8_t *)ctx->h_mbox + offset);
+    const uint64_t tag = (uint64_t)seq << 44, m = ((uint64_t)1 << 44) - 1;
+    int at = 0;  // words seen with the tag
+    uint64_t w[3];
+    return spin_wait(ctx, what, [&] {
+        for (; at < 3 * n; ++at) {
+            const uint64_t v = __atomic_load_n(hp + at, __ATOMIC_RELAXED);
+            if ((v & ~m) != tag) return false;
+            w[at % 3] = v & m;
+            if (at % 3 == 2) {
+                out[2 * (at / 3)] = w[0] | (w[1] << 44);
+                out[2 * (at / 3) + 1] = (w[1] >> 20) | (w[2] << 24);
+            }
+        }
+        return true;
+    });
+}
+
+int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2]) {
+    uint64_t u[4 * kMsgPosts];
+    const int rc = elements_wait(ctx, kMsgOffset, 2 * posts, seq, "sumcheck message", u);
     if (rc) return rc;
-    const volatile uint64_t *h = (const volatile uint64_t *)ctx->h_mbox;
-    if (u0) {
-        u0[0] = h[0];
-        u0[1] = h[1];
-    }
-    if (u2) {
-        u2[0] = h[2];
-        u2[1] = h[3];
-    }
+    for (int i = 4; i < 4 * posts; ++i) u[i & 3] ^= u[i];
+    if (u0) std::copy(u, u + 2, u0);
+    if (u2) std::copy(u + 2, u + 4, u2);
     return BZ_OK;
 }
 
@@ -939,9 +962,9 @@ int fold_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
     return BZ_OK;
 }
 
-// The gate: r at byte 128 and the go word at byte 192 of the mapped mailbox;
-// the kernel's time-out record at byte 832 of the small device buffer.
-static uint8_t *gate_host(bz_ctx *ctx) { return (uint8_t *)ctx->h_mbox + 128; }
+// The gate: three tagged words at byte 128 of the mapped mailbox; the kernel's
+// time-out record at byte 832 of the small device buffer.
+static uint64_t *gate_host(bz_ctx *ctx) { return (uint64_t *)((uint8_t *)ctx->h_mbox + 128); }
 
 // Armed only while every CTA of the fold fits on the GPU at once, so that
 // the CTAs that wait at the gate are few.
@@ -963,8 +986,7 @@ bool gate_gave_up(bz_ctx *ctx) {
 RGate next_gate(bz_ctx *ctx, uint64_t limit_ns) {
     if (++ctx->gate_seq >= kGateCancel) ctx->gate_seq = 1;
     RGate g;
-    g.r = (const uint64_t *)((uint8_t *)ctx->d_mbox + 128);
-    g.go = (const uint32_t *)((uint8_t *)ctx->d_mbox + 192);
+    g.words = (const uint64_t *)((uint8_t *)ctx->d_mbox + 128);
     g.seq = ctx->gate_seq;
     g.err = (uint32_t *)((uint8_t *)ctx->d_small + 832);
     g.limit_ns = limit_ns;
@@ -994,12 +1016,12 @@ int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, ui
     return BZ_OK;
 }
 
-// r first, then (release) the go word.
 void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]) {
-    uint64_t *hr = (uint64_t *)gate_host(ctx);
-    __atomic_store_n(&hr[0], r[0], __ATOMIC_RELAXED);
-    __atomic_store_n(&hr[1], r[1], __ATOMIC_RELAXED);
-    __atomic_store_n((uint32_t *)(gate_host(ctx) + 64), a->gate_seq, __ATOMIC_RELEASE);
+    uint64_t *g = gate_host(ctx);
+    const uint64_t tag = (uint64_t)a->gate_seq << 44, m = ((uint64_t)1 << 44) - 1;
+    __atomic_store_n(&g[0], (r[0] & m) | tag, __ATOMIC_RELAXED);
+    __atomic_store_n(&g[1], (((r[0] >> 44) | (r[1] << 20)) & m) | tag, __ATOMIC_RELAXED);
+    __atomic_store_n(&g[2], (r[1] >> 24) | tag, __ATOMIC_RELAXED);
     a->live = false;
 }
 
@@ -1007,8 +1029,8 @@ void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]) {
 // stream is drained so that nothing armed outlives the call.
 int fold_cancel(bz_ctx *ctx, ArmedFold *a) {
     if (!a->live) return BZ_OK;
-    __atomic_store_n((uint32_t *)(gate_host(ctx) + 64), a->gate_seq | kGateCancel,
-                     __ATOMIC_RELEASE);
+    __atomic_store_n(gate_host(ctx), (uint64_t)(a->gate_seq | kGateCancel) << 44,
+                     __ATOMIC_RELAXED);
     a->live = false;
     BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return BZ_OK;
@@ -1026,7 +1048,7 @@ int bz_fold_and_msg_lsb(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, s
     uint32_t seq = 0;
     int rc = fold_launch(ctx, d_f, d_b, n, r, d_nf, d_nb, &seq);
     if (rc) return rc;
-    return msg_wait(ctx, seq, u0, u2);
+    return msg_wait(ctx, seq, fold_posts(n, ctx->num_sms), u0, u2);
 }
 
 int bz_fold_gate_check(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
@@ -1040,7 +1062,7 @@ int bz_fold_gate_check(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, si
     if (rc) return rc;
     if (mode == 0) {
         fold_open(ctx, &a, r);
-        return msg_wait(ctx, a.msg_seq, u0, u2);
+        return msg_wait(ctx, a.msg_seq, fold_posts(n, ctx->num_sms), u0, u2);
     }
     if (mode == 1) return fold_cancel(ctx, &a);
     // mode 2: nothing is posted; the kernel's CTAs give up at the time limit
@@ -1065,7 +1087,7 @@ int bz_round_msg_lsb(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size
                                       (uint64_t *)ctx->scratch, nullptr, ctx->stream, ctx->num_sms,
                                       &post);
     BZ_CUDA(ctx, cudaGetLastError());
-    return msg_wait(ctx, post.seq_val, u0, u2);
+    return msg_wait(ctx, post.seq_val, round_msg_posts(n, ctx->num_sms), u0, u2);
 }
 
 int bz_partial_eval_lsb(bz_ctx *ctx, const uint64_t *d_in, size_t n, const uint64_t *rs, size_t k,
