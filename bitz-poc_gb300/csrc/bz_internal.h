@@ -152,6 +152,11 @@ struct MsgPost {
     uint64_t *words;       // device view of mapped host memory (6 tagged words a post)
     uint32_t seq_val;
 };
+// Elements posted to mapped host memory (post.cuh).
+struct ElementPost {
+    uint64_t *words;  // device view: 3 tagged words an element
+    uint32_t seq;
+};
 // Posts of a message kernel of `grid` CTAs: one by each CTA, whose sum is the
 // message, or one by the last.
 constexpr int kMsgPosts = 16;
@@ -185,8 +190,10 @@ int launch_partial_eval_round(const uint4 *d_in, size_t n, uint4 r, uint4 *d_out
                               cudaStream_t st);
 // eq over the k coordinates of `point` (host memory, 2 words each)
 int launch_build_eq(const uint64_t *point, size_t k, uint4 *d_out, cudaStream_t st, int num_sms);
+// Posts the 128 outputs.
 int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_partials,
-                   uint4 *d_sv, cudaStream_t st, int num_sms);
+                   const ElementPost &post, cudaStream_t st, int num_sms);
+int launch_post_elements(const uint4 *d_in, int n, const ElementPost &post, cudaStream_t st);
 size_t sv_partials_bytes(int num_sms);
 int launch_phi(const uint4 *d_eq_hi, size_t n, const uint4 *d_eq_r2, uint4 *d_out,
                cudaStream_t st, int num_sms);
@@ -222,15 +229,15 @@ int launch_induce_basis(uint4 *d_domain, int log_d, const uint64_t *d_pos, const
                         int nq, const uint4 *d_tw, cudaStream_t st);
 // d_b[j] += beta * d_nb[j]
 int launch_glue(uint4 *d_b, const uint4 *d_nb, size_t n, uint4 beta, cudaStream_t st);
-// d_out[0] = sum_j d_f[j] * d_b[j]; d_partial holds dot_partials_count(n) elements.
+// Posts sum_j d_f[j] * d_b[j]; d_partial holds dot_partials_count(n) elements.
 size_t dot_partials_count(size_t n, int num_sms);
-int launch_dot(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 *d_partial, uint4 *d_out,
-               cudaStream_t st, int num_sms);
-// d_out[0] = sum_h head[h] * sum_j p[h 2^lo + j] * tail[j] over n_blocks blocks;
+int launch_dot(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 *d_partial,
+               const ElementPost &post, cudaStream_t st, int num_sms);
+// Posts sum_h head[h] * sum_j p[h 2^lo + j] * tail[j] over n_blocks blocks;
 // d_partial holds split_dot_partials(n_blocks) elements.
 size_t split_dot_partials(size_t n_blocks, int num_sms);
 int launch_split_dot(const uint4 *d_p, const uint4 *d_tail, int lo, const uint4 *d_head,
-                     size_t n_blocks, uint4 *d_partial, uint4 *d_out, cudaStream_t st,
+                     size_t n_blocks, uint4 *d_partial, const ElementPost &post, cudaStream_t st,
                      int num_sms);
 // d_b[i] += eta * head[i >> lo] * tail[i mod 2^lo]
 int launch_eq_axpy(uint4 *d_b, const uint4 *d_tail, int lo, const uint4 *d_head, uint4 eta,

@@ -13,6 +13,7 @@
 #include "bz_internal.h"
 #include "chain.cuh"
 #include "gf128.cuh"
+#include "post.cuh"
 #include "t16.cuh"
 #include "t8.cuh"
 
@@ -77,27 +78,15 @@ __device__ __forceinline__ uint4 reduce_pair(uint64_t word) {
     return gf_reduce(x);
 }
 
-// Where a message goes: a mailbox in mapped host memory.  A field element is
-// posted as three words of 44 bits, each with the low 20 bits of the message's
-// number above them.  A 64-bit store is one access, so a word whose tag is
-// right holds this message's bits and the host needs no flag that is ordered
-// behind them.  With a system-scope release store of a flag (and the sums
-// reduced by shuffles) the end of a one-CTA round took 1.74 us, now 0.45.
-// Without a mailbox (ticket null) the caller launches finish_msg_kernel.
+// Where a message goes: a mailbox in mapped host memory, as tagged elements.
+// With a system-scope release store of a flag (and the sums reduced by
+// shuffles) the end of a one-CTA round took 1.74 us, now 0.45.  Without a
+// mailbox (ticket null) the caller launches finish_msg_kernel.
 struct MsgMailbox {
     unsigned int *ticket = nullptr;  // device counter, 0 between launches
     uint64_t *words = nullptr;       // mapped host memory: u0, u2
     uint32_t seq_val = 0;
 };
-
-__device__ __forceinline__ void post_element(uint64_t *words, uint32_t seq, uint4 v) {
-    const uint64_t lo = lo64(v), hi = hi64(v), tag = (uint64_t)seq << 44;
-    const uint64_t m = ((uint64_t)1 << 44) - 1;
-    volatile uint64_t *o = words;
-    o[0] = (lo & m) | tag;
-    o[1] = (((lo >> 44) | (hi << 20)) & m) | tag;
-    o[2] = (hi >> 24) | tag;
-}
 
 // Lanes 0 and 1 of the calling warp post u0 and u2.
 __device__ __forceinline__ void post_pair(uint64_t word, const MsgMailbox &mb) {
@@ -853,9 +842,9 @@ __global__ void __launch_bounds__(kSvTile *kSvGroups, 2) sv_fold_kernel(const ui
     }
 }
 
-// CTA j XORs output j of every partial.
+// CTA j XORs output j of every partial and posts it.
 __global__ void __launch_bounds__(128) sv_finish_kernel(const uint4 *partials, int n_ctas,
-                                                        uint4 *sv) {
+                                                        ElementPost post) {
     __shared__ uint4 red[4];
     chain_wait();
     uint4 acc = make_uint4(0, 0, 0, 0);
@@ -871,20 +860,33 @@ __global__ void __launch_bounds__(128) sv_finish_kernel(const uint4 *partials, i
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0)
-        sv[blockIdx.x] = gf_add(gf_add(red[0], red[1]), gf_add(red[2], red[3]));
+        post_element(post.words + 3 * blockIdx.x, post.seq,
+                     gf_add(gf_add(red[0], red[1]), gf_add(red[2], red[3])));
 }
 
 size_t sv_partials_bytes(int num_sms) { return (size_t)num_sms * 2 * 128 * sizeof(uint4); }
 
 int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_partials,
-                   uint4 *d_sv, cudaStream_t st, int num_sms) {
+                   const ElementPost &post, cudaStream_t st, int num_sms) {
     const uint64_t tiles = (n + kSvTile - 1) / kSvTile;
     const int grid = (int)std::max<uint64_t>(
         1, std::min<uint64_t>((tiles + kSvGroups - 1) / kSvGroups, (uint64_t)num_sms * 2));
     launch_chained(sv_fold_kernel, grid, kSvTile * kSvGroups, 0, st, d_packed, d_eq, n,
                    d_partials);
-    launch_chained(sv_finish_kernel, 128, 128, 0, st, d_partials, grid, d_sv);
+    launch_chained(sv_finish_kernel, 128, 128, 0, st, d_partials, grid, post);
     return 2;
+}
+
+// n elements of device memory to the mailbox.
+__global__ void post_elements_kernel(const uint4 *in, int n, ElementPost post) {
+    chain_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) post_element(post.words + 3 * i, post.seq, in[i]);
+}
+
+int launch_post_elements(const uint4 *d_in, int n, const ElementPost &post, cudaStream_t st) {
+    launch_chained(post_elements_kernel, (unsigned)(n + 127) / 128, 128, 0, st, d_in, n, post);
+    return 1;
 }
 
 // phi_from_words with phi_byte_tables (src/ligerito.rs:384-427): phi(y) =

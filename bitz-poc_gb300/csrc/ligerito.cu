@@ -26,6 +26,7 @@
 #include "bz_internal.h"
 #include "chain.cuh"
 #include "gf128.cuh"
+#include "post.cuh"
 #include "t8.cuh"
 
 namespace bz {
@@ -116,14 +117,14 @@ __global__ void __launch_bounds__(kThreads) tntt_tile_kernel(uint4 *data, int lo
     for (int i = threadIdx.x; i < (1 << kTileLog); i += blockDim.x) data[base + i] = tile[i];
 }
 
-// out[0] = XOR of in[0..n) (one CTA)
+// Posts the XOR of in[0..n) (one CTA).
 __global__ void __launch_bounds__(kThreads) xor_reduce_kernel(const uint4 *in, uint64_t n,
-                                                              uint4 *out) {
+                                                              ElementPost post) {
     chain_wait();
     uint4 acc = make_uint4(0, 0, 0, 0);
     for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) acc = gf_add(acc, in[i]);
     acc = cta_xor_u4(acc);
-    if (threadIdx.x == 0) out[0] = acc;
+    if (threadIdx.x == 0) post_element(post.words, post.seq, acc);
 }
 
 __global__ void glue_kernel(uint4 *b, const uint4 *nb, uint64_t n, uint4 beta) {
@@ -271,7 +272,7 @@ size_t split_dot_partials(size_t n_blocks, int num_sms) {
 }
 
 int launch_split_dot(const uint4 *d_p, const uint4 *d_tail, int lo, const uint4 *d_head,
-                     size_t n_blocks, uint4 *d_partial, uint4 *d_out, cudaStream_t st,
+                     size_t n_blocks, uint4 *d_partial, const ElementPost &post, cudaStream_t st,
                      int num_sms) {
     const size_t cap = split_dot_partials(n_blocks, num_sms);
     size_t ctas = std::max<size_t>(1, std::min(n_blocks, cap));
@@ -284,7 +285,7 @@ int launch_split_dot(const uint4 *d_p, const uint4 *d_tail, int lo, const uint4 
         launch_chained(split_dot_kernel, (unsigned)ctas, kThreads, 0, st, d_p, d_tail, lo, d_head,
                        n_blocks, d_partial);
     }
-    launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, d_out);
+    launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, post);
     return 2;
 }
 
@@ -333,11 +334,11 @@ size_t dot_partials_count(size_t n, int num_sms) {
     return want < cap ? (want ? want : 1) : cap;
 }
 
-int launch_dot(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 *d_partial, uint4 *d_out,
-               cudaStream_t st, int num_sms) {
+int launch_dot(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 *d_partial,
+               const ElementPost &post, cudaStream_t st, int num_sms) {
     const size_t ctas = dot_partials_count(n, num_sms);
     launch_chained(dot_kernel, (unsigned)ctas, kThreads, 0, st, d_f, d_b, n, d_partial);
-    launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, d_out);
+    launch_chained(xor_reduce_kernel, 1, kThreads, 0, st, d_partial, ctas, post);
     return 2;
 }
 

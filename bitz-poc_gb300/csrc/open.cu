@@ -204,24 +204,23 @@ struct Sumcheck {
         while (((size_t)1 << n) < len) ++n;
         const size_t parts = bz::dot_partials_count(len, ctx->num_sms);
         void *scratch = nullptr;
-        const size_t bytes = (len + 1 + parts) * 16;
+        const size_t bytes = (len + parts) * 16;
         int rc = bz::dev_alloc(ctx, bytes, &scratch, false);
         if (rc) return rc;
-        uint4 *d_eq = (uint4 *)scratch, *d_y = d_eq + len, *d_part = d_y + 1;
+        uint4 *d_eq = (uint4 *)scratch, *d_part = d_eq + len;
         std::vector<uint64_t> z(2 * (size_t)n);
         for (uint32_t s = 0; s < count && !rc; ++s) {
             for (uint32_t i = 0; i < n; ++i) tr->sample_f128(&z[2 * i]);
             ctx->launches += bz::launch_build_eq(z.data(), n, d_eq, ctx->stream, ctx->num_sms);
             uint64_t u0[2], u2[2], y[2];
-            rc = bz_round_msg_lsb(ctx, f, (const uint64_t *)d_eq, len, u0, u2);
-            if (rc) break;
-            ctx->launches += bz::launch_dot((const uint4 *)f, d_eq, len, d_part, d_y,
+            uint32_t seq = 0;
+            if ((rc = bz::round_msg_launch(ctx, f, (const uint64_t *)d_eq, len, &seq))) break;
+            const bz::ElementPost post = bz::next_element_post(ctx);
+            ctx->launches += bz::launch_dot((const uint4 *)f, d_eq, len, d_part, post,
                                             ctx->stream, ctx->num_sms);
-            if (cudaMemcpyAsync(y, d_y, 16, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-                cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-                rc = bz::set_msg(ctx, BZ_ERR_CUDA, "out-of-domain evaluation");
-                break;
-            }
+            rc = bz::msg_wait(ctx, seq, bz::round_msg_posts(len, ctx->num_sms), u0, u2);
+            if (!rc) rc = bz::posted_wait(ctx, post, 1, "out-of-domain evaluation", y);
+            if (rc) break;
             tr->observe_f128(y);
             ood_values.insert(ood_values.end(), {y[0], y[1]});
             record(u0, u2);
@@ -261,16 +260,17 @@ int open_rows_on(bz_commitment *c, const std::vector<uint64_t> &queries, bzp::Le
                  cudaStream_t st) {
     const size_t q = queries.size();
     const size_t lanes = c->shape.leaf_bytes() / 16;
+    std::vector<uint64_t> idx;
+    int rc = bz::commitment_proof_nodes(c, queries.data(), q, idx);
+    if (rc) return rc;
     out.rows.lens.assign(q, lanes);
+    out.rows.data.resize(q * lanes * 2 + 4 * idx.size());
+    rc = bz::commitment_open_on(c, queries.data(), q, idx, out.rows.data.data(), st);
+    if (rc) return rc;
+    const uint8_t *nodes = (const uint8_t *)(out.rows.data.data() + q * lanes * 2);
+    out.hashes.assign(nodes, nodes + 32 * idx.size());
     out.rows.data.resize(q * lanes * 2);
-    int rc = bz::commitment_rows_on(c, queries.data(), q, out.rows.data.data(), st);
-    if (rc) return rc;
-    size_t n_hashes = 0;
-    rc = bz::commitment_multiproof_on(c, queries.data(), q, nullptr, 0, &n_hashes, st);
-    if (rc) return rc;
-    out.hashes.resize(n_hashes * 32);
-    return bz::commitment_multiproof_on(c, queries.data(), q, out.hashes.data(), n_hashes,
-                                        &n_hashes, st);
+    return BZ_OK;
 }
 
 int open_rows(bz_commitment *c, const std::vector<uint64_t> &queries, bzp::Level &out) {
@@ -621,10 +621,17 @@ int bz_ligerito_prove(bz_ctx *ctx, bz_transcript *transcript, bz_commitment *c0,
         if (i == r - 1) {
             // finish(): yr = f, every element observed (:3776-3790)
             p->yr.resize(2 * sc.len);
-            if (cudaMemcpyAsync(p->yr.data(), sc.f, 16 * sc.len, cudaMemcpyDeviceToHost,
-                                ctx->stream) != cudaSuccess ||
-                cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+            if (sc.len <= (size_t)bz::kPostElements) {
+                const bz::ElementPost post = bz::next_element_post(ctx);
+                ctx->launches += bz::launch_post_elements((const uint4 *)sc.f, (int)sc.len, post,
+                                                          ctx->stream);
+                rc = bz::posted_wait(ctx, post, (int)sc.len, "final polynomial", p->yr.data());
+                if (rc) return finish(rc);
+            } else if (cudaMemcpyAsync(p->yr.data(), sc.f, 16 * sc.len, cudaMemcpyDeviceToHost,
+                                       ctx->stream) != cudaSuccess ||
+                       cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
                 return finish(bz::set_msg(ctx, BZ_ERR_CUDA, "final polynomial"));
+            }
             for (size_t e = 0; e < sc.len; ++e) tr->observe_f128(&p->yr[2 * e]);
             uint64_t nonce;
             rc = bz_transcript_grind_pow(ctx, transcript, cfg->grinding_bits[i + 1], &nonce);

@@ -148,6 +148,49 @@ void transpose_bits_128(const uint64_t *s, uint64_t *out) {
         }
 }
 
+// The ring switch, its basis left to the context stream's next kernels.
+int ring_switch(bz_ctx *ctx, bz_transcript *transcript, const uint64_t *d_packed, size_t n,
+                const uint64_t *r_hi, uint64_t s_v[256], uint64_t *d_basis, uint64_t target[2]) {
+    bzh::Transcript *tr = bz_transcript_inner(transcript);
+    if (!ctx || !tr || !d_packed || !s_v || !d_basis || !target) return BZ_ERR_ARG;
+    if (!pow2(n) || n > ((size_t)1 << 40))
+        return bz::set_msg(ctx, BZ_ERR_SHAPE, "packed message length must be a power of two");
+    const uint32_t m = log2_exact(n);
+    if (m && !r_hi) return BZ_ERR_ARG;
+    void *d_eq = nullptr;  // eq(r_hi) (n entries), then eq(r'') (128 entries)
+    int rc = bz::dev_alloc(ctx, (n + 128) * 16, &d_eq, false);
+    if (rc) return rc;
+    uint4 *d_eq_r2 = (uint4 *)d_eq + n;
+    auto done = [&](int code) {
+        bz::dev_free(ctx, d_eq, 0, false);
+        if (!code && cudaGetLastError() != cudaSuccess)
+            return bz::set_msg(ctx, BZ_ERR_CUDA, "ring switch");
+        return code;
+    };
+    ctx->launches += bz::launch_build_eq(r_hi, m, (uint4 *)d_eq, ctx->stream, ctx->num_sms);
+    if ((rc = bz_sv_fold(ctx, d_packed, (const uint64_t *)d_eq, n, s_v))) return done(rc);
+    absorb_gf_slice(tr, 0x20, s_v, 128);  // absorb_sv (src/ligerito.rs:248-250)
+    uint64_t r2[14], eq_r2[256];
+    for (int i = 0; i < 7; ++i) tr->sample_f128(r2 + 2 * i);
+    // eq(r'') on the device (128 entries), posted for beta0
+    const bz::ElementPost post = bz::next_element_post(ctx);
+    ctx->launches += bz::launch_build_eq(r2, 7, d_eq_r2, ctx->stream, ctx->num_sms);
+    ctx->launches += bz::launch_post_elements(d_eq_r2, 128, post, ctx->stream);
+    ctx->launches += bz::launch_phi((const uint4 *)d_eq, n, d_eq_r2, (uint4 *)d_basis, ctx->stream,
+                                    ctx->num_sms);
+    uint64_t s_u[256];
+    transpose_bits_128(s_v, s_u);
+    if ((rc = bz::posted_wait(ctx, post, 128, "ring switch", eq_r2))) return done(rc);
+    target[0] = target[1] = 0;
+    for (int u = 0; u < 128; ++u) {
+        uint64_t p[2];
+        bz::hgf_mul(s_u + 2 * u, eq_r2 + 2 * u, p);
+        target[0] ^= p[0];
+        target[1] ^= p[1];
+    }
+    return done(rc);
+}
+
 }  // namespace
 
 extern "C" {
@@ -189,14 +232,13 @@ int bz_pcs_prove_round0(bz_ctx *ctx, bz_transcript *transcript, const uint64_t *
     int rc = eq.build(ctx, r->point, r->vars);
     void *tmp = nullptr;
     const size_t parts = bz::split_dot_partials(eq.n_head, ctx->num_sms);
-    if (!rc) rc = bz::dev_alloc(ctx, (parts + 1) * 16, &tmp, false);
+    if (!rc) rc = bz::dev_alloc(ctx, parts * 16, &tmp, false);
     if (!rc) {
-        uint4 *d_part = (uint4 *)tmp, *d_y = d_part + parts;
+        const bz::ElementPost post = bz::next_element_post(ctx);
         ctx->launches += bz::launch_split_dot((const uint4 *)d_packed, eq.tail, eq.lo, eq.head,
-                                              eq.n_head, d_part, d_y, ctx->stream, ctx->num_sms);
-        if (cudaMemcpyAsync(r->y, d_y, 16, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-            cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-            rc = bz::set_msg(ctx, BZ_ERR_CUDA, "out-of-domain evaluation");
+                                              eq.n_head, (uint4 *)tmp, post, ctx->stream,
+                                              ctx->num_sms);
+        rc = bz::posted_wait(ctx, post, 1, "out-of-domain evaluation", r->y);
     }
     if (tmp) bz::dev_free(ctx, tmp, 0, false);
     eq.release(ctx);
@@ -236,39 +278,10 @@ int bz_round0_free(bz_round0 *r) {
 int bz_pcs_ring_switch(bz_ctx *ctx, bz_transcript *transcript, const uint64_t *d_packed, size_t n,
                        const uint64_t *r_hi, uint64_t s_v[256], uint64_t *d_basis,
                        uint64_t target[2]) {
-    bzh::Transcript *tr = bz_transcript_inner(transcript);
-    if (!ctx || !tr || !d_packed || !s_v || !d_basis || !target) return BZ_ERR_ARG;
-    if (!pow2(n) || n > ((size_t)1 << 40))
-        return bz::set_msg(ctx, BZ_ERR_SHAPE, "packed message length must be a power of two");
-    const uint32_t m = log2_exact(n);
-    if (m && !r_hi) return BZ_ERR_ARG;
-    void *d_eq = nullptr;  // eq(r_hi) (n entries), then eq(r'') (128 entries)
-    int rc = bz::dev_alloc(ctx, (n + 128) * 16, &d_eq, false);
+    const int rc = ring_switch(ctx, transcript, d_packed, n, r_hi, s_v, d_basis, target);
     if (rc) return rc;
-    uint64_t *d_eq_r2 = (uint64_t *)d_eq + 2 * n;
-    auto done = [&](int code) {
-        bz::dev_free(ctx, d_eq, 0, false);
-        return code;
-    };
-    if ((rc = bz_build_eq_lsb(ctx, r_hi, m, (uint64_t *)d_eq))) return done(rc);
-    if ((rc = bz_sv_fold(ctx, d_packed, (const uint64_t *)d_eq, n, s_v))) return done(rc);
-    absorb_gf_slice(tr, 0x20, s_v, 128);  // absorb_sv (src/ligerito.rs:248-250)
-    uint64_t r2[14], eq_r2[256];
-    for (int i = 0; i < 7; ++i) tr->sample_f128(r2 + 2 * i);
-    // eq(r'') on the device (128 entries), copied back for beta0 and Phi
-    if ((rc = bz_build_eq_lsb(ctx, r2, 7, d_eq_r2))) return done(rc);
-    if ((rc = bz_memcpy_d2h(ctx, eq_r2, d_eq_r2, 128 * 16))) return done(rc);
-    uint64_t s_u[256];
-    transpose_bits_128(s_v, s_u);
-    target[0] = target[1] = 0;
-    for (int u = 0; u < 128; ++u) {
-        uint64_t p[2];
-        bz::hgf_mul(s_u + 2 * u, eq_r2 + 2 * u, p);
-        target[0] ^= p[0];
-        target[1] ^= p[1];
-    }
-    rc = bz_phi_from_words(ctx, (const uint64_t *)d_eq, n, eq_r2, d_basis);
-    return done(rc);
+    BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return BZ_OK;
 }
 
 int bz_pcs_open_basis(bz_ctx *ctx, bz_transcript *transcript, bz_commitment *c0,
@@ -310,8 +323,7 @@ int bz_pcs_open_bit_mle(bz_ctx *ctx, bz_transcript *transcript, bz_commitment *c
     int rc = bz::dev_alloc(ctx, n * 16, &d_b, false);
     if (rc) return rc;
     uint64_t target[2];
-    rc = bz_pcs_ring_switch(ctx, transcript, d_packed, n, point + 2 * 7, s_v, (uint64_t *)d_b,
-                            target);
+    rc = ring_switch(ctx, transcript, d_packed, n, point + 2 * 7, s_v, (uint64_t *)d_b, target);
     if (!rc)
         rc = bz_pcs_open_basis(ctx, transcript, c0, d_packed, round0, (uint64_t *)d_b, target,
                                cfg, out);

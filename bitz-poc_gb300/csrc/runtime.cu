@@ -305,11 +305,11 @@ int commitment_rows_on(bz_commitment *c, const uint64_t *positions, size_t q, ui
     return BZ_OK;
 }
 
-int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t q, uint8_t *out,
-                             size_t cap, size_t *n_hashes, cudaStream_t st) {
+int commitment_proof_nodes(bz_commitment *c, const uint64_t *positions, size_t q,
+                           std::vector<uint64_t> &idx) {
     bz_ctx *ctx = c->ctx;
     const uint64_t num_leaves = c->shape.n_leaves();
-    *n_hashes = 0;
+    idx.clear();
     if (q == 0 || num_leaves == 1) return BZ_OK;
     // merkle_multi_proof (merkle.rs:688-741): sorted unique positions, walk
     // levels bottom-up, emit the sibling of every node whose sibling is not
@@ -319,7 +319,6 @@ int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t
         if (p >= num_leaves) return set_msg(ctx, BZ_ERR_ARG, "position out of range");
     std::sort(act.begin(), act.end());
     act.erase(std::unique(act.begin(), act.end()), act.end());
-    std::vector<uint64_t> idx;
     uint64_t level_start = 0, level_len = num_leaves;
     while (level_len > 1) {
         std::vector<uint64_t> next;
@@ -340,6 +339,15 @@ int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t
         level_start += level_len;
         level_len >>= 1;
     }
+    return BZ_OK;
+}
+
+int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t q, uint8_t *out,
+                             size_t cap, size_t *n_hashes, cudaStream_t st) {
+    bz_ctx *ctx = c->ctx;
+    std::vector<uint64_t> idx;
+    *n_hashes = 0;
+    if (int rc = commitment_proof_nodes(c, positions, q, idx)) return rc;
     *n_hashes = idx.size();
     if (!out) return BZ_OK;  // size query
     if (idx.size() > cap) return set_msg(ctx, BZ_ERR_ARG, "multiproof buffer too small");
@@ -357,6 +365,35 @@ int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t
     cudaMemcpyAsync(out, d_out, idx.size() * 32, cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d_idx, st);
     cudaFreeAsync(d_out, st);
+    BZ_CUDA(ctx, cudaStreamSynchronize(st));
+    return BZ_OK;
+}
+
+// One upload, two gathers, one download and one synchronisation.
+int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q,
+                       const std::vector<uint64_t> &idx, uint64_t *out, cudaStream_t st) {
+    bz_ctx *ctx = c->ctx;
+    if (!c->d_cw) return set_msg(ctx, BZ_ERR_STATE, "tree-only commitment: no codeword");
+    const uint64_t n_pos = c->shape.n_leaves();
+    for (size_t i = 0; i < q; ++i)
+        if (positions[i] >= n_pos) return set_msg(ctx, BZ_ERR_ARG, "position out of range");
+    if (q == 0) return BZ_OK;
+    const size_t row_words = c->shape.leaf_bytes() / 8, n_idx = q + idx.size();
+    const size_t out_words = q * row_words + 4 * idx.size();
+    void *mem = nullptr;  // the gathered words, then the indices
+    if (cudaMallocAsync(&mem, (out_words + n_idx) * 8, st) != cudaSuccess) {
+        cudaGetLastError();
+        return set_msg(ctx, BZ_ERR_NOMEM, "opened rows buffer");
+    }
+    uint64_t *d_out = (uint64_t *)mem, *d_idx = d_out + out_words;
+    std::vector<uint64_t> all(positions, positions + q);
+    all.insert(all.end(), idx.begin(), idx.end());
+    cudaMemcpyAsync(d_idx, all.data(), n_idx * 8, cudaMemcpyHostToDevice, st);
+    ctx->launches += launch_gather_rows(c->d_cw, c->shape.log_lanes, d_idx, q, (uint4 *)d_out, st);
+    ctx->launches += launch_gather_nodes(c->d_tree, d_idx + q, idx.size(),
+                                         (uint8_t *)(d_out + q * row_words), st);
+    cudaMemcpyAsync(out, d_out, out_words * 8, cudaMemcpyDeviceToHost, st);
+    cudaFreeAsync(mem, st);
     BZ_CUDA(ctx, cudaStreamSynchronize(st));
     return BZ_OK;
 }
@@ -483,7 +520,7 @@ int bz_ctx_create(int device, uint64_t mem_budget_bytes, bz_ctx **out) {
     }
     if (cudaMalloc(&ctx->d_small, 4096) != cudaSuccess ||
         cudaMemset(ctx->d_small, 0, 4096) != cudaSuccess ||
-        cudaHostAlloc(&ctx->h_mbox, 4096, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostAlloc(&ctx->h_mbox, kMboxBytes, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&ctx->d_mbox, ctx->h_mbox, 0) != cudaSuccess) {
         cudaGetLastError();
         if (ctx->d_small) cudaFree(ctx->d_small);
@@ -492,7 +529,7 @@ int bz_ctx_create(int device, uint64_t mem_budget_bytes, bz_ctx **out) {
         delete ctx;
         return BZ_ERR_CUDA;
     }
-    memset(ctx->h_mbox, 0, 4096);
+    memset(ctx->h_mbox, 0, kMboxBytes);
     *out = ctx;
     return BZ_OK;
 }
@@ -873,8 +910,11 @@ static bool pow2(size_t n) { return n && !(n & (n - 1)); }
 
 namespace bz {
 
-// The messages' posts in the mapped mailbox (kMsgPosts of 48 bytes).
-constexpr size_t kMsgOffset = 3072;
+// The messages' posts in the mapped mailbox (kMsgPosts of 48 bytes) and the
+// element posts (kPostElements of 24 bytes).
+constexpr size_t kMsgOffset = 3072, kElementsOffset = 4096;
+static_assert(kMsgOffset + 48 * kMsgPosts <= kElementsOffset &&
+              kElementsOffset + 24 * kPostElements <= kMboxBytes);
 
 // Mailbox post for the next message kernel on the context stream.
 static MsgPost next_post(bz_ctx *ctx) {
@@ -939,6 +979,15 @@ int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *w
     });
 }
 
+ElementPost next_element_post(bz_ctx *ctx) {
+    if (++ctx->mbox_seq == 0) ++ctx->mbox_seq;
+    return {(uint64_t *)((uint8_t *)ctx->d_mbox + kElementsOffset), ctx->mbox_seq};
+}
+
+int posted_wait(bz_ctx *ctx, const ElementPost &post, int n, const char *what, uint64_t *out) {
+    return elements_wait(ctx, kElementsOffset, n, post.seq, what, out);
+}
+
 int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2]) {
     uint64_t u[4 * kMsgPosts];
     const int rc = elements_wait(ctx, kMsgOffset, 2 * posts, seq, "sumcheck message", u);
@@ -957,6 +1006,19 @@ int fold_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
     ctx->launches += launch_fold_and_msg((const uint4 *)d_f, (const uint4 *)d_b, n, to_u4(r),
                                          (uint4 *)d_nf, (uint4 *)d_nb, (uint64_t *)ctx->scratch,
                                          nullptr, ctx->stream, ctx->num_sms, &post);
+    BZ_CUDA(ctx, cudaGetLastError());
+    *msg_seq = post.seq_val;
+    return BZ_OK;
+}
+
+int round_msg_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
+                     uint32_t *msg_seq) {
+    int rc = ensure_scratch(ctx, fold_partials_bytes(n));
+    if (rc) return rc;
+    const MsgPost post = next_post(ctx);
+    ctx->launches += launch_round_msg((const uint4 *)d_f, (const uint4 *)d_b, n,
+                                      (uint64_t *)ctx->scratch, nullptr, ctx->stream, ctx->num_sms,
+                                      &post);
     BZ_CUDA(ctx, cudaGetLastError());
     *msg_seq = post.seq_val;
     return BZ_OK;
@@ -1080,14 +1142,10 @@ int bz_round_msg_lsb(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size
                      uint64_t u0[2], uint64_t u2[2]) {
     if (!ctx || !d_f || !d_b) return BZ_ERR_ARG;
     if (!pow2(n) || n < 2) return set_msg(ctx, BZ_ERR_SHAPE, "n must be a power of two >= 2");
-    int rc = ensure_scratch(ctx, fold_partials_bytes(n));
+    uint32_t seq = 0;
+    const int rc = round_msg_launch(ctx, d_f, d_b, n, &seq);
     if (rc) return rc;
-    const MsgPost post = next_post(ctx);
-    ctx->launches += launch_round_msg((const uint4 *)d_f, (const uint4 *)d_b, n,
-                                      (uint64_t *)ctx->scratch, nullptr, ctx->stream, ctx->num_sms,
-                                      &post);
-    BZ_CUDA(ctx, cudaGetLastError());
-    return msg_wait(ctx, post.seq_val, round_msg_posts(n, ctx->num_sms), u0, u2);
+    return msg_wait(ctx, seq, round_msg_posts(n, ctx->num_sms), u0, u2);
 }
 
 int bz_partial_eval_lsb(bz_ctx *ctx, const uint64_t *d_in, size_t n, const uint64_t *rs, size_t k,
@@ -1134,15 +1192,13 @@ int bz_build_eq_lsb(bz_ctx *ctx, const uint64_t *point, size_t k, uint64_t *d_ou
 int bz_sv_fold(bz_ctx *ctx, const uint64_t *d_packed, const uint64_t *d_eq, size_t n,
                uint64_t *sv) {
     if (!ctx || !d_packed || !d_eq || !sv) return BZ_ERR_ARG;
-    int rc = ensure_scratch(ctx, sv_partials_bytes(ctx->num_sms) + 128 * 16);
+    int rc = ensure_scratch(ctx, sv_partials_bytes(ctx->num_sms));
     if (rc) return rc;
-    uint4 *d_sv = (uint4 *)(ctx->scratch + sv_partials_bytes(ctx->num_sms));
+    const ElementPost post = next_element_post(ctx);
     ctx->launches += launch_sv_fold((const uint4 *)d_packed, (const uint4 *)d_eq, n,
-                                    (uint4 *)ctx->scratch, d_sv, ctx->stream, ctx->num_sms);
+                                    (uint4 *)ctx->scratch, post, ctx->stream, ctx->num_sms);
     BZ_CUDA(ctx, cudaGetLastError());
-    BZ_CUDA(ctx, cudaMemcpyAsync(sv, d_sv, 128 * 16, cudaMemcpyDeviceToHost, ctx->stream));
-    BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return BZ_OK;
+    return posted_wait(ctx, post, 128, "partial evaluations", sv);
 }
 
 int bz_phi_from_words(bz_ctx *ctx, const uint64_t *d_eq_hi, size_t n, const uint64_t *eq_r2,

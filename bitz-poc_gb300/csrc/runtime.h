@@ -37,6 +37,10 @@ struct bz_aux_stream {
     cudaEvent_t ev[16] = {};
 };
 
+namespace bz {
+constexpr size_t kMboxBytes = 8192;
+}
+
 struct bz_ctx {
     int device = 0;
     int num_sms = 0;
@@ -53,7 +57,7 @@ struct bz_ctx {
     size_t scratch_bytes = 0;
     void *h_small = nullptr;  // 4 KiB pinned
     void *d_small = nullptr;  // 4 KiB device (zeroed; word 192 is the message ticket)
-    void *h_mbox = nullptr;   // 4 KiB mapped pinned: sumcheck message mailbox
+    void *h_mbox = nullptr;   // 8 KiB mapped pinned: mailbox of posted results
     void *d_mbox = nullptr;   // its device view
     uint32_t mbox_seq = 0;    // last posted sequence number
     std::atomic<uint32_t> root_seq{0};  // commits whose root the mailbox was offered to
@@ -126,6 +130,12 @@ int commitment_rows_on(bz_commitment *c, const uint64_t *positions, size_t q, ui
                        cudaStream_t st);
 int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t q, uint8_t *out,
                              size_t cap, size_t *n_hashes, cudaStream_t st);
+// Tree indices of the nodes of a multi-proof, in its order.
+int commitment_proof_nodes(bz_commitment *c, const uint64_t *positions, size_t q,
+                           std::vector<uint64_t> &idx);
+// Rows and proof nodes together: out holds q rows, then 4 words a node.
+int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q,
+                       const std::vector<uint64_t> &idx, uint64_t *out, cudaStream_t st);
 int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out);
 uint32_t schedule_for(bz_ctx *ctx, const Shape &s);
 int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out,
@@ -178,6 +188,14 @@ int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2
 // message seq, then unpack their n elements (2 words each).
 int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
                   uint64_t *out);
+// The post of up to kPostElements elements by the next kernels on the context
+// stream (one at a time), and the wait for its first n.
+constexpr int kPostElements = 128;
+ElementPost next_element_post(bz_ctx *ctx);
+int posted_wait(bz_ctx *ctx, const ElementPost &post, int n, const char *what, uint64_t *out);
+// bz_round_msg_lsb without the wait.
+int round_msg_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
+                     uint32_t *msg_seq);
 // Spin until the 32-bit word at byte `offset` of the mapped mailbox reads
 // seq, checking the context stream for errors (and for having gone idle
 // without posting) every few hundred spins; 60 s limit.
