@@ -138,10 +138,9 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
                   const RootPost *post = nullptr);
 
 // Gathers: rows of the codeword and arbitrary tree nodes.
-int launch_gather_rows(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, size_t q,
-                       uint4 *d_out, cudaStream_t st);
-int launch_gather_nodes(const uint8_t *d_tree, const uint64_t *d_idx, size_t n, uint8_t *d_out,
-                        cudaStream_t st);
+int launch_gather_open(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, size_t q,
+                       uint4 *d_rows, const uint8_t *d_tree, const uint64_t *d_idx, size_t n,
+                       uint8_t *d_nodes, cudaStream_t st);
 
 // Folds.  d_partials holds fold_partials_bytes(n) bytes.  With `post`, the
 // last CTA of the fold (or message) kernel reduces the partials itself and

@@ -417,40 +417,34 @@ int launch_combine_shard_cvs(const uint8_t *d_cvs, uint32_t world, uint64_t n_le
 // ---------------------------------------------------------------------------
 // Gathers for openings.
 // ---------------------------------------------------------------------------
-__global__ void gather_rows(const uint4 *cw, int log_lanes, const uint64_t *pos, size_t q,
-                            uint4 *out) {
+// Rows `pos` of the codeword to `rows`, nodes `idx` of the tree to `nodes`.  The
+// positions and the outputs may lie in mapped host memory.
+__global__ void gather_open(const uint4 *cw, int log_lanes, const uint64_t *pos, uint64_t q,
+                            uint4 *rows, const uint4 *tree, const uint64_t *idx, uint64_t n,
+                            uint4 *nodes) {
     chain_wait();
     const uint64_t L = (uint64_t)1 << log_lanes;
-    const uint64_t total = q * L;
+    const uint64_t in_rows = q * L, total = in_rows + 2 * n;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = i >> log_lanes, ln = i & (L - 1);
-        out[i] = cw[(pos[r] << log_lanes) | ln];
+        if (i < in_rows) {
+            rows[i] = cw[(pos[i >> log_lanes] << log_lanes) | (i & (L - 1))];
+        } else {
+            const uint64_t k = i - in_rows;
+            nodes[k] = tree[idx[k >> 1] * 2 + (k & 1)];
+        }
     }
 }
 
-__global__ void gather_nodes(const uint4 *tree, const uint64_t *idx, size_t n, uint4 *out) {
-    chain_wait();
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * n) return;
-    out[i] = tree[idx[i >> 1] * 2 + (i & 1)];
-}
-
-int launch_gather_rows(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, size_t q,
-                       uint4 *d_out, cudaStream_t st) {
-    if (q == 0) return 0;
-    const uint64_t total = (uint64_t)q << log_lanes;
+int launch_gather_open(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, size_t q,
+                       uint4 *d_rows, const uint8_t *d_tree, const uint64_t *d_idx, size_t n,
+                       uint8_t *d_nodes, cudaStream_t st) {
+    const uint64_t total = ((uint64_t)q << log_lanes) + 2 * (uint64_t)n;
+    if (total == 0) return 0;
     const unsigned grid = (unsigned)std::min<uint64_t>((total + 255) / 256, 4096);
-    launch_chained(gather_rows, grid, 256, 0, st, d_cw, log_lanes, d_pos, q, d_out);
-    return 1;
-}
-
-int launch_gather_nodes(const uint8_t *d_tree, const uint64_t *d_idx, size_t n, uint8_t *d_out,
-                        cudaStream_t st) {
-    if (n == 0) return 0;
-    launch_chained(gather_nodes, (unsigned)((2 * n + 255) / 256), 256, 0, st,
-                   reinterpret_cast<const uint4 *>(d_tree), d_idx, n,
-                   reinterpret_cast<uint4 *>(d_out));
+    launch_chained(gather_open, grid, 256, 0, st, d_cw, log_lanes, d_pos, (uint64_t)q, d_rows,
+                   reinterpret_cast<const uint4 *>(d_tree), d_idx, (uint64_t)n,
+                   reinterpret_cast<uint4 *>(d_nodes));
     return 1;
 }
 

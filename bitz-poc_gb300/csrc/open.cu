@@ -264,13 +264,10 @@ int open_rows_on(bz_commitment *c, const std::vector<uint64_t> &queries, bzp::Le
     int rc = bz::commitment_proof_nodes(c, queries.data(), q, idx);
     if (rc) return rc;
     out.rows.lens.assign(q, lanes);
-    out.rows.data.resize(q * lanes * 2 + 4 * idx.size());
-    rc = bz::commitment_open_on(c, queries.data(), q, idx, out.rows.data.data(), st);
-    if (rc) return rc;
-    const uint8_t *nodes = (const uint8_t *)(out.rows.data.data() + q * lanes * 2);
-    out.hashes.assign(nodes, nodes + 32 * idx.size());
     out.rows.data.resize(q * lanes * 2);
-    return BZ_OK;
+    out.hashes.resize(32 * idx.size());
+    return bz::commitment_open_on(c, queries.data(), q, out.rows.data.data(), idx.data(),
+                                  idx.size(), out.hashes.data(), st);
 }
 
 int open_rows(bz_commitment *c, const std::vector<uint64_t> &queries, bzp::Level &out) {

@@ -39,6 +39,7 @@ struct bz_aux_stream {
 
 namespace bz {
 constexpr size_t kMboxBytes = 8192;
+constexpr size_t kOpenIdxBytes = (size_t)32 << 10, kOpenBytes = (size_t)256 << 10;
 }
 
 struct bz_ctx {
@@ -59,6 +60,10 @@ struct bz_ctx {
     void *d_small = nullptr;  // 4 KiB device (zeroed; word 192 is the message ticket)
     void *h_mbox = nullptr;   // 8 KiB mapped pinned: mailbox of posted results
     void *d_mbox = nullptr;   // its device view
+    // positions in, rows and nodes out of small openings (mapped pinned); held by
+    // one opening at a time
+    std::mutex open_mu;
+    void *h_open = nullptr, *d_open = nullptr;
     uint32_t mbox_seq = 0;    // last posted sequence number
     std::atomic<uint32_t> root_seq{0};  // commits whose root the mailbox was offered to
     uint32_t gate_seq = 0;    // last armed fold's gate number
@@ -124,18 +129,13 @@ int ensure_scratch(bz_ctx *ctx, size_t bytes);
 // Run job on the context's helper thread; the future holds its status.
 std::future<int> side_async(bz_ctx *ctx, std::function<int()> job);
 void side_shutdown(bz_ctx *ctx);
-// Opened rows and multi-proof of a commitment on stream st (synchronised on
-// return); the C ABI calls run them on the context stream.
-int commitment_rows_on(bz_commitment *c, const uint64_t *positions, size_t q, uint64_t *out,
-                       cudaStream_t st);
-int commitment_multiproof_on(bz_commitment *c, const uint64_t *positions, size_t q, uint8_t *out,
-                             size_t cap, size_t *n_hashes, cudaStream_t st);
 // Tree indices of the nodes of a multi-proof, in its order.
 int commitment_proof_nodes(bz_commitment *c, const uint64_t *positions, size_t q,
                            std::vector<uint64_t> &idx);
-// Rows and proof nodes together: out holds q rows, then 4 words a node.
-int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q,
-                       const std::vector<uint64_t> &idx, uint64_t *out, cudaStream_t st);
+// q opened rows and n nodes of a commitment on stream st (synchronised on
+// return); the C ABI calls run it on the context stream.
+int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q, uint64_t *rows,
+                       const uint64_t *idx, size_t n, uint8_t *nodes, cudaStream_t st);
 int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out);
 uint32_t schedule_for(bz_ctx *ctx, const Shape &s);
 int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out,

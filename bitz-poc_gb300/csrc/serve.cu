@@ -256,8 +256,8 @@ int enqueue_open(bz_server *S, Request *r, cudaStream_t st, uint8_t *h) {
     uint8_t *d_nodes = d + o_nodes;
     if (q) cudaMemcpyAsync(d_pos, r->positions.data(), q * 8, cudaMemcpyHostToDevice, st);
     if (nn) cudaMemcpyAsync(d_idx, r->node_idx.data(), nn * 8, cudaMemcpyHostToDevice, st);
-    int n = launch_gather_rows(r->commit->d_cw, s.log_lanes, d_pos, q, d_rows, st);
-    n += launch_gather_nodes(r->commit->d_tree, d_idx, nn, d_nodes, st);
+    const int n = launch_gather_open(r->commit->d_cw, s.log_lanes, d_pos, q, d_rows,
+                                     r->commit->d_tree, d_idx, nn, d_nodes, st);
     ctx->launches += (uint64_t)n;
     if (q) cudaMemcpyAsync(h, d_rows, q * row_bytes, cudaMemcpyDeviceToHost, st);
     if (nn) cudaMemcpyAsync(h + q * row_bytes, d_nodes, nn * 32, cudaMemcpyDeviceToHost, st);
