@@ -126,11 +126,10 @@ int launch_combine_shard_cvs(const uint8_t *d_cvs, uint32_t world, uint64_t n_le
 // Merkle tree over the codeword rows (leaves = positions).  d_scratch must hold
 // merkle_scratch_bytes(s).  Returns kernels launched.  With `post`, the kernel
 // that writes the root of a tree of at least two leaves also posts it to mapped
-// host memory: four 64-bit words, then the sequence number.
+// host memory, as two elements (post.cuh).
 struct RootPost {
     uint64_t *words = nullptr;  // device view of mapped host memory
-    uint32_t *seq = nullptr;    // device view of mapped host memory
-    uint32_t seq_val = 0;
+    uint32_t seq = 0;
 };
 size_t merkle_scratch_bytes(const Shape &s);
 int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d_scratch,
@@ -255,6 +254,7 @@ int launch_unpack_columns(const uint64_t *d_packed, int row_vars, int col_vars, 
 void init_ntt_kernels();
 void init_group_kernels();
 void init_fold_kernels();
+void init_merkle_kernels();
 
 // Host GF(2^128) (twiddle tables, host-side checks of transcript values).
 void hgf_mul(const uint64_t a[2], const uint64_t b[2], uint64_t out[2]);

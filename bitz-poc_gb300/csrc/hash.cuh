@@ -215,6 +215,41 @@ __device__ __forceinline__ void sha256_compress_kw(uint32_t st[8], const ShaWord
     for (int i = 0; i < 8; ++i) st[i] += v[i];
 }
 
+// The two halves of a block by two warps of a CTA, for chains too few to fill
+// the schedulers: a lone warp issues an ALU instruction every second clock, and
+// of a round's 21 the message schedule is 8.  sha_schedule stores
+// kSHA[i] + w_i for i in [FROM, TO) at kw[i * 32] (w: the sixteen words before
+// FROM, or the block when FROM is 0); sha_rounds runs those rounds on v.
+template <int FROM, int TO>
+__device__ __forceinline__ void sha_schedule(uint32_t w[16], uint32_t *kw) {
+    const uint32_t one = kOne;
+    if constexpr (FROM == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) kw[i * 32] = w[i] * one + kSHA.w[i];
+    }
+#pragma unroll 1
+    for (int r = FROM == 0 ? 16 : FROM; r < TO; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
+            const uint32_t s0 = rotr(x, 7) ^ rotr(x, 18) ^ (x >> 3);
+            const uint32_t s1 = rotr(y, 17) ^ rotr(y, 19) ^ (y >> 10);
+            w[i] = s1 * one + (s0 * one + (w[(i + 9) & 15] * one + w[i]));
+            kw[(r + i) * 32] = w[i] * one + kSHA.w[r + i];
+        }
+    }
+}
+
+template <int FROM, int TO>
+__device__ __forceinline__ void sha_rounds(uint32_t v[8], const uint32_t *kw) {
+    const uint32_t one = kOne;
+#pragma unroll 1
+    for (int r = FROM; r < TO; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) BZ_SHA_ROUND_AT(v, i, kw[(r + i) * 32]);
+    }
+}
+
 __device__ __forceinline__ uint32_t bswap32(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
 }  // namespace bz

@@ -7,18 +7,16 @@
 
 #include "bz_internal.h"
 #include "hash.cuh"
+#include "post.cuh"
 
 namespace bz {
 
-// The root o to mapped host memory, by the thread that the CTA's barrier has
-// ordered behind every write of the tree.  The host reads the words once it sees
-// the sequence number, instead of copying the root and waiting for the stream.
+// The root o to mapped host memory: the host reads it there instead of copying
+// it and waiting for the stream.
 __device__ __forceinline__ void post_root(const RootPost &p, const uint32_t o[8]) {
-    if (!p.seq) return;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        p.words[i] = (uint64_t)o[2 * i] | ((uint64_t)o[2 * i + 1] << 32);
-    asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p.seq), "r"(p.seq_val) : "memory");
+    if (!p.words) return;
+    post_element(p.words, p.seq, make_uint4(o[0], o[1], o[2], o[3]));
+    post_element(p.words + 3, p.seq, make_uint4(o[4], o[5], o[6], o[7]));
 }
 
 // ---------------------------------------------------------------------------

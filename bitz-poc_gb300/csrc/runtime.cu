@@ -269,7 +269,7 @@ int launch_commit_kernels(bz_ctx *ctx, const Shape &s, uint32_t schedule, const 
             const int n = launch_commit_pipelined(s, schedule, d_msg, d_cw, d_tree, d_tw, st, ax->s,
                                                   ax->ev, ctx->num_sms, log);
             if (n >= 0) {
-                if (post) post->seq = nullptr;
+                if (post) post->words = nullptr;
                 return n;
             }
         }
@@ -481,6 +481,7 @@ int bz_ctx_create(int device, uint64_t mem_budget_bytes, bz_ctx **out) {
     ctx->budget = mem_budget_bytes ? mem_budget_bytes : (uint64_t)(free_b * 0.9);
     init_ntt_kernels();
     init_fold_kernels();
+    init_merkle_kernels();
     cudaEventCreate(&ctx->ev0);
     cudaEventCreate(&ctx->ev1);
     if (cudaMallocHost(&ctx->h_small, 4096) != cudaSuccess) {
@@ -603,7 +604,7 @@ uint64_t bz_kernel_launches(const bz_ctx *ctx) { return ctx ? ctx->launches.load
 
 // ---- commit ---------------------------------------------------------------
 // Roots of synchronous commits: 16 slots of the mapped mailbox from byte 1024
-// (32 bytes of root, the sequence number at byte 64), taken in turn.
+// (two posted elements), taken in turn.
 constexpr size_t kRootMbox = 1024, kRootSlotBytes = 128;
 constexpr uint32_t kRootSlots = 16;
 
@@ -639,14 +640,14 @@ int bz_commit_device(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words, const b
     const size_t slot = kRootMbox + (seq % kRootSlots) * kRootSlotBytes;
     RootPost post;
     post.words = (uint64_t *)((uint8_t *)ctx->d_mbox + slot);
-    post.seq = (uint32_t *)((uint8_t *)ctx->d_mbox + slot + 64);
-    post.seq_val = seq;
+    post.seq = seq;
     int rc = commit_device_enqueue(ctx, d_msg, n_words, params, out, &post);
     if (rc) return rc;
-    if (post.seq) {
-        rc = mapped_wait(ctx, slot + 64, seq, "commit");
+    if (post.words) {
+        uint64_t r[4];
+        rc = elements_wait(ctx, slot, 2, seq, "commit", r);
         if (!rc) {
-            memcpy((*out)->root, (const uint8_t *)ctx->h_mbox + slot, 32);
+            memcpy((*out)->root, r, 32);
             (*out)->root_ready = true;
         }
     } else {

@@ -140,7 +140,7 @@ int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out);
 uint32_t schedule_for(bz_ctx *ctx, const Shape &s);
 int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out,
                      bool with_codeword = true);
-// With `post`, the commit's last kernel posts the root; post->seq is null on
+// With `post`, the commit's last kernel posts the root; post->words is null on
 // return when it does not (the two-stream pipeline).
 int enqueue_commit(bz_ctx *ctx, const Shape &s, const uint4 *d_msg, bz_commitment *c,
                    cudaStream_t st, uint32_t schedule, RootPost *post = nullptr);
