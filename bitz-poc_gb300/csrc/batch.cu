@@ -360,7 +360,8 @@ int bz_batch_plan_create(bz_ctx *ctx, size_t count, const uint64_t *const *d_msg
         if (rc == BZ_OK) {
             scratch = std::max(scratch, merkle_scratch_bytes(p->shapes[i]));
             p->msgs.push_back((const uint4 *)d_msgs[i]);
-            p->schedules.push_back(schedule_for(ctx, p->shapes[i]));
+            p->schedules.push_back(
+                schedule_for(ctx, p->shapes[i], p->n_branches > 1 && count > 1));
             bz_commitment *c = nullptr;
             rc = alloc_commitment(ctx, p->shapes[i], &c);
             p->commits.push_back(c);

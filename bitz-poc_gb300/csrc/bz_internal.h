@@ -71,7 +71,7 @@ enum : uint32_t {
     SCHED_GROUP = 0x20000,        // the deepest layers as group passes (ntt_group.cuh)
     SCHED_SHORT_CTAS = 0x200000,  // table passes in 16 CTAs per SM instead of one long one
 };
-uint32_t default_schedule(const Shape &s);
+uint32_t default_schedule(const Shape &s, bool shared = false);
 
 // Twiddle heap for AdditiveNttF128::standard(ell): tw[(1 << l) + b] =
 // twiddle(l, b) for 0 <= l < ell, 0 <= b < 2^l (entry 0 unused).

@@ -181,12 +181,12 @@ int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out) {
     return BZ_OK;
 }
 
-uint32_t schedule_for(bz_ctx *ctx, const Shape &s) {
+uint32_t schedule_for(bz_ctx *ctx, const Shape &s, bool shared) {
     std::lock_guard<std::mutex> g(ctx->sched_mu);
     const uint64_t key = shape_key(s);
     auto it = ctx->schedules.find(key);
     if (it != ctx->schedules.end()) return it->second;
-    return default_schedule(s);
+    return default_schedule(s, shared);
 }
 
 // Every live commitment of every context: bz_commitment_free checks a handle

@@ -137,7 +137,7 @@ int commitment_proof_nodes(bz_commitment *c, const uint64_t *positions, size_t q
 int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q, uint64_t *rows,
                        const uint64_t *idx, size_t n, uint8_t *nodes, cudaStream_t st);
 int get_twiddles(bz_ctx *ctx, int ell, const uint4 **out);
-uint32_t schedule_for(bz_ctx *ctx, const Shape &s);
+uint32_t schedule_for(bz_ctx *ctx, const Shape &s, bool shared = false);
 int alloc_commitment(bz_ctx *ctx, const Shape &s, bz_commitment **out,
                      bool with_codeword = true);
 // With `post`, the commit's last kernel posts the root; post->words is null on

@@ -400,7 +400,7 @@ int start_commit(bz_server *S, Request *r, int slot) {
     // schedules), which would bypass the slot's priority.  A large request's
     // table passes run as short CTAs when small requests have priority, so
     // their kernels get SMs within a fraction of a pass.
-    uint32_t schedule = default_schedule(s);
+    uint32_t schedule = default_schedule(s, true);
 #if BZ_SERVE_SHORT_CTAS
     if (S->small_log >= 0 && large) schedule |= SCHED_SHORT_CTAS;
 #endif
