@@ -68,10 +68,11 @@ SMEM_BYTES_PER_CLK_PER_SM = 128
 # captures of the same kernels on GB300 (dram__bytes_read.sum +
 # dram__bytes_write.sum), with the profile they come from.
 NCU_TRAFFIC_PER_CW_BYTE = {
-    "ntt_pass8_first": (1.424, "profiles/launches_commit_2e24.md"),
+    "ntt_pass8_first": (1.951, "profiles/launches_commit_2e24.md"),
     "ntt_pass8": (1.941, "profiles/launches_commit_2e24.md (both in-place byte-table passes)"),
     "ntt_pass8_nw": (1.940, "profiles/launches_commit_2e24.md"),
-    "b3_leaves_chunked": (1.057, "profiles/launches_commit_2e24.md"),
+    "ntt_group8": (1.940, "profiles/launches_commit_2e24.md"),
+    "b3_leaves_chunked": (1.005, "profiles/launches_commit_2e24.md"),
     # radix-4 schedules sweep the codeword the same way: one read and one
     # write in place, the first pass reading the message instead
     "ntt_table_pass2_first": (1.424, "profiles/launches_commit_2e24.md (a first sweep)"),
@@ -91,8 +92,8 @@ def table_pass_lookup_bytes(kernel: str, layer: int, log_positions_lanes: int) -
     twiddle (the span of no evaluation is 0), so its quads skip the t_o and
     t_a products and its pairs skip theirs."""
     n = 1 << log_positions_lanes
-    if kernel.endswith("_nw"):
-        return None   # compact 4-byte tables for narrow twiddles: not this model
+    if kernel.endswith("_nw") or kernel.startswith("ntt_group"):
+        return None   # compact 4-byte tables, or products grouped over layers: not this model
     if kernel.startswith("ntt_pass8"):
         # radix-8: 12 products per octet; block 0's seven zero twiddles skip
         # 4 + 2 + 1 of them in the first super-block

@@ -142,9 +142,9 @@ int launch_gather_open(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, 
                        uint8_t *d_nodes, cudaStream_t st);
 
 // Folds.  d_partials holds fold_partials_bytes(n) bytes.  With `post`, the
-// last CTA of the fold (or message) kernel reduces the partials itself and
-// posts {u0, u2} to mapped host memory, then the sequence number (no finish
-// kernel, no copy); without it a finish kernel writes d_msg_out.
+// fold (or message) kernel posts {u0, u2} to mapped host memory as tagged
+// elements (no finish kernel, no copy): fold_posts or round_msg_posts parts
+// whose sum it is.  Without it a finish kernel writes d_msg_out.
 struct MsgPost {
     unsigned int *ticket;  // device counter, 0 between launches
     uint64_t *words;       // device view of mapped host memory (6 tagged words a post)
