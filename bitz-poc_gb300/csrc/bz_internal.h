@@ -147,12 +147,12 @@ int launch_gather_open(const uint4 *d_cw, int log_lanes, const uint64_t *d_pos, 
 // whose sum it is.  Without it a finish kernel writes d_msg_out.
 struct MsgPost {
     unsigned int *ticket;  // device counter, 0 between launches
-    uint64_t *words;       // device view of mapped host memory (6 tagged words a post)
+    uint64_t *words;       // device view of mapped host memory (8 tagged words a post)
     uint32_t seq_val;
 };
 // Elements posted to mapped host memory (post.cuh).
 struct ElementPost {
-    uint64_t *words;  // device view: 3 tagged words an element
+    uint64_t *words;  // device view: 4 tagged words an element
     uint32_t seq;
 };
 // Posts of a message kernel of `grid` CTAs: one by each CTA, whose sum is the
@@ -160,12 +160,12 @@ struct ElementPost {
 constexpr int kMsgPosts = 16;
 __host__ __device__ inline int msg_posts(int grid) { return grid <= kMsgPosts ? grid : 1; }
 // Challenge gate of a fold launched ahead of its challenge: the host writes r
-// to mapped memory as three words of 44 bits tagged with the gate's number
+// to mapped memory as four words of 32 bits below the gate's number
 // (or the first word tagged seq | kGateCancel to cancel).  The kernel waits at most limit_ns, then sets bit 0 of *err.  The
 // host posts r within microseconds; the limit only bounds a gate that nothing
 // opens (an error path, or a tool that runs each launch to completion before
 // returning), and the prover then runs the round again unarmed.
-constexpr uint32_t kGateCancel = 0x80000u;  // of a 20-bit tag
+constexpr uint32_t kGateCancel = 0x80000000u;
 constexpr uint64_t kGateLimitNs = 100000000ull;  // 100 ms
 struct RGate {
     const uint64_t *words = nullptr;  // device view of mapped host memory
@@ -207,7 +207,7 @@ int launch_chacha(uint64_t seed, uint64_t first_word, uint4 *d_out, size_t n_wor
 // (sum_end, sum_inf) to the mapped mailbox as the sumcheck rounds do.
 // A small round's fold writes d_nl, d_nr (2 h entries each) and not in place,
 // its rho may come through `gate`, and the round of h = 1 posts the four
-// entries it leaves to d_tail (mapped, 12 tagged words).
+// entries it leaves to d_tail (mapped, 16 tagged words).
 int launch_gkr_product(const uint4 *d_in, size_t half, uint4 *d_out, cudaStream_t st,
                        int num_sms);
 bool gkr_small_round(size_t h);

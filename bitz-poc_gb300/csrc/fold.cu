@@ -92,7 +92,7 @@ struct MsgMailbox {
 __device__ __forceinline__ void post_pair(uint64_t word, const MsgMailbox &mb) {
     const uint4 v = reduce_pair(word);
     const int ln = threadIdx.x & 31;
-    if (ln < 2) post_element(mb.words + 3 * ln, mb.seq_val, v);
+    if (ln < 2) post_element(mb.words + 4 * ln, mb.seq_val, v);
 }
 
 // XOR of the partials (8 words each) of n CTAs, by all threads; lanes of warp
@@ -120,7 +120,7 @@ __device__ uint64_t partials_xor(const uint64_t *partials, int n) {
 // all, posts and resets the ticket for the next launch.
 __device__ __forceinline__ void msg_out(uint64_t word, uint64_t *partials, MsgMailbox mb) {
     if (mb.ticket && msg_posts(gridDim.x) == (int)gridDim.x) {
-        mb.words += 6 * blockIdx.x;
+        mb.words += 8 * blockIdx.x;
         if (threadIdx.x < 32) post_pair(word, mb);
         return;
     }
@@ -164,7 +164,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
-// Warp 0 of each CTA polls the gate's three words, sleeping between polls,
+// Warp 0 of each CTA polls the gate's four words, sleeping between polls,
 // until all carry the round's number (open: together they hold r, as
 // post_element lays it out, so one access brings both), the first carries the
 // number with its top bit set (cancelled) or the time limit passes (bit 0 of
@@ -179,9 +179,9 @@ __device__ bool gate_wait(const RGate &g, uint4 &r) {
         int st = 0;
         uint64_t v = 0;
         for (;;) {
-            if (ln < 3) v = ld_relaxed_sys(g.words + ln);
-            const uint32_t tag = (uint32_t)(v >> 44);
-            if (__all_sync(0xffffffffu, ln >= 3 || tag == g.seq)) {
+            if (ln < 4) v = ld_relaxed_sys(g.words + ln);
+            const uint32_t tag = (uint32_t)(v >> 32);
+            if (__all_sync(0xffffffffu, ln >= 4 || tag == g.seq)) {
                 st = 1;
                 break;
             }
@@ -192,12 +192,12 @@ __device__ bool gate_wait(const RGate &g, uint4 &r) {
             }
             __nanosleep(128);
         }
-        const uint64_t m = ((uint64_t)1 << 44) - 1;
-        const uint64_t v0 = __shfl_sync(0xffffffffu, v, 0) & m;
-        const uint64_t v1 = __shfl_sync(0xffffffffu, v, 1) & m;
-        const uint64_t v2 = __shfl_sync(0xffffffffu, v, 2) & m;
+        const uint32_t x = __shfl_sync(0xffffffffu, (uint32_t)v, 0);
+        const uint32_t y = __shfl_sync(0xffffffffu, (uint32_t)v, 1);
+        const uint32_t z = __shfl_sync(0xffffffffu, (uint32_t)v, 2);
+        const uint32_t w = __shfl_sync(0xffffffffu, (uint32_t)v, 3);
         if (ln == 0) {
-            rs = mk(v0 | (v1 << 44), (v1 >> 20) | (v2 << 24));
+            rs = make_uint4(x, y, z, w);
             open = st;
         }
     }
@@ -354,7 +354,7 @@ struct CoopRound {
     uint4 *na, *nb;
     const uint4 *w;
     uint4 *w_next;
-    uint64_t *tail;  // mapped: the round's four entries, 3 tagged words each
+    uint64_t *tail;  // mapped: the round's four entries, 4 tagged words each
     uint64_t h;
     int per;  // slots a CTA takes at a time
     uint4 r;
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kCoopThreads) coop_round_kernel(
             return e[GKR && a.send_one];
         };
         if constexpr (GKR) {
-            if (a.tail && tid < 4) post_element(a.tail + 3 * tid, a.mb.seq_val, base);
+            if (a.tail && tid < 4) post_element(a.tail + 4 * tid, a.mb.seq_val, base);
             coop_each<2>(2 * ns, [&](int p, bool) {
                 prod[q][p] = clmul32(part.of(operand(p, 0)), part.of(wgt[p >> 1]));
             });
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(128) sv_finish_kernel(const uint4 *partials, i
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0)
-        post_element(post.words + 3 * blockIdx.x, post.seq,
+        post_element(post.words + 4 * blockIdx.x, post.seq,
                      gf_add(gf_add(red[0], red[1]), gf_add(red[2], red[3])));
 }
 
@@ -881,7 +881,7 @@ int launch_sv_fold(const uint4 *d_packed, const uint4 *d_eq, size_t n, uint4 *d_
 __global__ void post_elements_kernel(const uint4 *in, int n, ElementPost post) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) post_element(post.words + 3 * i, post.seq, in[i]);
+    if (i < n) post_element(post.words + 4 * i, post.seq, in[i]);
 }
 
 int launch_post_elements(const uint4 *d_in, int n, const ElementPost &post, cudaStream_t st) {

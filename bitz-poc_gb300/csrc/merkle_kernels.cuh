@@ -16,7 +16,7 @@ namespace bz {
 __device__ __forceinline__ void post_root(const RootPost &p, const uint32_t o[8]) {
     if (!p.words) return;
     post_element(p.words, p.seq, make_uint4(o[0], o[1], o[2], o[3]));
-    post_element(p.words + 3, p.seq, make_uint4(o[4], o[5], o[6], o[7]));
+    post_element(p.words + 4, p.seq, make_uint4(o[4], o[5], o[6], o[7]));
 }
 
 // ---------------------------------------------------------------------------

@@ -893,11 +893,11 @@ static bool pow2(size_t n) { return n && !(n & (n - 1)); }
 
 namespace bz {
 
-// The messages' posts in the mapped mailbox (kMsgPosts of 48 bytes) and the
-// element posts (kPostElements of 24 bytes).
+// The messages' posts in the mapped mailbox (kMsgPosts of 64 bytes) and the
+// element posts (kPostElements of 32 bytes).
 constexpr size_t kMsgOffset = 3072, kElementsOffset = 4096;
-static_assert(kMsgOffset + 48 * kMsgPosts <= kElementsOffset &&
-              kElementsOffset + 24 * kPostElements <= kMboxBytes);
+static_assert(kMsgOffset + 64 * kMsgPosts <= kElementsOffset &&
+              kElementsOffset + 32 * kPostElements <= kMboxBytes);
 
 // Mailbox post for the next message kernel on the context stream.
 static MsgPost next_post(bz_ctx *ctx) {
@@ -940,23 +940,18 @@ int mapped_wait(bz_ctx *ctx, size_t offset, uint32_t seq, const char *what) {
     return spin_wait(ctx, what, [&] { return *sp == seq; });
 }
 
-// An element is three words of 44 bits below the low 20 bits of the message's
-// number; each word is one access, so those that carry the number are final.
+// An element is four words of 32 bits below the post's number; each word is one
+// access, so those that carry the number are final.
 int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
                   uint64_t *out) {
     const uint64_t *hp = (const uint64_t *)((uint8_t *)ctx->h_mbox + offset);
-    const uint64_t tag = (uint64_t)seq << 44, m = ((uint64_t)1 << 44) - 1;
-    int at = 0;  // words seen with the tag
-    uint64_t w[3];
+    int at = 0;  // words seen with the number
     return spin_wait(ctx, what, [&] {
-        for (; at < 3 * n; ++at) {
+        for (; at < 4 * n; ++at) {
             const uint64_t v = __atomic_load_n(hp + at, __ATOMIC_RELAXED);
-            if ((v & ~m) != tag) return false;
-            w[at % 3] = v & m;
-            if (at % 3 == 2) {
-                out[2 * (at / 3)] = w[0] | (w[1] << 44);
-                out[2 * (at / 3) + 1] = (w[1] >> 20) | (w[2] << 24);
-            }
+            if ((uint32_t)(v >> 32) != seq) return false;
+            if (at & 1) out[at / 2] |= v << 32;
+            else out[at / 2] = (uint32_t)v;
         }
         return true;
     });
@@ -1007,7 +1002,7 @@ int round_msg_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size
     return BZ_OK;
 }
 
-// The gate: three tagged words at byte 128 of the mapped mailbox; the kernel's
+// The gate: four tagged words at byte 128 of the mapped mailbox; the kernel's
 // time-out record at byte 832 of the small device buffer.
 static uint64_t *gate_host(bz_ctx *ctx) { return (uint64_t *)((uint8_t *)ctx->h_mbox + 128); }
 
@@ -1063,10 +1058,9 @@ int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, ui
 
 void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]) {
     uint64_t *g = gate_host(ctx);
-    const uint64_t tag = (uint64_t)a->gate_seq << 44, m = ((uint64_t)1 << 44) - 1;
-    __atomic_store_n(&g[0], (r[0] & m) | tag, __ATOMIC_RELAXED);
-    __atomic_store_n(&g[1], (((r[0] >> 44) | (r[1] << 20)) & m) | tag, __ATOMIC_RELAXED);
-    __atomic_store_n(&g[2], (r[1] >> 24) | tag, __ATOMIC_RELAXED);
+    const uint64_t tag = (uint64_t)a->gate_seq << 32;
+    for (int i = 0; i < 4; ++i)
+        __atomic_store_n(&g[i], tag | (uint32_t)(r[i / 2] >> (32 * (i & 1))), __ATOMIC_RELAXED);
     a->live = false;
 }
 
@@ -1074,7 +1068,7 @@ void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]) {
 // stream is drained so that nothing armed outlives the call.
 int fold_cancel(bz_ctx *ctx, ArmedFold *a) {
     if (!a->live) return BZ_OK;
-    __atomic_store_n(gate_host(ctx), (uint64_t)(a->gate_seq | kGateCancel) << 44,
+    __atomic_store_n(gate_host(ctx), (uint64_t)(a->gate_seq | kGateCancel) << 32,
                      __ATOMIC_RELAXED);
     a->live = false;
     BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
