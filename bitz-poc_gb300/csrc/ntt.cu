@@ -138,12 +138,13 @@ int twiddle_bits(int ell, int layer) {
 //
 // `shared`: the commit runs beside others (a plan's branches, a server's
 // slots), so what counts is the SM time of its passes, and up to 2^18 codeword
-// elements the group passes' tables (96 KB a CTA) cost more of it than the
-// layers they save.  Eight commits on four branches, with and without them: 2^17
-// elements of 64 lanes 234 and 169 us, 2^18 of 256 lanes 257 and 231, 2^19 of
-// 128 lanes 354 and 381, 2^20 577 and 645.
+// elements, 2^19 from 256 lanes, the group passes' tables (96 KB a CTA) cost
+// more of it than the layers they save.  Eight commits on four branches, with
+// and without them: 2^17 elements of 64 lanes 234 and 169 us, 2^18 of 256 lanes
+// 257 and 231, 2^19 of 128 lanes 354 and 381, of 256 lanes 330 and 331 (among
+// smaller ones 293 and 268), 2^20 577 and 645.
 uint32_t default_schedule(const Shape &s, bool shared) {
-    const bool small = s.cw_words() <= ((uint64_t)1 << 18);
+    const bool small = s.cw_words() <= (uint64_t)1 << (s.log_lanes >= 8 ? 19 : 18);
     const uint32_t group = group8_ok(s) && !(shared && small) ? SCHED_GROUP : 0u;
     if (s.log_lanes >= 9 && s.k_code() - s.log_inv_rate >= 3) return SCHED_RADIX8 | group;
     if (s.log_lanes >= 9) return SCHED_PREFETCH | SCHED_NARROW;

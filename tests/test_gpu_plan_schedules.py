@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("count,branches", [(1, 4), (3, 1), (5, 4)])
-@pytest.mark.parametrize("lm,r,lb", [(15, 2, 6), (16, 2, 5), (17, 1, 4), (17, 2, 7)])
+@pytest.mark.parametrize("lm,r,lb", [(15, 2, 6), (16, 2, 5), (17, 1, 4), (17, 2, 7),
+                                     (17, 2, 8), (18, 2, 8)])
 def test_plan_equals_oracle(oracle, ctx, count, branches, lm, r, lb):
     from bitz_gb300 import BatchPlan, DeviceArray, PcsParams
 
