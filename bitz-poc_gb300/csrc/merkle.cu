@@ -22,14 +22,15 @@
 namespace bz {
 
 // ---- kernels around the bodies of merkle_kernels.cuh -----------------------
+template <bool LEVELS>
 __global__ void __launch_bounds__(256) b3_leaves_chunked(const uint4 *cw, uint64_t n_chunks,
                                                          uint32_t *tree_leaves, int log_c,
                                                          uint64_t chunk0, int levels,
                                                          uint64_t n_leaves) {
     __shared__ uint32_t cvs[256][9];  // padded rows
     chain_wait();
-    b3_leaves_chunked_body(cw, n_chunks, tree_leaves, log_c, chunk0,
-                           (uint64_t)blockIdx.x * blockDim.x, cvs, levels, n_leaves);
+    b3_leaves_chunked_body<LEVELS>(cw, n_chunks, tree_leaves, log_c, chunk0,
+                                   (uint64_t)blockIdx.x * blockDim.x, cvs, levels, n_leaves);
 }
 
 __global__ void b3_leaves_small(const uint4 *cw, int log_lanes, uint64_t n_leaves,
@@ -318,8 +319,8 @@ int launch_leaves_range(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint
             const int log_c = s.log_lanes - 6;
             const uint64_t n_chunks = n << log_c;
             const unsigned t = leaf_threads(n_chunks, log_c, num_sms);
-            launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, cw,
-                           n_chunks, leaves, log_c, s.chunk0, 0, n);
+            launch_chained(b3_leaves_chunked<false>, (unsigned)((n_chunks + t - 1) / t), t, 0, st,
+                           cw, n_chunks, leaves, log_c, s.chunk0, 0, n);
         }
     } else {
         launch_chained(sha_leaves, (unsigned)((n + 127) / 128), 128, 0, st, cw, s.log_lanes, n,
@@ -407,8 +408,8 @@ int launch_merkle(const Shape &s, const uint4 *d_cw, uint8_t *d_tree, uint8_t *d
             int most = 0;
             while (n_chunks >= t && (t >> log_c) >> (most + 1)) ++most;
             from = post ? leaf_levels(n_leaves, most) : 0;
-            launch_chained(b3_leaves_chunked, (unsigned)((n_chunks + t - 1) / t), t, 0, st, d_cw,
-                           n_chunks, tree, log_c, s.chunk0, from, n_leaves);
+            launch_chained(from ? b3_leaves_chunked<true> : b3_leaves_chunked<false>,
+                           (unsigned)((n_chunks + t - 1) / t), t, 0, st, d_cw, n_chunks, tree, log_c, s.chunk0, from, n_leaves);
             mark("b3_leaves_chunked");
             ++launches;
         } else {

@@ -30,9 +30,11 @@ __device__ __forceinline__ void post_root(const RootPost &p, const uint32_t o[8]
 // Body: the CTA's blockDim.x chunks from chunk_base (a multiple of blockDim.x,
 // blockDim.x a multiple of C); cvs holds blockDim.x padded rows of 9 words.
 //
-// levels > 0 (at most log2 of the CTA's leaves): the CTA goes on merging its
-// leaves into that many levels of the tree above them (n_leaves leaves), whose
-// parents are the same PARENT merge as those inside a leaf.
+// LEVELS: the CTA goes on merging its leaves into `levels` levels of the tree
+// above them (n_leaves leaves; at most log2 of the CTA's), whose parents are the
+// same PARENT merge as those inside a leaf.  A kernel of its own: one loop for
+// both cost the leaves alone 1 to 1.5 us.
+template <bool LEVELS = false>
 __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t n_chunks,
                                                        uint32_t *tree_leaves, int log_c,
                                                        uint64_t chunk0, uint64_t chunk_base,
@@ -63,21 +65,9 @@ __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t
 #pragma unroll
     for (int i = 0; i < 8; ++i) cvs[threadIdx.x][i] = cv[i];
     __syncthreads();
-    // Step s merges nodes (2j, 2j+1): inside the leaf below log_c, then the
-    // levels above.  The level of step s is stored when it is one of the tree.
-    uint64_t off = 0, cnt = n_leaves;  // the tree level's first node and size
-    for (int s = 0;; ++s) {
-        const int t = threadIdx.x;
-        if (s >= log_c) {
-            if ((t & ((1 << s) - 1)) == 0 && chunk < n_chunks) {
-                const uint64_t node = off + (chunk >> s);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) tree_leaves[node * 8 + i] = cvs[t][i];
-            }
-            off += cnt;
-            cnt >>= 1;
-        }
-        if (s == log_c + levels) break;
+    // Step s merges nodes (2j, 2j+1) of the CTA.
+    const int t = threadIdx.x;
+    auto merge = [&](int s) {
         const int stride = 1 << s;
         if ((t & ((stride << 1) - 1)) == 0 && t + stride < (int)blockDim.x) {
             uint32_t out[8];
@@ -86,6 +76,28 @@ __device__ __forceinline__ void b3_leaves_chunked_body(const uint4 *cw, uint64_t
             for (int i = 0; i < 8; ++i) cvs[t][i] = out[i];
         }
         __syncthreads();
+    };
+    auto store = [&](int s, uint64_t off) {
+        if ((t & ((1 << s) - 1)) == 0 && chunk < n_chunks) {
+            const uint64_t node = off + (chunk >> s);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tree_leaves[node * 8 + i] = cvs[t][i];
+        }
+    };
+    if constexpr (!LEVELS) {
+        for (int s = 0; s < log_c; ++s) merge(s);
+        store(log_c, 0);
+    } else {
+        uint64_t off = 0, cnt = n_leaves;  // the tree level's first node and size
+        for (int s = 0;; ++s) {
+            if (s >= log_c) {
+                store(s, off);
+                off += cnt;
+                cnt >>= 1;
+            }
+            if (s == log_c + levels) break;
+            merge(s);
+        }
     }
 }
 
