@@ -149,6 +149,10 @@ struct MsgPost {
     unsigned int *ticket;  // device counter, 0 between launches
     uint64_t *words;       // device view of mapped host memory (8 tagged words a post)
     uint32_t seq_val;
+    // 1: the post ends a synchronous call, and any stream may read the folded
+    // arrays next (post_release).  0 in the provers' own rounds, whose arrays
+    // only the context stream reads.
+    uint32_t release;
 };
 // Elements posted to mapped host memory (post.cuh).
 struct ElementPost {

@@ -86,12 +86,15 @@ struct MsgMailbox {
     unsigned int *ticket = nullptr;  // device counter, 0 between launches
     uint64_t *words = nullptr;       // mapped host memory: u0, u2
     uint32_t seq_val = 0;
+    uint32_t release = 0;            // release the folded arrays before the post
 };
 
-// Lanes 0 and 1 of the calling warp post u0 and u2.
+// Lanes 0 and 1 of the calling warp post u0 and u2, behind a barrier that
+// follows the CTA's stores.
 __device__ __forceinline__ void post_pair(uint64_t word, const MsgMailbox &mb) {
     const uint4 v = reduce_pair(word);
     const int ln = threadIdx.x & 31;
+    if (mb.release) post_release();
     if (ln < 2) post_element(mb.words + 4 * ln, mb.seq_val, v);
 }
 
@@ -520,7 +523,7 @@ int launch_fold_and_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint4 r, u
     const uint64_t half = n / 2;
     const int grid = fold_grid(n, num_sms);
     MsgMailbox mb;
-    if (post) mb = {post->ticket, post->words, post->seq_val};
+    if (post) mb = {post->ticket, post->words, post->seq_val, post->release};
     if (n / 4 <= kCoopFoldSlots) {
         const CoopRound a = {d_f, d_b, d_nf, d_nb, nullptr, nullptr, nullptr,
                              std::max<uint64_t>(n / 4, 1), coop_per(n / 4), r, 0, n == 2, d_partials, mb};
@@ -547,7 +550,7 @@ int launch_round_msg(const uint4 *d_f, const uint4 *d_b, size_t n, uint64_t *d_p
     const uint64_t pairs = n / 2;
     const int grid = round_grid(pairs, kCoopMsgSlots, num_sms);
     MsgMailbox mb;
-    if (post) mb = {post->ticket, post->words, post->seq_val};
+    if (post) mb = {post->ticket, post->words, post->seq_val, post->release};
     if (pairs <= kCoopMsgSlots) {
         const CoopRound a = {d_f, d_b, nullptr, nullptr, nullptr, nullptr, nullptr, pairs,
                              coop_per(pairs), make_uint4(0, 0, 0, 0), 0, 0, d_partials, mb};
@@ -1088,7 +1091,7 @@ int launch_gkr_round(uint4 *d_l, uint4 *d_r, uint4 *d_nl, uint4 *d_nr, const uin
                      bool fold, uint4 rho, bool send_one, uint4 *d_w_next, uint64_t *d_partials,
                      cudaStream_t st, int num_sms, const MsgPost &post, uint64_t *d_tail,
                      const RGate *gate) {
-    const MsgMailbox mb = {post.ticket, post.words, post.seq_val};
+    const MsgMailbox mb = {post.ticket, post.words, post.seq_val, post.release};
     const int grid = gkr_round_grid(h, num_sms);
     if (gkr_small_round(h)) {
         const CoopRound a = {d_l, d_r, d_nl, d_nr, d_w, d_w_next, h == 1 ? d_tail : nullptr, h,

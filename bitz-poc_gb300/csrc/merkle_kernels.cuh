@@ -12,9 +12,11 @@
 namespace bz {
 
 // The root o to mapped host memory: the host reads it there instead of copying
-// it and waiting for the stream.
+// it and waiting for the stream.  Called behind a barrier that follows the CTA's
+// tree stores, so the tree and the codeword are released before the root.
 __device__ __forceinline__ void post_root(const RootPost &p, const uint32_t o[8]) {
     if (!p.words) return;
+    post_release();
     post_element(p.words, p.seq, make_uint4(o[0], o[1], o[2], o[3]));
     post_element(p.words + 4, p.seq, make_uint4(o[4], o[5], o[6], o[7]));
 }

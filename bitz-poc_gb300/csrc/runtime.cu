@@ -906,6 +906,7 @@ static MsgPost next_post(bz_ctx *ctx) {
     p.words = (uint64_t *)((uint8_t *)ctx->d_mbox + kMsgOffset);
     if (++ctx->mbox_seq == 0) ++ctx->mbox_seq;  // 0 is the initial mailbox value
     p.seq_val = ctx->mbox_seq;
+    p.release = 0;
     return p;
 }
 
@@ -977,10 +978,12 @@ int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2
 }
 
 int fold_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
-                const uint64_t r[2], uint64_t *d_nf, uint64_t *d_nb, uint32_t *msg_seq) {
+                const uint64_t r[2], uint64_t *d_nf, uint64_t *d_nb, uint32_t *msg_seq,
+                bool release) {
     int rc = ensure_scratch(ctx, fold_partials_bytes(n));
     if (rc) return rc;
-    const MsgPost post = next_post(ctx);
+    MsgPost post = next_post(ctx);
+    post.release = release;
     ctx->launches += launch_fold_and_msg((const uint4 *)d_f, (const uint4 *)d_b, n, to_u4(r),
                                          (uint4 *)d_nf, (uint4 *)d_nb, (uint64_t *)ctx->scratch,
                                          nullptr, ctx->stream, ctx->num_sms, &post);
@@ -1034,12 +1037,13 @@ RGate next_gate(bz_ctx *ctx, uint64_t limit_ns) {
 }
 
 int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, uint64_t *d_nf,
-             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns) {
+             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns, bool release) {
     if (a->live) return set_msg(ctx, BZ_ERR_STATE, "a fold is already armed");
     int rc = ensure_scratch(ctx, fold_partials_bytes(n));
     if (rc) return rc;
     const RGate g = next_gate(ctx, limit_ns);
-    const MsgPost post = next_post(ctx);
+    MsgPost post = next_post(ctx);
+    post.release = release;
     ctx->launches += launch_fold_and_msg((const uint4 *)d_f, (const uint4 *)d_b, n,
                                          make_uint4(0, 0, 0, 0), (uint4 *)d_nf, (uint4 *)d_nb,
                                          (uint64_t *)ctx->scratch, nullptr, ctx->stream,
@@ -1085,7 +1089,7 @@ int bz_fold_and_msg_lsb(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, s
     if (!ctx || !d_f || !d_b || !r || !d_nf || !d_nb) return BZ_ERR_ARG;
     if (!pow2(n) || n < 2) return set_msg(ctx, BZ_ERR_SHAPE, "n must be a power of two >= 2");
     uint32_t seq = 0;
-    int rc = fold_launch(ctx, d_f, d_b, n, r, d_nf, d_nb, &seq);
+    int rc = fold_launch(ctx, d_f, d_b, n, r, d_nf, d_nb, &seq, true);
     if (rc) return rc;
     return msg_wait(ctx, seq, fold_posts(n, ctx->num_sms), u0, u2);
 }
@@ -1097,7 +1101,7 @@ int bz_fold_gate_check(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, si
         return BZ_ERR_ARG;
     if (!pow2(n) || n < 2) return set_msg(ctx, BZ_ERR_SHAPE, "n must be a power of two >= 2");
     ArmedFold a;
-    int rc = fold_arm(ctx, d_f, d_b, n, d_nf, d_nb, &a, limit_ns ? limit_ns : kGateLimitNs);
+    int rc = fold_arm(ctx, d_f, d_b, n, d_nf, d_nb, &a, limit_ns ? limit_ns : kGateLimitNs, true);
     if (rc) return rc;
     if (mode == 0) {
         fold_open(ctx, &a, r);

@@ -161,6 +161,8 @@ int launch_commit_kernels(bz_ctx *ctx, const Shape &s, uint32_t schedule, const 
 // transcript work; fold_open posts the challenge, fold_cancel withdraws it.
 // Between fold_arm and fold_open/fold_cancel the host must not wait on the
 // context stream (the armed kernel would hold it until its time limit).
+// `release`: the message ends a synchronous call, and any stream may read the
+// folded arrays next.
 struct ArmedFold {
     uint32_t gate_seq = 0;
     uint32_t msg_seq = 0;
@@ -170,10 +172,12 @@ struct ArmedFold {
     bool live = false;
 };
 int fold_launch(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n,
-                const uint64_t r[2], uint64_t *d_nf, uint64_t *d_nb, uint32_t *msg_seq);
+                const uint64_t r[2], uint64_t *d_nf, uint64_t *d_nb, uint32_t *msg_seq,
+                bool release = false);
 bool fold_armable(const bz_ctx *ctx, size_t n);
 int fold_arm(bz_ctx *ctx, const uint64_t *d_f, const uint64_t *d_b, size_t n, uint64_t *d_nf,
-             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns = kGateLimitNs);
+             uint64_t *d_nb, ArmedFold *a, uint64_t limit_ns = kGateLimitNs,
+             bool release = false);
 // The gate of the next armed launch (its number is what fold_open posts).
 RGate next_gate(bz_ctx *ctx, uint64_t limit_ns);
 void fold_open(bz_ctx *ctx, ArmedFold *a, const uint64_t r[2]);
