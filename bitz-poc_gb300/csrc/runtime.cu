@@ -604,7 +604,8 @@ uint64_t bz_kernel_launches(const bz_ctx *ctx) { return ctx ? ctx->launches.load
 
 // ---- commit ---------------------------------------------------------------
 // Roots of synchronous commits: 16 slots of the mapped mailbox from byte 1024
-// (two posted elements), taken in turn.
+// (two posted elements), taken in turn.  The post only saves the copy and the
+// synchronisation: whatever becomes of it, the tree holds the root.
 constexpr size_t kRootMbox = 1024, kRootSlotBytes = 128;
 constexpr uint32_t kRootSlots = 16;
 
@@ -633,6 +634,23 @@ int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
     return commit_device_enqueue(ctx, d_msg, n_words, params, out, nullptr);
 }
 
+// The posted root; or the tree's, when other threads' commits took the slot
+// before this one read it, or the work queued before the commit outlasts the
+// spin.
+static int root_wait(bz_ctx *ctx, size_t slot, uint32_t seq, bz_commitment *c) {
+    uint64_t r[4];
+    bool taken = false;
+    if (elements_wait(ctx, slot, 2, seq, "commit", r, &taken) == BZ_OK && !taken) {
+        memcpy(c->root, r, 32);
+    } else {
+        const uint8_t *src = c->d_tree + (c->shape.tree_nodes() - 1) * 32;
+        BZ_CUDA(ctx, cudaMemcpyAsync(c->root, src, 32, cudaMemcpyDeviceToHost, ctx->stream));
+        BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    c->root_ready = true;
+    return BZ_OK;
+}
+
 int bz_commit_device(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words, const bz_params *params,
                      bz_commitment **out, uint8_t root[32]) {
     if (!ctx) return BZ_ERR_ARG;
@@ -643,16 +661,7 @@ int bz_commit_device(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words, const b
     post.seq = seq;
     int rc = commit_device_enqueue(ctx, d_msg, n_words, params, out, &post);
     if (rc) return rc;
-    if (post.words) {
-        uint64_t r[4];
-        rc = elements_wait(ctx, slot, 2, seq, "commit", r);
-        if (!rc) {
-            memcpy((*out)->root, r, 32);
-            (*out)->root_ready = true;
-        }
-    } else {
-        rc = fetch_root(*out);
-    }
+    rc = post.words ? root_wait(ctx, slot, seq, *out) : fetch_root(*out);
     if (rc) {
         bz_commitment_free(*out);
         *out = nullptr;
@@ -942,15 +951,17 @@ int mapped_wait(bz_ctx *ctx, size_t offset, uint32_t seq, const char *what) {
 }
 
 // An element is four words of 32 bits below the post's number; each word is one
-// access, so those that carry the number are final.
+// access, so those that carry the number are final.  A later number ends the
+// wait with *taken set, where the caller asks for that.
 int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
-                  uint64_t *out) {
+                  uint64_t *out, bool *taken) {
     const uint64_t *hp = (const uint64_t *)((uint8_t *)ctx->h_mbox + offset);
     int at = 0;  // words seen with the number
     return spin_wait(ctx, what, [&] {
         for (; at < 4 * n; ++at) {
             const uint64_t v = __atomic_load_n(hp + at, __ATOMIC_RELAXED);
-            if ((uint32_t)(v >> 32) != seq) return false;
+            const uint32_t tag = (uint32_t)(v >> 32);
+            if (tag != seq) return taken && (*taken = (int32_t)(tag - seq) > 0);
             if (at & 1) out[at / 2] |= v << 32;
             else out[at / 2] = (uint32_t)v;
         }

@@ -189,9 +189,10 @@ bool gate_gave_up(bz_ctx *ctx);
 // `posts` as the launch's fold_posts / round_msg_posts / gkr_round_posts
 int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2]);
 // Spin until the 4 n tagged words at byte `offset` of the mapped mailbox carry
-// message seq, then unpack their n elements (2 words each).
+// message seq, then unpack their n elements (2 words each).  `taken` is set when
+// a word carries a later number instead: another thread's post overwrote it.
 int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
-                  uint64_t *out);
+                  uint64_t *out, bool *taken = nullptr);
 // The post of up to kPostElements elements by the next kernels on the context
 // stream (one at a time), and the wait for its first n.
 constexpr int kPostElements = 128;

@@ -1,0 +1,95 @@
+// Host paths that a GPU cannot be made to take at will, over the fake runtime:
+// `host_paths CASE` prints what the case found and exits with 0 when it held.
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "fake_cudart.h"
+#include "runtime.h"
+
+#define CHECK(x)                                                    \
+    do {                                                            \
+        if (!(x)) {                                                 \
+            printf("%s:%d: %s\n", __FILE__, __LINE__, #x);          \
+            return 1;                                               \
+        }                                                           \
+    } while (0)
+
+namespace {
+
+bz_ctx *ctx;
+const bz_params kSmall = {8, 1, 3, BZ_HASH_BLAKE3};
+
+// A commit whose kernels post nothing: its root is what the tree's memory
+// holds, 0xA5 in every byte.
+int commit_root_is_the_trees() {
+    std::vector<uint64_t> msg(2 << 8);
+    bz_commitment *c = nullptr;
+    uint8_t root[32] = {0};
+    CHECK(bz_commit(ctx, msg.data(), 1 << 8, &kSmall, &c, root) == BZ_OK);
+    for (int i = 0; i < 32; ++i) CHECK(root[i] == 0xA5);
+    CHECK(bz_commitment_root(c, root) == BZ_OK && root[0] == 0xA5);
+    CHECK(bz_commitment_free(c) == BZ_OK);
+    return 0;
+}
+
+// The stream goes idle and the mailbox has no root.
+int root_not_posted() { return commit_root_is_the_trees(); }
+
+// Commits of other threads took the slot before the owner read it: every word
+// of the 16 slots carries a later number.
+int root_slot_reused() {
+    int queries = 0;
+    fake::query = [&] {
+        uint64_t *w = (uint64_t *)((uint8_t *)ctx->h_mbox + 1024);
+        for (int i = 0; i < 16 * 16; ++i) w[i] = (uint64_t)(ctx->root_seq + 16) << 32;
+        return ++queries < 100 ? cudaErrorNotReady : cudaSuccess;
+    };
+    return commit_root_is_the_trees();
+}
+
+// The work queued before the commit takes longer than a spinning wait allows.
+int root_slow() {
+    bool done = false;
+    fake::query = [&] {
+        fake::clock_skew_s += 61;
+        return done ? cudaSuccess : cudaErrorNotReady;
+    };
+    fake::sync = [&] {
+        done = true;
+        return cudaSuccess;
+    };
+    return commit_root_is_the_trees();
+}
+
+// A failed stream still fails the commit.
+int root_stream_error() {
+    fake::query = [] { return cudaErrorLaunchFailure; };
+    fake::sync = [] { return cudaErrorLaunchFailure; };
+    std::vector<uint64_t> msg(2 << 8);
+    bz_commitment *c = nullptr;
+    uint8_t root[32];
+    CHECK(bz_commit(ctx, msg.data(), 1 << 8, &kSmall, &c, root) == BZ_ERR_CUDA);
+    CHECK(!c);
+    return 0;
+}
+
+const struct {
+    const char *name;
+    int (*run)();
+} kCases[] = {
+    {"root_not_posted", root_not_posted},
+    {"root_slot_reused", root_slot_reused},
+    {"root_slow", root_slow},
+    {"root_stream_error", root_stream_error},
+};
+
+}  // namespace
+
+int main(int argc, char **argv) {
+    if (bz_ctx_create(0, 0, &ctx) != BZ_OK) return 2;
+    for (const auto &c : kCases)
+        if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();
+    for (const auto &c : kCases) printf("%s\n", c.name);
+    return argc == 1 ? 0 : 2;
+}
