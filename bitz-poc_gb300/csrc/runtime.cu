@@ -975,6 +975,10 @@ ElementPost next_element_post(bz_ctx *ctx) {
 }
 
 int posted_wait(bz_ctx *ctx, const ElementPost &post, int n, const char *what, uint64_t *out) {
+    const int rc = elements_wait(ctx, kElementsOffset, n, post.seq, what, out);
+    if (rc != BZ_ERR_TIMEOUT) return rc;
+    // the work queued before the post outlasts the spin
+    BZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return elements_wait(ctx, kElementsOffset, n, post.seq, what, out);
 }
 

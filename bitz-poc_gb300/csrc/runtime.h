@@ -194,7 +194,7 @@ int msg_wait(bz_ctx *ctx, uint32_t seq, int posts, uint64_t u0[2], uint64_t u2[2
 int elements_wait(bz_ctx *ctx, size_t offset, int n, uint32_t seq, const char *what,
                   uint64_t *out, bool *taken = nullptr);
 // The post of up to kPostElements elements by the next kernels on the context
-// stream (one at a time), and the wait for its first n.
+// stream (one at a time), and the wait for its first n (no time limit).
 constexpr int kPostElements = 128;
 ElementPost next_element_post(bz_ctx *ctx);
 int posted_wait(bz_ctx *ctx, const ElementPost &post, int n, const char *what, uint64_t *out);

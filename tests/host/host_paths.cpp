@@ -74,6 +74,39 @@ int root_stream_error() {
     return 0;
 }
 
+// Posted elements behind work that outlasts the spin: the partial evaluations
+// come when the stream is synchronised.
+int elements_slow() {
+    bool done = false;
+    fake::query = [&] {
+        fake::clock_skew_s += 61;
+        return done ? cudaSuccess : cudaErrorNotReady;
+    };
+    fake::sync = [&] {
+        uint64_t *w = (uint64_t *)((uint8_t *)ctx->h_mbox + 4096);
+        for (int i = 0; i < 4 * 128; ++i) w[i] = (uint64_t)ctx->mbox_seq << 32 | i;
+        done = true;
+        return cudaSuccess;
+    };
+    std::vector<uint64_t> d(2 << 8), sv(256);
+    CHECK(bz_sv_fold(ctx, d.data(), d.data(), 1 << 8, sv.data()) == BZ_OK);
+    for (uint64_t i = 0; i < 256; ++i) CHECK(sv[i] == ((2 * i) | (2 * i + 1) << 32));
+    return 0;
+}
+
+// A stream that goes idle, or fails, without the post is an error.
+int elements_not_posted() {
+    std::vector<uint64_t> d(2 << 8), sv(256);
+    CHECK(bz_sv_fold(ctx, d.data(), d.data(), 1 << 8, sv.data()) == BZ_ERR_CUDA);
+    fake::query = [] {
+        fake::clock_skew_s += 61;
+        return cudaErrorNotReady;
+    };
+    fake::sync = [] { return cudaErrorLaunchFailure; };
+    CHECK(bz_sv_fold(ctx, d.data(), d.data(), 1 << 8, sv.data()) == BZ_ERR_CUDA);
+    return 0;
+}
+
 const struct {
     const char *name;
     int (*run)();
@@ -82,6 +115,8 @@ const struct {
     {"root_slot_reused", root_slot_reused},
     {"root_slow", root_slow},
     {"root_stream_error", root_stream_error},
+    {"elements_slow", elements_slow},
+    {"elements_not_posted", elements_not_posted},
 };
 
 }  // namespace
