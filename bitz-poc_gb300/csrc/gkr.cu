@@ -94,9 +94,9 @@ struct Armed {
 
 // The whole proof from device leaves (n of them, overwritten: the leaf layer
 // is folded in place as the rounds go).
-int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_t *point,
-            bz_gkr_transcript_fn fn, void *user, uint64_t *roots, uint64_t *out_point,
-            uint64_t out_claim[2]) {
+int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_t *point,
+               bz_gkr_transcript_fn fn, void *user, uint64_t *roots, uint64_t *out_point,
+               uint64_t out_claim[2]) {
     cudaStream_t st = ctx->stream;
     const int L = log2u(n), S = log2u(groups), layers = L - S;
     // layers 1 .. layers above the leaves, each half the one below
@@ -267,6 +267,18 @@ int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_
     out_claim[0] = claim.w[0];
     out_claim[1] = claim.w[1];
     return BZ_OK;
+}
+
+// A round's post orders its sums alone.  The caller may use its leaves buffer,
+// which the rounds fold in, on any stream, and roots in pinned memory at once,
+// whether the proof was finished or ended early: so the stream is waited for.
+int gkr_run(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint64_t *point,
+            bz_gkr_transcript_fn fn, void *user, uint64_t *roots, uint64_t *out_point,
+            uint64_t out_claim[2]) {
+    const int rc = gkr_rounds(ctx, d_leaves, n, groups, point, fn, user, roots, out_point,
+                              out_claim);
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    return rc || e == cudaSuccess ? rc : set_err(ctx, BZ_ERR_CUDA, "grand-product proof", e);
 }
 
 int check_shape(bz_ctx *ctx, size_t n, size_t groups) {

@@ -2,7 +2,8 @@
 non-blocking stream: the tree and codeword of a commit, whose root the last
 kernel posts (one-CTA trees of both hashes, levels above leaf kernels), and the
 folded arrays of a public fold, whose message one to sixteen CTAs or the last of
-many post.  Compared with the oracle for equality."""
+many post; and the leaves buffer that a grand-product proof folds in.  Compared
+with the oracle for equality."""
 import ctypes
 
 import numpy as np
@@ -66,3 +67,35 @@ def test_folds_on_another_stream(oracle, ctx, other, log_n):
         gf = _read(other, nf.ptr.value, ef.shape, np.uint64)
         assert (gb == eb).all() and (gf == ef).all()
         assert (u0 == e0).all() and (u2 == e2).all()
+
+
+@pytest.mark.parametrize("log_n,fails", [(1, False), (2, False), (6, False), (12, False),
+                                         (12, True)])
+def test_leaves_reused_on_another_stream(ctx, other, log_n, fails):
+    """A proof folds in its leaves buffer; what another stream writes there as
+    soon as the call returns stays."""
+    from bitz_gb300 import DeviceArray, _lib, lib
+    from bitz_gb300 import gkr as K
+    from oracle import gkr as G
+
+    rng = np.random.default_rng(log_n)
+    n = 1 << log_n
+    leaves, marks = (rng.integers(0, 2**64, (n, 2), dtype=np.uint64) for _ in range(2))
+
+    class Failing(G.HashChallenges):
+        def challenge(self, stage):
+            if fails and len(self.messages) > 20:
+                raise RuntimeError("no challenge")
+            return super().challenge(stage)
+
+    d = DeviceArray.from_host(leaves, ctx)
+    for _ in range(16):
+        assert lib().bz_memcpy_h2d(ctx.handle, d.ptr, _lib.ptr(leaves), leaves.nbytes) == 0
+        if fails:
+            with pytest.raises(RuntimeError):
+                K.prove(d, 1, [], Failing(b"reuse"), ctx)
+        else:
+            K.prove(d, 1, [], Failing(b"reuse"), ctx)
+        assert lib().bz_memcpy_h2d(other.handle, d.ptr, _lib.ptr(marks), marks.nbytes) == 0
+        assert lib().bz_ctx_synchronize(ctx.handle) == 0
+        assert (_read(other, d.ptr.value, marks.shape, np.uint64) == marks).all()
