@@ -77,8 +77,11 @@ struct DevBuf {
 
 // A GKR round's gate waits for the caller's transcript.  A transcript that
 // takes longer (or waits on the context's stream, which the armed round holds)
-// costs this once per context; the round then runs unarmed.
+// costs this once per proof, whose later rounds run unarmed.  One pause of the
+// host passes; after kGkrGateProofs proofs in a row the transcript is taken to be
+// slow and the context arms no further.
 constexpr uint64_t kGkrGateLimitNs = 2000000ull;
+constexpr int kGkrGateProofs = 3;
 
 // The armed round, withdrawn when the proof ends early.
 struct Armed {
@@ -116,6 +119,7 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
     constexpr size_t kTailOffset = 512;
     uint64_t *d_tail = (uint64_t *)((uint8_t *)ctx->d_mbox + kTailOffset);
     Armed armed{ctx};
+    bool arm = ctx->gkr_gates_out < kGkrGateProofs;
     std::vector<uint4 *> layer(layers + 1);
     layer[0] = d_leaves;
     size_t off = 0;
@@ -187,7 +191,7 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
                 // The next round, if a small one, is enqueued behind this one
                 // and waits on the device for the challenge: its launch
                 // overlaps the wait, the sums' host work and the transcript.
-                if (rnd + 1 < k && ctx->arm_gkr && small(rnd + 1)) {
+                if (rnd + 1 < k && arm && small(rnd + 1)) {
                     const RGate g = next_gate(ctx, kGkrGateLimitNs);
                     armed.post = next_msg_post(ctx);
                     if ((rc = launch(rnd + 1, armed.post, &g))) return rc;
@@ -200,13 +204,15 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
                 if (rc && was_armed) {
                     // the gate ran out before the challenge came (a transcript
                     // that took long or used the context's stream): the round
-                    // was left undone, so run it unarmed and arm no further
+                    // was left undone, so run it unarmed and arm no further in
+                    // this proof
                     if (armed.fold.live) fold_cancel(ctx, &armed.fold);
                     const bool arm_folds = ctx->arm_folds;
                     const bool gave_up = gate_gave_up(ctx);
                     ctx->arm_folds = arm_folds;
                     if (gave_up) {
-                        ctx->arm_gkr = false;
+                        arm = false;
+                        ++ctx->gkr_gates_out;
                         reset_msg_ticket(ctx);
                         flip(rnd);
                         post = next_msg_post(ctx);
@@ -266,6 +272,7 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
     }
     out_claim[0] = claim.w[0];
     out_claim[1] = claim.w[1];
+    if (arm) ctx->gkr_gates_out = 0;
     return BZ_OK;
 }
 

@@ -68,7 +68,7 @@ struct bz_ctx {
     std::atomic<uint32_t> root_seq{0};  // commits whose root the mailbox was offered to
     uint32_t gate_seq = 0;    // last armed fold's gate number
     bool arm_folds = true;    // cleared after a gate ran out (the prover stops arming)
-    bool arm_gkr = true;      // the same for GKR rounds, whose transcript is the caller's
+    int gkr_gates_out = 0;    // GKR proofs in a row in which a gate ran out
     uint32_t pow_seq = 0;     // last proof-of-work search's mailbox number
     bool pow_ready = false;   // the search's device counters hold their idle values
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
