@@ -357,14 +357,19 @@ int commitment_open_on(bz_commitment *c, const uint64_t *positions, size_t q, ui
     }
     uint8_t *d_out = (uint8_t *)mem;
     uint64_t *d_idx = (uint64_t *)(d_out + out_bytes);
-    if (q) cudaMemcpyAsync(d_idx, positions, q * 8, cudaMemcpyHostToDevice, st);
-    if (n) cudaMemcpyAsync(d_idx + q, idx, n * 8, cudaMemcpyHostToDevice, st);
-    gather(d_idx, d_out);
-    if (q) cudaMemcpyAsync(rows, d_out, row_bytes, cudaMemcpyDeviceToHost, st);
-    if (n) cudaMemcpyAsync(nodes, d_out + row_bytes, 32 * n, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(mem, st);
-    BZ_CUDA(ctx, cudaStreamSynchronize(st));
-    return BZ_OK;
+    cudaError_t err = cudaSuccess;  // the first
+    auto check = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
+    if (q) check(cudaMemcpyAsync(d_idx, positions, q * 8, cudaMemcpyHostToDevice, st));
+    if (n) check(cudaMemcpyAsync(d_idx + q, idx, n * 8, cudaMemcpyHostToDevice, st));
+    if (err == cudaSuccess) gather(d_idx, d_out);
+    check(cudaGetLastError());
+    if (q) check(cudaMemcpyAsync(rows, d_out, row_bytes, cudaMemcpyDeviceToHost, st));
+    if (n) check(cudaMemcpyAsync(nodes, d_out + row_bytes, 32 * n, cudaMemcpyDeviceToHost, st));
+    check(cudaFreeAsync(mem, st));
+    check(cudaStreamSynchronize(st));
+    if (err == cudaSuccess) return BZ_OK;
+    cudaGetLastError();  // reported here, not by the next call
+    return set_err(ctx, BZ_ERR_CUDA, "opening", err);
 }
 
 std::future<int> side_async(bz_ctx *ctx, std::function<int()> job) {

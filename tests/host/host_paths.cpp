@@ -107,6 +107,38 @@ int elements_not_posted() {
     return 0;
 }
 
+// Openings through device buffers (the mapped one is held): a refused launch and
+// each copy that fails are errors, not rows that were never gathered.
+int opening_errors() {
+    std::vector<uint64_t> msg(2 << 8);
+    bz_commitment *c = nullptr;
+    uint8_t root[32];
+    CHECK(bz_commit(ctx, msg.data(), 1 << 8, &kSmall, &c, root) == BZ_OK);
+    const std::vector<uint64_t> pos = {1, 5, 9};
+    std::vector<uint64_t> rows(3 * 8 * 2);
+    std::vector<uint8_t> nodes(32 * 64);
+    size_t n = 0;
+    auto open_rows = [&] { return bz_commitment_rows(c, pos.data(), 3, rows.data()); };
+    auto open_nodes = [&] {
+        return bz_commitment_multiproof(c, pos.data(), 3, nodes.data(), 64, &n);
+    };
+    std::lock_guard<std::mutex> held(ctx->open_mu);
+    CHECK(open_rows() == BZ_OK && open_nodes() == BZ_OK);
+    fake::launch = [] { return cudaErrorInvalidConfiguration; };
+    CHECK(open_rows() == BZ_ERR_CUDA && open_nodes() == BZ_ERR_CUDA);
+    fake::launch = nullptr;
+    for (int bad = 0; bad < 2; ++bad) {  // the indices up, the results down
+        int at = 0;
+        fake::copy = [&] { return at++ == bad ? cudaErrorInvalidValue : cudaSuccess; };
+        CHECK(open_rows() == BZ_ERR_CUDA);
+        at = 0;
+        CHECK(open_nodes() == BZ_ERR_CUDA);
+    }
+    fake::copy = nullptr;
+    CHECK(open_rows() == BZ_OK && open_nodes() == BZ_OK);
+    return 0;
+}
+
 const struct {
     const char *name;
     int (*run)();
@@ -117,6 +149,7 @@ const struct {
     {"root_stream_error", root_stream_error},
     {"elements_slow", elements_slow},
     {"elements_not_posted", elements_not_posted},
+    {"opening_errors", opening_errors},
 };
 
 }  // namespace
