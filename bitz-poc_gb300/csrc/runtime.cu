@@ -613,6 +613,13 @@ uint64_t bz_kernel_launches(const bz_ctx *ctx) { return ctx ? ctx->launches.load
 // synchronisation: whatever becomes of it, the tree holds the root.
 constexpr size_t kRootMbox = 1024, kRootSlotBytes = 128;
 constexpr uint32_t kRootSlots = 16;
+static RootPost next_root_post(bz_ctx *ctx) {
+    RootPost p;
+    p.seq = ++ctx->root_seq;
+    p.words = (uint64_t *)((uint8_t *)ctx->d_mbox + kRootMbox +
+                           (p.seq % kRootSlots) * kRootSlotBytes);
+    return p;
+}
 
 static int commit_device_enqueue(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
                                  const bz_params *params, bz_commitment **out, RootPost *post) {
@@ -642,10 +649,11 @@ int bz_commit_device_async(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
 // The posted root; or the tree's, when other threads' commits took the slot
 // before this one read it, or the work queued before the commit outlasts the
 // spin.
-static int root_wait(bz_ctx *ctx, size_t slot, uint32_t seq, bz_commitment *c) {
+static int root_wait(bz_ctx *ctx, const RootPost &post, bz_commitment *c) {
+    const size_t slot = (uint8_t *)post.words - (uint8_t *)ctx->d_mbox;
     uint64_t r[4];
     bool taken = false;
-    if (elements_wait(ctx, slot, 2, seq, "commit", r, &taken) == BZ_OK && !taken) {
+    if (elements_wait(ctx, slot, 2, post.seq, "commit", r, &taken) == BZ_OK && !taken) {
         memcpy(c->root, r, 32);
     } else {
         const uint8_t *src = c->d_tree + (c->shape.tree_nodes() - 1) * 32;
@@ -659,14 +667,10 @@ static int root_wait(bz_ctx *ctx, size_t slot, uint32_t seq, bz_commitment *c) {
 int bz_commit_device(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words, const bz_params *params,
                      bz_commitment **out, uint8_t root[32]) {
     if (!ctx) return BZ_ERR_ARG;
-    const uint32_t seq = ++ctx->root_seq;
-    const size_t slot = kRootMbox + (seq % kRootSlots) * kRootSlotBytes;
-    RootPost post;
-    post.words = (uint64_t *)((uint8_t *)ctx->d_mbox + slot);
-    post.seq = seq;
+    RootPost post = next_root_post(ctx);
     int rc = commit_device_enqueue(ctx, d_msg, n_words, params, out, &post);
     if (rc) return rc;
-    rc = post.words ? root_wait(ctx, slot, seq, *out) : fetch_root(*out);
+    rc = post.words ? root_wait(ctx, post, *out) : fetch_root(*out);
     if (rc) {
         bz_commitment_free(*out);
         *out = nullptr;
@@ -855,8 +859,9 @@ int bz_commit_profile(bz_ctx *ctx, const uint64_t *d_msg, size_t n_words,
         LaunchLog log;
         log.st = ctx->stream;
         log.mark("start");
+        RootPost post = next_root_post(ctx);  // the kernels of a commit that posts its root
         int n = launch_commit_kernels(ctx, s, schedule_for(ctx, s), (const uint4 *)d_msg, c->d_cw,
-                                      c->d_tree, d_tw, ctx->stream, &log);
+                                      c->d_tree, d_tw, ctx->stream, &log, &post);
         ctx->launches += (uint64_t)n;
         cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) {

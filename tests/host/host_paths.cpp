@@ -139,6 +139,27 @@ int opening_errors() {
     return 0;
 }
 
+// A profile runs the launches of the commit that a caller waits for.
+int profile_is_the_commit() {
+    const bz_params shapes[] = {kSmall, {12, 1, 1, BZ_HASH_BLAKE3}, {16, 1, 6, BZ_HASH_BLAKE3},
+                                {14, 2, 7, BZ_HASH_BLAKE3}, {14, 1, 2, BZ_HASH_SHA256}};
+    for (const bz_params &p : shapes) {
+        const size_t n = (size_t)1 << p.log_msg_len;
+        std::vector<uint64_t> msg(2 * n);
+        bz_commitment *c = nullptr;
+        uint8_t root[32];
+        uint64_t before = bz_kernel_launches(ctx);
+        CHECK(bz_commit_device(ctx, msg.data(), n, &p, &c, root) == BZ_OK);
+        const uint64_t launches = bz_kernel_launches(ctx) - before;
+        size_t count = 0;
+        before = bz_kernel_launches(ctx);
+        CHECK(bz_commit_profile(ctx, msg.data(), n, &p, 0, nullptr, nullptr, &count, root) == BZ_OK);
+        CHECK(count == launches && bz_kernel_launches(ctx) - before == launches);
+        CHECK(bz_commitment_free(c) == BZ_OK);
+    }
+    return 0;
+}
+
 const struct {
     const char *name;
     int (*run)();
@@ -150,6 +171,7 @@ const struct {
     {"elements_slow", elements_slow},
     {"elements_not_posted", elements_not_posted},
     {"opening_errors", opening_errors},
+    {"profile_is_the_commit", profile_is_the_commit},
 };
 
 }  // namespace

@@ -1,7 +1,7 @@
 """Host paths of the library over a fake CUDA runtime (tests/host): a posted
 root that never comes, comes after a later commit took its mailbox slot, or
-takes longer than the host spins for, posted elements that do, and openings
-whose copies or launch are refused."""
+takes longer than the host spins for, posted elements that do, openings whose
+copies or launch are refused, and the launches of a profiled commit."""
 import os
 import shutil
 import subprocess
@@ -34,7 +34,7 @@ def host_paths(tmp_path_factory):
 
 @pytest.mark.parametrize("case", ["root_not_posted", "root_slot_reused", "root_slow",
                                   "root_stream_error", "elements_slow", "elements_not_posted",
-                                  "opening_errors"])
+                                  "opening_errors", "profile_is_the_commit"])
 def test_host_path(host_paths, case):
     r = subprocess.run([host_paths, case], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
