@@ -199,6 +199,54 @@ __device__ __forceinline__ void sha256_compress(uint32_t st[8], const uint32_t w
     for (int i = 0; i < 8; ++i) st[i] += v[i];
 }
 
+// The same with every round unrolled, plain additions and the state moved from
+// name to name, for the persistent batch kernel's tree levels.  That kernel's 27
+// item functions share its registers, and with either form above in the levels
+// the compiler leaves the NTT passes fewer (2^24-element passes spill 128 bytes
+// a thread against 92): 48 commits of 2^16 to 2^24 elements 61.0 ms, 60.0 with
+// this one.  SHA-256 trees of 32 lanes pay for it with 91.5 -> 92.2 ms.
+__device__ __forceinline__ void sha256_compress_moved(uint32_t st[8], const uint32_t w_in[16]) {
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = w_in[i];
+    uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6],
+             h = st[7];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) {
+        uint32_t wi;
+        if (i < 16) {
+            wi = w[i];
+        } else {
+            const uint32_t x = w[(i - 15) & 15], y = w[(i - 2) & 15];
+            const uint32_t s0 = rotr(x, 7) ^ rotr(x, 18) ^ (x >> 3);
+            const uint32_t s1 = rotr(y, 17) ^ rotr(y, 19) ^ (y >> 10);
+            wi = w[i & 15] + s0 + w[(i - 7) & 15] + s1;
+            w[i & 15] = wi;
+        }
+        const uint32_t S1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);
+        const uint32_t ch = (e & f) ^ (~e & g);
+        const uint32_t t1 = h + S1 + ch + kSHA.w[i] + wi;
+        const uint32_t S0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);
+        const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+        h = g;
+        g = f;
+        f = e;
+        e = d + t1;
+        d = c;
+        c = b;
+        b = a;
+        a = t1 + S0 + mj;
+    }
+    st[0] += a;
+    st[1] += b;
+    st[2] += c;
+    st[3] += d;
+    st[4] += e;
+    st[5] += f;
+    st[6] += g;
+    st[7] += h;
+}
+
 // A block whose kSHA[i] + w_i are known: no message schedule.
 template <bool ROLLED>
 __device__ __forceinline__ void sha256_compress_kw(uint32_t st[8], const ShaWords &kw) {

@@ -147,6 +147,8 @@ __device__ __forceinline__ void b3_leaves_small_body(const uint4 *cw, int log_la
 // of the flat tree), so a 2^20-leaf tree needs 3 launches instead of 20.
 // kind: 0 = SHA-256, 1 = BLAKE3.
 // ---------------------------------------------------------------------------
+// MOVED: by sha256_compress_moved, padding block and all.
+template <bool MOVED>
 __device__ __forceinline__ void sha256_pair(const uint32_t l[8], const uint32_t r[8],
                                             uint32_t out[8]) {
     uint32_t st[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
@@ -157,16 +159,26 @@ __device__ __forceinline__ void sha256_pair(const uint32_t l[8], const uint32_t 
         w[i] = bswap32(l[i]);
         w[8 + i] = bswap32(r[i]);
     }
-    sha256_compress<true>(st, w);
-    sha256_compress_kw<true>(st, kShaPairPad);
+    if constexpr (MOVED) {
+        sha256_compress_moved(st, w);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[i] = 0;
+        w[0] = 0x80000000u;
+        w[15] = 512;
+        sha256_compress_moved(st, w);
+    } else {
+        sha256_compress<true>(st, w);
+        sha256_compress_kw<true>(st, kShaPairPad);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) out[i] = bswap32(st[i]);
 }
 
+template <bool MOVED>
 __device__ __forceinline__ void hash_pair(int kind, const uint32_t l[8], const uint32_t r[8],
                                           uint32_t out[8]) {
     if (kind == 1) b3_parent(l, r, out);
-    else sha256_pair(l, r, out);
+    else sha256_pair<MOVED>(l, r, out);
 }
 
 // in: n_in nodes (32 B each); outputs levels written at out_levels[0..k-1]
@@ -183,6 +195,7 @@ struct LevelsArgs {
 
 // Body: unit u (512 input nodes) with threads 0..255; any further threads of
 // the CTA only take part in its barriers.  nodes holds 256 padded rows.
+template <bool MOVED = false>
 __device__ __forceinline__ void merkle_levels_body(const LevelsArgs &a, uint64_t u,
                                                    uint32_t (*nodes)[9]) {
     const int t = threadIdx.x;
@@ -209,7 +222,7 @@ __device__ __forceinline__ void merkle_levels_body(const LevelsArgs &a, uint64_t
                     r[i] = nodes[2 * t + 1][i];
                 }
             }
-            hash_pair(a.kind, l, r, o);
+            hash_pair<MOVED>(a.kind, l, r, o);
             uint4 *po = reinterpret_cast<uint4 *>(a.out[lv] + (u * (256 >> lv) + t) * 8);
             po[0] = make_uint4(o[0], o[1], o[2], o[3]);
             po[1] = make_uint4(o[4], o[5], o[6], o[7]);

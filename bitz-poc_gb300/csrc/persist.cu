@@ -211,7 +211,7 @@ __device__ __noinline__ void levels_item(const PStep *st, uint64_t b, uint64_t e
     const LevelsArgs a = st->lv;
     uint32_t(*nodes)[9] = reinterpret_cast<uint32_t(*)[9]>(base);
     for (uint64_t u = b; u < e; ++u) {
-        merkle_levels_body(a, u, nodes);
+        merkle_levels_body<true>(a, u, nodes);
         __syncthreads();
     }
 }
