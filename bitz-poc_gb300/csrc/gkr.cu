@@ -143,7 +143,7 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
         const int k = L - j - 1;  // coordinates of this layer's point
         uint4 *l = layer[j], *r = layer[j] + ((size_t)1 << k);
         uint4 *nl = (uint4 *)((uint8_t *)scratch.p + part_bytes), *nr = nl + 2 * coop;
-        uint32_t tail_seq = 0;
+        uint64_t lr[8] = {0};  // the close's entries
         Gf factor = gone(), rho;
         std::vector<Gf> next;
         bool pending = false;
@@ -226,7 +226,11 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
                     reset_msg_ticket(ctx);
                     return rc;
                 }
-                tail_seq = post.seq_val;
+                // the close's entries, before a callback that proves on this
+                // context takes their place in the mailbox
+                if (rnd == k - 1 &&
+                    (rc = elements_wait(ctx, kTailOffset, 4, post.seq_val, "layer close", lr)))
+                    return rc;
                 se = gmul(factor, se);
                 si = gmul(factor, si);
                 const uint64_t msg[4] = {se.w[0], se.w[1], si.w[0], si.w[1]};
@@ -242,10 +246,7 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
         // the close (gkr.rs:270-281): the last fold of the two-entry halves
         // two entries per half still to fold, posted by the last round, or (a
         // layer without rounds) one
-        uint64_t lr[8] = {0};
-        if (pending) {
-            if ((rc = elements_wait(ctx, kTailOffset, 4, tail_seq, "layer close", lr))) return rc;
-        } else {
+        if (!pending) {
             BZ_CUDA(ctx, cudaMemcpyAsync(lr, l, 16, cudaMemcpyDeviceToHost, st));
             BZ_CUDA(ctx, cudaMemcpyAsync(lr + 4, r, 16, cudaMemcpyDeviceToHost, st));
             BZ_CUDA(ctx, cudaStreamSynchronize(st));
