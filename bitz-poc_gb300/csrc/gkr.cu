@@ -207,10 +207,13 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
                     // was left undone, so run it unarmed and arm no further in
                     // this proof
                     if (armed.fold.live) fold_cancel(ctx, &armed.fold);
+                    // (a proof that the callback ran on this context may have
+                    // cleared the gate's record: a stream drained without the
+                    // post says the same)
                     const bool arm_folds = ctx->arm_folds;
-                    const bool gave_up = gate_gave_up(ctx);
+                    gate_gave_up(ctx);
                     ctx->arm_folds = arm_folds;
-                    if (gave_up) {
+                    if (cudaStreamSynchronize(st) == cudaSuccess) {
                         arm = false;
                         ++ctx->gkr_gates_out;
                         reset_msg_ticket(ctx);

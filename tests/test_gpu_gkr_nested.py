@@ -1,6 +1,9 @@
-"""A transcript that itself proves on the same context, before a layer's close
-(whose entries the last round posts) and while a round is armed.  Both proofs
-equal the oracle's."""
+"""A transcript that itself proves on the same context: before a layer's close
+(whose entries the last round posts), while a round is armed, and with a pause of
+its own behind an armed round of the inner proof.  Both proofs equal the
+oracle's."""
+import time
+
 import numpy as np
 import pytest
 from test_gpu_gkr_armed import _case, _oracle
@@ -9,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("at", [1, 2, 3, 6, 7, 20, 40, 41, 42])
-def test_proof_inside_a_callback(at):
+@pytest.mark.parametrize("pause", [False, True])
+def test_proof_inside_a_callback(at, pause):
     from bitz_gb300 import Context
     from bitz_gb300 import gkr as K
     from oracle import gkr as G
@@ -21,10 +25,16 @@ def test_proof_inside_a_callback(at):
     exp_inner = _oracle(inner, [])
     got_inner = []
 
+    class Pausing(G.HashChallenges):
+        def challenge(self, stage):
+            if pause and len(self.messages) == 12:
+                time.sleep(0.01)
+            return super().challenge(stage)
+
     class Nested(G.HashChallenges):
         def challenge(self, stage):
             if len(self.messages) == at:
-                tr = G.HashChallenges(b"armed")
+                tr = Pausing(b"armed")
                 _, _, claim = K.prove(inner, 1, [], tr, own)
                 got_inner.append((tr.messages, G.gf_key(claim)))
             return super().challenge(stage)
