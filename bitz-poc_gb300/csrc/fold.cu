@@ -590,7 +590,8 @@ int launch_partial_eval_round(const uint4 *d_in, size_t n, uint4 r, uint4 *d_out
 }
 
 // The point of an eq table is a kernel argument: no upload and no buffer, and
-// the small tables are built while the previous kernel still runs.
+// the small tables are built before chain_wait, while the previous kernel, whose
+// CTAs have exited, is retired and its writes are flushed.
 constexpr int kEqSplitMaxK = 22;
 struct EqPoint {
     uint4 r[kEqSplitMaxK];
@@ -777,6 +778,7 @@ int launch_build_eq(const uint64_t *point, size_t k, uint4 *d_out, cudaStream_t 
 // of one group by every thread.  A CTA runs four such tiles side by side and
 // stores its sums; a CTA per output adds them (2^20 words: 80 us before).
 constexpr int kSvTile = 128;
+// Block swaps of halving size (Warren, Hacker's Delight, 7-3), a row a lane.
 __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll

@@ -177,8 +177,9 @@ int gkr_rounds(bz_ctx *ctx, uint4 *d_leaves, size_t n, size_t groups, const uint
             };
             for (int rnd = 0; rnd < k; ++rnd) {
                 const Gf &z = p[rnd];
-                // the round's last CTA posts the two sums to the mapped
-                // mailbox: no finish kernel, copy or stream synchronisation
+                // up to kMsgPosts CTAs post their two sums to the mapped mailbox
+                // and the host adds them (of more, the last posts for all): no
+                // finish kernel, copy or stream synchronisation
                 const bool was_armed = armed.fold.live;
                 MsgPost post = armed.post;
                 if (was_armed) {

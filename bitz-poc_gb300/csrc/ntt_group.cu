@@ -107,8 +107,8 @@ int launch_group8(const Shape &s, int depth, const uint4 *src, int src_bits, uin
     }
     const int w2 = narrow_class(twiddle_bits(ell, ell - 3));
     const int w1 = narrow_class(twiddle_bits(ell, ell - 2));
-    // the offsets of a block in a chunk of 2^t tasks have up to
-    // 4 (t - L) <= 32 bits at depth 2, which the 64-bit product holds
+    // the offsets of a block in a chunk of 2^t tasks have t - L bits and their
+    // twiddles a degree of up to 4 (t - L) <= 32 at depth 2: 33 bits, two words
 #define BZ_G_RUN(A, B, C)                                                                     \
     {                                                                                         \
         if (L >= t) launch_chained(ntt_group8<A, B, C, 0>, grid, 1u << t, kGroup8Smem, st, a);\

@@ -33,12 +33,11 @@ struct GroupPassArgs {
 // The byte tables of t8.cuh and the compact tables of ntt_kernels.cuh with
 // rows of 128 bytes at a pitch of 256: two tables share 64 KB.  A byte of the
 // operand that stands at bits 8-15 of a word is then a row offset as it is,
-// and the other three are brought there by one multiply with a power of two,
-// so a lookup costs one ALU operation (mask and lane offset in one LOP3)
-// beside its shared-memory wavefronts.  The powers of two come from constant
-// memory, because the compiler turns a multiply by a known one into a shift
-// on the ALU pipe, which bounds the four-layer pass (75 % busy with shifts,
-// the FMA pipes 6 %).
+// and the other three are brought there by one shift, so a lookup costs one or
+// two ALU operations (mask and lane offset in one LOP3) beside its shared-memory
+// wavefronts.  Multiplies by powers of two in place of the shifts leave the ALU
+// pipe 59 % busy instead of 75, and the four-layer pass takes as long (2^26
+// elements of 4096 lanes 496 us, 475 with shifts): the issue slots bound it too.
 constexpr int kGPairBytes = 65536;
 
 __device__ __forceinline__ int group_slot(int j) { return (j >> 1) * kGPairBytes + (j & 1) * 128; }

@@ -127,6 +127,7 @@ uint32_t log2_exact(size_t n) {
 }
 
 // 64 x 64 bits: out[u] bit v = in[v] bit u, by swapping blocks of halving size
+// (Warren, Hacker's Delight, 7-3)
 void transpose_bits_64(uint64_t x[64]) {
     uint64_t m = 0x00000000FFFFFFFFull;
     for (int j = 32; j; j >>= 1, m ^= m << j)
