@@ -90,11 +90,13 @@ struct MsgMailbox {
 };
 
 // Lanes 0 and 1 of the calling warp post u0 and u2, behind a barrier that
-// follows the CTA's stores.
+// follows the CTA's stores.  RELEASE is false in the kernels whose arrays only
+// the provers read: GKR rounds pay 0.3 us each for the fence's branch and code.
+template <bool RELEASE>
 __device__ __forceinline__ void post_pair(uint64_t word, const MsgMailbox &mb) {
     const uint4 v = reduce_pair(word);
     const int ln = threadIdx.x & 31;
-    if (mb.release) post_release();
+    if (RELEASE && mb.release) post_release();
     if (ln < 2) post_element(mb.words + 4 * ln, mb.seq_val, v);
 }
 
@@ -121,10 +123,11 @@ __device__ uint64_t partials_xor(const uint64_t *partials, int n) {
 // the ticket takes 0.9 to 2.1).  Otherwise every CTA stores its partial, and
 // with a mailbox the last one (whose ticket completes the count) reduces them
 // all, posts and resets the ticket for the next launch.
+template <bool RELEASE>
 __device__ __forceinline__ void msg_out(uint64_t word, uint64_t *partials, MsgMailbox mb) {
     if (mb.ticket && msg_posts(gridDim.x) == (int)gridDim.x) {
         mb.words += 8 * blockIdx.x;
-        if (threadIdx.x < 32) post_pair(word, mb);
+        if (threadIdx.x < 32) post_pair<RELEASE>(word, mb);
         return;
     }
     if (threadIdx.x < 8) partials[(uint64_t)blockIdx.x * 8 + threadIdx.x] = word;
@@ -139,20 +142,22 @@ __device__ __forceinline__ void msg_out(uint64_t word, uint64_t *partials, MsgMa
     if (!last) return;
     __threadfence();
     const uint64_t sum = partials_xor(partials, (int)gridDim.x);
-    if (threadIdx.x < 32) post_pair(sum, mb);
+    if (threadIdx.x < 32) post_pair<RELEASE>(sum, mb);
     if (threadIdx.x == 0) *mb.ticket = 0;
 }
 
+template <bool RELEASE>
 __device__ __forceinline__ void msg_finish(const gf_wide &u0, const gf_wide &u2,
                                            uint64_t *partials, const MsgMailbox &mb) {
-    msg_out(cta_xor_pair(u0, u2), partials, mb);
+    msg_out<RELEASE>(cta_xor_pair(u0, u2), partials, mb);
 }
 
 // Out of line for the fold kernel: its loop runs at the 128-register cap, and
 // an inlined epilogue adds spills to it.
+template <bool RELEASE>
 __device__ __noinline__ void msg_finish_call(gf_wide u0, gf_wide u2, uint64_t *partials,
                                              const MsgMailbox &mb) {
-    msg_finish(u0, u2, partials, mb);
+    msg_finish<RELEASE>(u0, u2, partials, mb);
 }
 
 __device__ __forceinline__ uint64_t ld_relaxed_sys(const uint64_t *p) {
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(256, 2) fold_and_msg_kernel(const uint4 *f, co
         gf_wide_xor(u0, gf_mul_wide(x0, y0));
         gf_wide_xor(u2, gf_mul_wide(gf_add(x0, x1), gf_add(y0, y1)));
     }
-    msg_finish_call(u0, u2, partials, mb);
+    msg_finish_call<true>(u0, u2, partials, mb);
 }
 
 __global__ void __launch_bounds__(256) round_msg_kernel(const uint4 *f, const uint4 *b,
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(256) round_msg_kernel(const uint4 *f, const ui
         gf_wide_xor(u0, gf_mul_wide(f0, b0));
         gf_wide_xor(u2, gf_mul_wide(gf_add(f0, f1), gf_add(b0, b1)));
     }
-    msg_finish(u0, u2, partials, mb);
+    msg_finish<false>(u0, u2, partials, mb);
 }
 
 // Final XOR of per-CTA partials and the single reduction: out = {u0, u2}.
@@ -469,7 +474,7 @@ __global__ void __launch_bounds__(kCoopThreads) coop_round_kernel(
         for (int k = 0; k < 4; ++k)
             if ((tid & 3) == k) word = x.w[k];
     }
-    msg_out(word, a.partials, a.mb);
+    msg_out<FOLD && !GKR>(word, a.partials, a.mb);
 }
 
 // Up to kMsgPosts CTAs while they take at most kCoopSlots each (the host adds
@@ -1056,7 +1061,7 @@ __global__ void __launch_bounds__(256, 2) gkr_round_kernel(uint4 *l, uint4 *r, c
         gf_wide_xor(e, gf_mul_wide(gf_mul(wc, le), re));
         gf_wide_xor(f, gf_mul_wide(gf_mul(wc, gf_add(l1, l0)), gf_add(r1, r0)));
     }
-    msg_finish_call(e, f, partials, mb);
+    msg_finish_call<false>(e, f, partials, mb);
 }
 
 // The leaf grid of the BitZ forest (src/bitz/forest_tests.rs:42-68): leaf
